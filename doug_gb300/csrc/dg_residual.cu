@@ -6,8 +6,8 @@
 // internally; this file exposes it to callers that hold their own device
 // CSR matrix (for example to check a solution written by dg_solve_device).
 //
-// The norm is reduced deterministically: each block of kResidRowsPerBlock
-// rows writes one partial sum, and one block adds the partials in order.
+// The norm is reduced deterministically: each block of rows_per_block rows
+// writes one partial sum, and one block adds the partials in order.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -19,32 +19,62 @@ namespace dg {
 namespace resid {
 
 constexpr int kThreads = 256;
-constexpr int kLanes = 8;                         // lanes per row
-constexpr int kRowsPerBlock = 1024;               // rows per partial sum
+constexpr int kMaxRowsPerBlock = 1024;            // rows per partial sum
 
-// r = b - A x for rows [blk*1024, (blk+1)*1024); partial[blk] = sum r_i^2
-__global__ void __launch_bounds__(kThreads)
-residual_partials(int n, const long long *__restrict__ rp, const int *__restrict__ col,
-                  const double *__restrict__ val, const double *__restrict__ x,
-                  const double *__restrict__ b, double *__restrict__ r, double *__restrict__ partial) {
-  __shared__ double sh[kThreads / 32];
-  const int sub = threadIdx.x % kLanes;
-  const int row_in_pass = threadIdx.x / kLanes;   // 32 rows per pass
-  const int r0 = blockIdx.x * kRowsPerBlock;
+// A block's rows with L lanes per row; returns this thread's part of sum r_i^2.
+// Four entries of a lane's share are loaded before they are summed.
+template <int L>
+__device__ __forceinline__ double block_rows(int r0, int r1, const long long *__restrict__ rp,
+                                             const int *__restrict__ col, const double *__restrict__ val,
+                                             const double *__restrict__ x, const double *__restrict__ b,
+                                             double *__restrict__ r) {
+  const int sub = threadIdx.x % L;
   double acc = 0.0;
-  for (int pass = 0; pass < kRowsPerBlock / (kThreads / kLanes); pass++) {
-    const int i = r0 + pass * (kThreads / kLanes) + row_in_pass;
+  for (int i0 = r0; i0 < r1; i0 += kThreads / L) {
+    const int i = i0 + threadIdx.x / L;
     double s = 0.0;
-    if (i < n)
-      for (long long e = rp[i] + sub; e < rp[i + 1]; e += kLanes) s = __fma_rn(val[e], x[col[e]], s);
+    if (i < r1) {
+      long long e = rp[i] + sub;
+      const long long e1 = rp[i + 1];
+      for (; e + 3 * L < e1; e += 4 * L) {
+        const int c0 = col[e], c1 = col[e + L], c2 = col[e + 2 * L], c3 = col[e + 3 * L];
+        const double a0 = val[e], a1 = val[e + L], a2 = val[e + 2 * L], a3 = val[e + 3 * L];
+        const double x0 = x[c0], x1 = x[c1], x2 = x[c2], x3 = x[c3];
+        s = __fma_rn(a0, x0, s);
+        s = __fma_rn(a1, x1, s);
+        s = __fma_rn(a2, x2, s);
+        s = __fma_rn(a3, x3, s);
+      }
+      for (; e < e1; e += L) s = __fma_rn(val[e], x[col[e]], s);
+    }
 #pragma unroll
-    for (int o = kLanes / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, kLanes);
-    if (i < n && sub == 0) {
+    for (int o = L / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, L);
+    if (i < r1 && sub == 0) {
       const double ri = __dsub_rn(b[i], s);
       r[i] = ri;
       acc += ri * ri;
     }
   }
+  return acc;
+}
+
+// r = b - A x for rows [blk*rpb, (blk+1)*rpb); partial[blk] = sum r_i^2.
+// HBM bound: each block takes about 12 entries per lane for its own rows
+// (rows of a 7-point stencil: one lane each).  Eight lanes for every row left
+// one of eight idle, three shuffles per row and one load in flight.
+__global__ void __launch_bounds__(kThreads)
+residual_partials(int n, int rpb, const long long *__restrict__ rp, const int *__restrict__ col,
+                  const double *__restrict__ val, const double *__restrict__ x,
+                  const double *__restrict__ b, double *__restrict__ r, double *__restrict__ partial) {
+  __shared__ double sh[kThreads / 32];
+  const int r0 = blockIdx.x * rpb;
+  const int r1 = n - r0 > rpb ? r0 + rpb : n;
+  const long long per = (rp[r1] - rp[r0]) / (r1 - r0);
+  double acc;
+  if (per <= 12) acc = block_rows<1>(r0, r1, rp, col, val, x, b, r);
+  else if (per <= 48) acc = block_rows<4>(r0, r1, rp, col, val, x, b, r);
+  else if (per <= 192) acc = block_rows<16>(r0, r1, rp, col, val, x, b, r);
+  else acc = block_rows<32>(r0, r1, rp, col, val, x, b, r);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
@@ -71,7 +101,80 @@ sum_partials_ordered(int np, const double *__restrict__ partial, double *__restr
   if (threadIdx.x == 0) *out = sh[0];
 }
 
-int blocks_for(int n) { return (n + kRowsPerBlock - 1) / kRowsPerBlock; }
+// rows per block: 1,024 for large systems; a quarter of that keeps more SMs
+// busy below about eight blocks per SM
+int rows_per_block(int n) { return n >= 1200 * kMaxRowsPerBlock ? kMaxRowsPerBlock : kMaxRowsPerBlock / 4; }
+int blocks_for(int n) {
+  const int rpb = rows_per_block(n);
+  return (int)(((long long)n + rpb - 1) / rpb);
+}
+
+// Scratch of dg_residual_csr: a memory pool of its own per device that keeps
+// up to kPoolKeep bytes between calls.  The default pool gives everything
+// back to the driver at each synchronisation, so that every call after one
+// paid for a new mapping: 231 us a call on a 128^3 matrix (440 us after a
+// synchronisation) against 63 us with the kept pool and the kernel above.  Allocation and release stay stream
+// ordered: any number of threads and streams may call at once.  The pool
+// belongs to the context (its id is kept beside it) and goes with it.
+constexpr unsigned long long kPoolKeep = 1ull << 20;  // 131,072 partial sums
+constexpr int kMaxDevices = 128;
+cudaError_t current_context_id(unsigned long long *id);
+
+struct ScratchPool {
+  cudaMemPool_t pool = nullptr;
+  unsigned long long ctx = 0;
+};
+ScratchPool g_pool[kMaxDevices];
+std::mutex g_mu;  // this table, the fixed scratch's and the driver entry points below
+
+cudaMemPool_t scratch_pool(int dev) {  // null: use the device's default pool
+  if (dev < 0 || dev >= kMaxDevices) return nullptr;
+  std::lock_guard<std::mutex> lk(g_mu);
+  unsigned long long ctx = 0;
+  if (current_context_id(&ctx) != cudaSuccess || ctx == 0) return nullptr;
+  ScratchPool &p = g_pool[dev];
+  if (p.pool && p.ctx == ctx) return p.pool;
+  p = ScratchPool{};
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  unsigned long long keep = kPoolKeep;
+  // another stream of this thread may be under capture: creating a pool must
+  // not count as an unsafe call of it
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t made = cudaMemPoolCreate(&pool, &props);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (made != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
+  p.pool = pool;
+  p.ctx = ctx;
+  return pool;
+}
+
+// stream-ordered scratch: from the kept pool of the stream's own device,
+// which must be the current one; while the stream is captured (and anywhere
+// else the pool cannot be had) from the default pool
+cudaError_t alloc_scratch(double **p, size_t bytes, cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  int cur = -1, dev = -1;
+  if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+      cudaGetDevice(&cur) == cudaSuccess && cudaStreamGetDevice(s, &dev) == cudaSuccess && cur == dev) {
+    cudaMemPool_t pool = scratch_pool(dev);
+    if (pool) {
+      if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, pool, s) == cudaSuccess) return cudaSuccess;
+      cudaGetLastError();
+    }
+  } else {
+    cudaGetLastError();
+  }
+  return cudaMallocAsync(p, bytes, s);
+}
 
 }  // namespace resid
 }  // namespace dg
@@ -84,8 +187,8 @@ extern "C" dg_status dg_residual_csr(int n, const long long *d_rowptr, const int
   cudaStream_t s = (cudaStream_t)cuda_stream;
   const int nb = blocks_for(n);
   double *partial = nullptr;
-  if (cudaMallocAsync(&partial, (size_t)nb * sizeof(double), s) != cudaSuccess) return DG_CUDA_ERROR;
-  residual_partials<<<nb, kThreads, 0, s>>>(n, d_rowptr, d_col, d_val, d_x, d_b, d_r, partial);
+  if (alloc_scratch(&partial, (size_t)nb * sizeof(double), s) != cudaSuccess) return DG_CUDA_ERROR;
+  residual_partials<<<nb, kThreads, 0, s>>>(n, rows_per_block(n), d_rowptr, d_col, d_val, d_x, d_b, d_r, partial);
   sum_partials_ordered<<<1, kThreads, 0, s>>>(nb, partial, d_norm2);
   cudaError_t e = cudaGetLastError();
   cudaFreeAsync(partial, s);
@@ -110,7 +213,7 @@ namespace dg {
 namespace resid {
 
 constexpr int kNoAllocMaxPartials = 65536;  // 512 KiB of doubles
-constexpr long long kNoAllocMaxRows = (long long)kNoAllocMaxPartials * kRowsPerBlock;  // 67,108,864
+constexpr long long kNoAllocMaxRows = (long long)kNoAllocMaxPartials * kMaxRowsPerBlock;  // 67,108,864
 
 static __device__ __align__(256) double g_noalloc_partials[kNoAllocMaxPartials];
 
@@ -121,10 +224,8 @@ static __device__ __align__(256) double g_noalloc_partials[kNoAllocMaxPartials];
 // cudaDeviceReset the device gets a new primary context, into which the
 // library's module (and the array) is loaded again, possibly elsewhere, so a
 // changed context id makes the next call look the address up again.
-constexpr int kMaxDevices = 128;
 static double *g_noalloc_ptr[kMaxDevices];
 static unsigned long long g_noalloc_ctx[kMaxDevices];
-static std::mutex g_noalloc_mu;
 
 // cuCtxGetCurrent / cuCtxGetId through the runtime's driver entry points,
 // so that the library does not link the driver library itself.
@@ -134,7 +235,7 @@ static ctx_get_current_fn g_ctx_get_current;
 static ctx_get_id_fn g_ctx_get_id;
 
 // The id of the calling thread's current context (0: none yet).
-static cudaError_t current_context_id(unsigned long long *id) {
+cudaError_t current_context_id(unsigned long long *id) {
   *id = 0;
   if (!g_ctx_get_current || !g_ctx_get_id) {
     cudaDriverEntryPointQueryResult q1, q2;
@@ -158,7 +259,7 @@ static cudaError_t noalloc_scratch(double **out) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> lk(g_noalloc_mu);
+  std::lock_guard<std::mutex> lk(g_mu);
   unsigned long long ctx = 0;
   e = current_context_id(&ctx);
   if (e != cudaSuccess) return e;
@@ -191,7 +292,7 @@ extern "C" dg_status dg_residual_csr_noalloc(int n, const long long *d_rowptr, c
   const int nb = blocks_for(n);
   // every partial of [0, nb) is written before it is read, so the contents
   // left by an earlier call need no clearing
-  residual_partials<<<nb, kThreads, 0, s>>>(n, d_rowptr, d_col, d_val, d_x, d_b, d_r, partial);
+  residual_partials<<<nb, kThreads, 0, s>>>(n, rows_per_block(n), d_rowptr, d_col, d_val, d_x, d_b, d_r, partial);
   sum_partials_ordered<<<1, kThreads, 0, s>>>(nb, partial, d_norm2);
   return cudaGetLastError() == cudaSuccess ? DG_OK : DG_CUDA_ERROR;
 }

@@ -32,19 +32,29 @@ constexpr int kVecThreads = 256;
 enum : int { ERR_NOT_SPD = 1, ERR_NAN = 2, ERR_BREAKDOWN = 4, ERR_WAIT = 8 };
 
 // one entry of a front's child list (child ci of f_children): the child's
-// relative-row map offset, update-vector offset and update-row count, for
-// the forward solves' right-hand-side assembly in one load
+// relative-row map offset, update-vector offset and update-row count
 struct ChildEdge {
   int64_t relmap, uoff;
   int rc, pad;
 };
 
-// the front of a large-front solve task, stored beside the task so that the
-// task's first E loads need one load of the task list only
-struct __align__(16) TaskFront {
+// What a solve reads about a front, in one load: beside each large-front
+// task, and per front for the small ones.  tab: per row of the front its
+// place in the first two children's update vectors (16 bits each, kNoChild:
+// none), so that the right-hand side is gathered in one round of loads; cu0,
+// cu1: those vectors.  Children beyond the second: ch_edge[ch2 .. ch2 + nch - 2).
+struct __align__(16) SolveFront {
   int m, k;
   int64_t e_off;
+  int64_t xo, xb;          // position of the first pivot, of the matrix's first row
+  int64_t rows;            // offset into MfView::rows
+  int64_t uoff;            // update vector
+  int64_t tab;             // offset into the child table
+  int64_t cu0, cu1;
+  int nch, ch2;
 };
+static_assert(sizeof(SolveFront) == 80, "five 16-byte loads");
+constexpr unsigned kNoChild = 0xffffu;
 
 struct MfView {  // device pointers of one multifrontal batch
   const int64_t *f_off;
@@ -58,6 +68,8 @@ struct MfView {  // device pointers of one multifrontal batch
   const int64_t *asm_tgt, *asm_sp, *asm_src;
   const int64_t *e_off;        // offset of the front's elimination matrix E (m x k, ld round4(m))
   const ChildEdge *ch_edge;    // per child-list entry: see ChildEdge
+  const SolveFront *sfront;    // per front: see SolveFront
+  const unsigned *ctab;        // child tables
 };
 
 __host__ __device__ __forceinline__ int round4(int x) { return (x + 3) & ~3; }
@@ -1036,6 +1048,10 @@ template <> struct Vec16<float> {
     const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
     o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
   }
+  __device__ static __forceinline__ void lds(const float *p, float *o) {
+    const float4 t = *reinterpret_cast<const float4 *>(p);
+    o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
+  }
 };
 template <> struct Vec16<double> {
   static constexpr int N = 2;
@@ -1043,12 +1059,14 @@ template <> struct Vec16<double> {
     const double2 t = __ldg(reinterpret_cast<const double2 *>(p));
     o[0] = t.x; o[1] = t.y;
   }
+  __device__ static __forceinline__ void lds(const double *p, double *o) {
+    const double2 t = *reinterpret_cast<const double2 *>(p);
+    o[0] = t.x; o[1] = t.y;
+  }
 };
 
 constexpr int kSolveSmall = 128;   // fronts of at most this many rows: one warp each
 constexpr int kEThreads = 256;
-constexpr int kELeanThreads = 128;
-constexpr int kEUnroll = 8;        // independent E loads in flight per thread
 
 // Small fronts are solved by groups of G lanes (G = 8, 16 or 32; 32 / G
 // fronts per warp): a front of at most 4G rows, lane l of its group holding
@@ -1083,15 +1101,14 @@ __device__ __forceinline__ void load_e_batch(const T *Ef, int ld, int m, int k, 
   }
 }
 
-// small fronts, forward: the first batch of E is loaded before the
-// right-hand side is assembled.  cta: this CTA's index within its bucket.
 // Programmatic dependent launch of the level solves.  pdl_trigger (at the
 // start of a CTA) lets the next kernel of the stream start its CTAs once
 // every CTA of this one has started; pdl_wait returns once the previous
 // kernel has completed and its writes are visible.  The solve bodies issue
 // their first loads of E (written by the factorisation, before any of these
-// kernels) and only then wait, before they read a vector that the previous
-// level wrote.  Without the launch attribute both instructions do nothing.
+// kernels) and read their index lists, and only then wait, before they read a
+// vector that the previous level wrote.  Without the launch attribute both
+// instructions do nothing.
 __device__ __forceinline__ void pdl_trigger() {
 #if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1103,10 +1120,25 @@ __device__ __forceinline__ void pdl_wait() {
 #endif
 }
 
+// x + the first two children's updates at a row (t: the row's child table
+// entry), children in order
+template <typename T>
+__device__ __forceinline__ T add_children(T x, unsigned t, const T *__restrict__ u, int64_t cu0, int64_t cu1) {
+  const unsigned t0 = t & 0xffffu, t1 = t >> 16;
+  const T a = t0 != kNoChild ? __ldcg(u + cu0 + t0) : T(0);
+  const T b = t1 != kNoChild ? __ldcg(u + cu1 + t1) : T(0);
+  if (t0 != kNoChild) x += a;
+  if (t1 != kNoChild) x += b;
+  return x;
+}
+
+// small fronts, forward: the first batch of E is loaded before the
+// right-hand side is assembled.  cta: this CTA's index within its bucket.
 template <typename T, int G>
 __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__restrict__ fronts, int nf,
                                                const T *__restrict__ E, const T *__restrict__ xl,
-                                               T *__restrict__ yl, T *__restrict__ uvec, int cta, T *wsh) {
+                                               T *__restrict__ yl, T *__restrict__ uvec, int cta,
+                                               T *wsh) {
   constexpr int VN = Vec16<T>::N, M = 4 * G, PASS = M / (G * VN), FPW = 32 / G;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int grp = lane / G, sl = lane % G;
@@ -1114,23 +1146,35 @@ __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__res
   const int gf = (cta * 8 + wid) * FPW + grp;
   if (gf >= nf) return;  // group-level work: no block barriers below
   T *w = wsh + (wid * FPW + grp) * M;
-  const int f = fronts[gf];
-  const int m = v.f_m[f], k = v.f_k[f], ld = round4(m);
-  const int64_t xo = v.f_xoff[f] + v.f_p0[f];
-  const T *Ef = E + v.e_off[f];
+  const SolveFront &f = v.sfront[fronts[gf]];
+  const int m = f.m, k = f.k, ld = round4(m), nch = f.nch;
+  const int64_t xo = f.xo, cu0 = f.cu0, cu1 = f.cu1;
+  const T *Ef = E + f.e_off;
   T e[PASS][kSmallUnroll][VN];
   load_e_batch<T, PASS, G>(Ef, ld, m, k, sl, 0, e);
-  // the child list is static: its first entry is read before the wait
-  const int cb = v.f_child_ptr[f], ce = v.f_child_ptr[f + 1];
-  ChildEdge ed = cb < ce ? v.ch_edge[cb] : ChildEdge{0, 0, 0, 0};
+  // the child table is static: read before the wait (a lane has at most 4 rows)
+  unsigned t[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) t[q] = nch && sl + q * G < m ? v.ctab[f.tab + sl + q * G] : ~0u;
   pdl_wait();
-  for (int i = sl; i < m; i += G) w[i] = i < k ? xl[xo + i] : T(0);
+#pragma unroll
+  for (int h = 0; h < 4; h += 2) {  // two rows at once: more do not fit the registers
+    T x[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int i = sl + (h + q) * G;
+      x[q] = add_children(i < k ? xl[xo + i] : T(0), t[h + q], uvec, cu0, cu1);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+      if (sl + (h + q) * G < m) w[sl + (h + q) * G] = x[q];
+    asm volatile("" ::: "memory");
+  }
   __syncwarp(gm);
-  for (int ci = cb; ci < ce; ci++) {
-    if (ci > cb) ed = v.ch_edge[ci];
+  for (int ci = 0; ci < nch - 2; ci++) {
+    const ChildEdge ed = v.ch_edge[f.ch2 + ci];
     const int *rel = v.relmap + ed.relmap;
-    const T *u = uvec + ed.uoff;
-    for (int a = sl; a < ed.rc; a += G) w[rel[a]] += __ldcg(u + a);
+    for (int a = sl; a < ed.rc; a += G) w[rel[a]] += __ldcg(uvec + ed.uoff + a);
     __syncwarp(gm);
   }
   T acc[PASS][VN];
@@ -1142,14 +1186,16 @@ __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__res
     if (j0 > 0) load_e_batch<T, PASS, G>(Ef, ld, m, k, sl, j0, e);
 #pragma unroll
     for (int u = 0; u < kSmallUnroll; u++) {
-      const T bj = j0 + u < k ? w[j0 + u] : T(0);
+      if (j0 + u >= k) break;
+      const T bj = w[j0 + u];
 #pragma unroll
       for (int p = 0; p < PASS; p++)
+        if (VN * sl + G * VN * p < m)  // (FP64: the pipe is the limit; no rows of padding)
 #pragma unroll
-        for (int q = 0; q < VN; q++) acc[p][q] += e[p][u][q] * bj;
+          for (int q = 0; q < VN; q++) acc[p][q] += e[p][u][q] * bj;
     }
   }
-  T *uf = uvec + v.f_uoff[f];
+  T *uf = uvec + f.uoff;
 #pragma unroll
   for (int p = 0; p < PASS; p++)
 #pragma unroll
@@ -1160,28 +1206,43 @@ __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__res
     }
 }
 
+// the sums over G lanes of four values per lane: every step halves the
+// values a lane still holds (5 additions a lane for G = 16, not 16); lane
+// G/4 * c .. of the group holds the sum of value c
+template <typename T, int G>
+__device__ __forceinline__ T reduce4(const T (&s)[4], int sl, unsigned gm) {
+  const bool hi = (sl & (G / 2)) != 0;
+  const T a0 = (hi ? s[2] : s[0]) + __shfl_xor_sync(gm, hi ? s[0] : s[2], G / 2);
+  const T a1 = (hi ? s[3] : s[1]) + __shfl_xor_sync(gm, hi ? s[1] : s[3], G / 2);
+  const bool h2 = (sl & (G / 4)) != 0;
+  T t = (h2 ? a1 : a0) + __shfl_xor_sync(gm, h2 ? a0 : a1, G / 4);
+#pragma unroll
+  for (int o = G / 8; o > 0; o >>= 1) t += __shfl_xor_sync(gm, t, o);
+  return t;
+}
+
 // small fronts, backward: the first batch of E is loaded before v is gathered
 template <typename T, int G>
 __device__ __forceinline__ void bwd_small_body(const MfView &v, const int *__restrict__ fronts, int nf,
                                                const T *__restrict__ E, const T *__restrict__ yl,
                                                T *__restrict__ xl, int cta, T *wsh) {
   constexpr int VN = Vec16<T>::N, M = 4 * G, PASS = M / (G * VN), FPW = 32 / G;
-  static_assert(G >= kSmallUnroll, "a group stores one column sum per lane");
+  static_assert(kSmallUnroll == 4, "four column sums are reduced together");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int grp = lane / G, sl = lane % G;
   const unsigned gm = group_mask<G>(lane);
   const int gf = (cta * 8 + wid) * FPW + grp;
   if (gf >= nf) return;
   T *w = wsh + (wid * FPW + grp) * M;
-  const int f = fronts[gf];
-  const int m = v.f_m[f], k = v.f_k[f], ld = round4(m);
-  const int64_t xo = v.f_xoff[f] + v.f_p0[f];
-  const T *Ef = E + v.e_off[f];
+  const SolveFront &f = v.sfront[fronts[gf]];
+  const int m = f.m, k = f.k, ld = round4(m);
+  const int64_t xo = f.xo;
+  const T *Ef = E + f.e_off;
   T e[PASS][kSmallUnroll][VN];
   load_e_batch<T, PASS, G>(Ef, ld, m, k, sl, 0, e);
   // the ancestor rows' positions are static: read before the wait (a lane
   // has at most 4 of the front's ld <= 4G rows)
-  const int *rows = v.rows + v.f_rows[f];
+  const int *rows = v.rows + f.rows;
   int rw[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -1189,7 +1250,7 @@ __device__ __forceinline__ void bwd_small_body(const MfView &v, const int *__res
     rw[q] = (i >= k && i < m) ? rows[i] : 0;
   }
   pdl_wait();
-  const T *xb = xl + v.f_xoff[f];
+  const T *xb = xl + f.xb;
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const int i = sl + q * G;
@@ -1201,29 +1262,25 @@ __device__ __forceinline__ void bwd_small_body(const MfView &v, const int *__res
   for (int p = 0; p < PASS; p++)
 #pragma unroll
     for (int q = 0; q < VN; q++) {
-      const int r = VN * sl + G * VN * p + q;
-      wr[p][q] = r < ld ? w[r] : T(0);
+      const int i = VN * sl + G * VN * p + q;
+      wr[p][q] = i < ld ? w[i] : T(0);
     }
-  // each column sum is reduced over the group; lane u of the batch keeps column u
   for (int c0 = 0; c0 < k; c0 += kSmallUnroll) {
     if (c0 > 0) load_e_batch<T, PASS, G>(Ef, ld, m, k, sl, c0, e);
     T s[kSmallUnroll];
 #pragma unroll
     for (int u = 0; u < kSmallUnroll; u++) {
       s[u] = T(0);
+      if (c0 + u < k)
 #pragma unroll
-      for (int p = 0; p < PASS; p++)
+        for (int p = 0; p < PASS; p++)
+          if (VN * sl + G * VN * p < m)
 #pragma unroll
-        for (int q = 0; q < VN; q++) s[u] += e[p][u][q] * wr[p][q];
-#pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) s[u] += __shfl_xor_sync(gm, s[u], o);
+            for (int q = 0; q < VN; q++) s[u] += e[p][u][q] * wr[p][q];
     }
-    if (sl < kSmallUnroll && c0 + sl < k) {
-      T out = s[0];
-#pragma unroll
-      for (int u = 1; u < kSmallUnroll; u++) if (sl == u) out = s[u];
-      xl[xo + c0 + sl] = out;
-    }
+    const T t = reduce4<T, G>(s, sl, gm);
+    const int c = c0 + sl / (G / 4);
+    if (sl % (G / 4) == 0 && c < k) xl[xo + c] = t;
   }
 }
 
@@ -1274,36 +1331,45 @@ mf_bwd_small(MfView v, const int *__restrict__ fronts, SmallBuckets sb, const T 
     bwd_small_body<T, 32>(v, fronts + sb.cnt0 + sb.cnt1, sb.cnt2, E, yl, xl, b - sb.nb0 - sb.nb1, wsh);
 }
 
-// large fronts, forward: task = {front, (first chunk << 16) | chunk count};
-// a chunk is FwdRows<T>::N rows.  The CTA assembles the front's whole
-// right-hand side b (m entries) once, then per chunk each warp takes every
-// 8th column of E and each lane VN rows (one coalesced 512-byte row segment
-// per warp and column); the 8 warp sums are added in a fixed order.
-// Pivot-row chunks need the columns j < min(k, r0 + N) only, and a vector
-// of rows wholly above the diagonal of E is zero and not loaded.
-template <typename T> struct FwdRows { static constexpr int N = 32 * Vec16<T>::N; };
+// Large fronts, forward: task = {front, (first chunk << 16) | chunk count}; a
+// chunk is LPR * VN rows.  The CTA assembles the part of the right-hand side
+// b that its chunks need (the pivots up to their last row, and their own
+// update rows) once, then per chunk every warp takes CW = 32 / LPR columns
+// of E at a time, LPR lanes of VN rows each; the warps' sums are added in a
+// fixed order.  Pivot-row chunks need the columns below their last row only,
+// and a vector of rows wholly above the diagonal of E is zero and not loaded.
+//
+// Variants (kFwdVariants, chosen per level): threads, E loads in flight per
+// thread and lanes per column.  The loads of one batch are issued together,
+// the first batch before the dependency wait; each further batch costs
+// another round to memory, so levels with few tasks take more threads and
+// shorter chunks until one batch holds a task, and levels with many take
+// 128-thread CTAs at high occupancy.
+struct FwdVariant { int nt, un, lpr, ctas; };  // ctas per SM (launch bounds)
+constexpr FwdVariant kFwdVariants[4] = {{128, 4, 32, 12}, {256, 8, 32, 4}, {256, 8, 16, 4}, {128, 8, 32, 7}};
+template <typename T, int LPR> __host__ __device__ constexpr int fwd_rows() { return LPR * Vec16<T>::N; }
 
-// the task body; b: shared memory for the front's right-hand side (m
-// values), red: the warp sums of one chunk
-template <typename T, int NT>
-__device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, TaskFront tf, const T *__restrict__ E,
+// the task body; b: shared memory for the right-hand side (at most the
+// front's rows), red: the warp sums of one chunk
+template <typename T, int NT, int UN, int LPR>
+__device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const SolveFront &f, const T *__restrict__ E,
                                              const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec,
-                                             T *b, T (*red)[FwdRows<T>::N]) {
-  constexpr int VN = Vec16<T>::N, RC = FwdRows<T>::N, NW = NT / 32, UN = NT == kELeanThreads ? 4 : kEUnroll;
-  const int f = tk.x;
+                                             T *b, T *red) {
+  constexpr int VN = Vec16<T>::N, RC = LPR * VN, NW = NT / 32, CW = 32 / LPR, STEP = NW * CW;
   const int ch0 = tk.y >> 16, nch = tk.y & 0xffff;
-  const int m = tf.m, k = tf.k, ld = round4(m);
-  const int64_t xo = v.f_xoff[f] + v.f_p0[f];
+  const int m = f.m, k = f.k, ld = round4(m), nc = f.nch;
+  const int64_t xo = f.xo, cu0 = f.cu0, cu1 = f.cu1, tab = f.tab;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const T *Ef = E + tf.e_off;
-  // one batch: columns j + u*NW (u < UN) of the chunk's rows of this lane;
+  const int sl = lane % LPR, j0 = wid * CW + lane / LPR;
+  const T *Ef = E + f.e_off;
+  // one batch: columns j + u*STEP (u < UN) of the chunk's rows of this lane;
   // a vector wholly above E's diagonal (rb + VN <= column) is zero
   T e[UN][VN];
   auto load_batch = [&](int r0, int K, int j) {
-    const int rb = r0 + lane * VN;
+    const int rb = r0 + sl * VN;
 #pragma unroll
     for (int u = 0; u < UN; u++) {
-      const int jj = j + u * NW;
+      const int jj = j + u * STEP;
       if (rb < m && jj < K && rb + VN > jj) Vec16<T>::load(Ef + (int64_t)jj * ld + rb, e[u]);
       else {
 #pragma unroll
@@ -1312,91 +1378,124 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, TaskFront
     }
   };
   auto chunk_cols = [&](int r0) { return r0 < k ? min(k, r0 + RC) : k; };
-  load_batch(ch0 * RC, chunk_cols(ch0 * RC), wid);  // in flight while b is assembled
-  // the child list is static: its first entry is read before the wait, and
-  // each entry's successor while the entry is added
-  const int cb = v.f_child_ptr[f], ce = v.f_child_ptr[f + 1];
-  ChildEdge ed = cb < ce ? v.ch_edge[cb] : ChildEdge{0, 0, 0, 0};
-  pdl_wait();
-  for (int i = tid; i < m; i += NT) b[i] = i < k ? xl[xo + i] : T(0);
-  __syncthreads();
-  for (int ci = cb; ci < ce; ci++) {
-    const ChildEdge nx = ci + 1 < ce ? v.ch_edge[ci + 1] : ed;
-    const int *rel = v.relmap + ed.relmap;
-    const T *u = uvec + ed.uoff;
-    for (int a = tid; a < ed.rc; a += NT) b[rel[a]] += __ldcg(u + a);
-    __syncthreads();
-    ed = nx;
+  load_batch(ch0 * RC, chunk_cols(ch0 * RC), j0);  // in flight while b is assembled
+  // rows of b: pivots [0, kn), then update rows [rlo, rhi); the child table
+  // is static, its entries of this thread's first rows are read before the wait
+  const int kn = min(k, (ch0 + nch) * RC), rlo = max(k, ch0 * RC), rhi = min(m, (ch0 + nch) * RC);
+  const int nrow = kn + max(0, rhi - rlo);
+  constexpr int NP = NT == 128 && UN == 4 ? 2 : 4;
+  unsigned t[NP];
+#pragma unroll
+  for (int q = 0; q < NP; q++) {
+    const int i = tid + q * NT;
+    t[q] = nc && i < nrow ? v.ctab[tab + (i < kn ? i : rlo + i - kn)] : ~0u;
   }
-  T *uf = uvec + v.f_uoff[f];
+  pdl_wait();
+  T x[NP];
+#pragma unroll
+  for (int q = 0; q < NP; q++) {
+    const int i = tid + q * NT;
+    x[q] = add_children(i < kn ? xl[xo + i] : T(0), t[q], uvec, cu0, cu1);
+  }
+#pragma unroll
+  for (int q = 0; q < NP; q++)
+    if (tid + q * NT < nrow) b[tid + q * NT] = x[q];
+  for (int i = tid + NP * NT; i < nrow; i += NT)
+    b[i] = add_children(i < kn ? xl[xo + i] : T(0),
+                        nc ? v.ctab[tab + (i < kn ? i : rlo + i - kn)] : ~0u, uvec, cu0, cu1);
+  __syncthreads();
+  for (int ci = 0; ci < nc - 2; ci++) {  // children beyond the second, in order
+    const ChildEdge ed = v.ch_edge[f.ch2 + ci];
+    const int *rel = v.relmap + ed.relmap;
+    for (int a = tid; a < ed.rc; a += NT) {
+      const int row = rel[a], i = row < kn ? row : row >= rlo && row < rhi ? kn + row - rlo : -1;
+      if (i >= 0) b[i] += __ldcg(uvec + ed.uoff + a);
+    }
+    __syncthreads();
+  }
   for (int ch = ch0; ch < ch0 + nch; ch++) {
     const int r0 = ch * RC;
     const int K = chunk_cols(r0);
     T acc[VN];
 #pragma unroll
     for (int q = 0; q < VN; q++) acc[q] = T(0);
-    for (int j = wid; j < K; j += UN * NW) {
-      if (j != wid) load_batch(r0, K, j);  // every chunk's first batch was loaded ahead
+    for (int jw = wid * CW; jw < K; jw += UN * STEP) {
+      const int j = jw + lane / LPR;
+      if (jw != wid * CW) load_batch(r0, K, j);  // every chunk's first batch was loaded ahead
 #pragma unroll
       for (int u = 0; u < UN; u++) {
-        const int jj = j + u * NW;
-        const T bj = jj < K ? b[jj] : T(0);  // b holds rows [0, m): columns past K are not read
+        if (jw + u * STEP >= K) break;  // (warp-uniform: no multiplications of padding columns)
+        const T bj = j + u * STEP < K ? b[j + u * STEP] : T(0);
 #pragma unroll
         for (int q = 0; q < VN; q++) acc[q] += e[u][q] * bj;
       }
     }
     // the next chunk's first batch is in flight during this chunk's reduction
-    if (ch + 1 < ch0 + nch) load_batch((ch + 1) * RC, chunk_cols((ch + 1) * RC), wid);
+    if (ch + 1 < ch0 + nch) load_batch((ch + 1) * RC, chunk_cols((ch + 1) * RC), j0);
 #pragma unroll
-    for (int q = 0; q < VN; q++) red[wid][lane * VN + q] = acc[q];
+    for (int o = LPR; o < 32; o <<= 1)
+#pragma unroll
+      for (int q = 0; q < VN; q++) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+    if (lane < LPR)
+#pragma unroll
+      for (int q = 0; q < VN; q++) red[wid * RC + sl * VN + q] = acc[q];
     __syncthreads();
-    for (int t = tid; t < RC; t += NT) {
-      T s = T(0);
-#pragma unroll
-      for (int w = 0; w < NW; w++) s += red[w][t];
-      const int row = r0 + t;
+    const int nw = min(NW, (K + CW - 1) / CW);  // warps that had columns
+    for (int i = tid; i < RC; i += NT) {
+      const int row = r0 + i;
+      T s = red[i];
+      for (int w = 1; w < nw; w++) s += red[w * RC + i];
       if (row < k) yl[xo + row] = s;
-      else if (row < m) uf[row - k] = b[row] + s;
+      else if (row < m) uvec[f.uoff + row - k] = b[kn + row - rlo] + s;
     }
     __syncthreads();
   }
 }
 
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT, NT == kELeanThreads ? 12 : 4)
-mf_fwd_big(MfView v, const int2 *__restrict__ tasks, const TaskFront *__restrict__ tmeta, const T *__restrict__ E,
+template <typename T, int V>
+__global__ void __launch_bounds__(kFwdVariants[V].nt, kFwdVariants[V].ctas)
+mf_fwd_big(MfView v, const int2 *__restrict__ tasks, const SolveFront *__restrict__ tmeta, const T *__restrict__ E,
            const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec, int nrhs = 1, int64_t xs = 0,
            int64_t us = 0) {
+  constexpr FwdVariant fv = kFwdVariants[V];
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ T red[NT / 32][FwdRows<T>::N];
+  __shared__ T red[fv.nt / 32 * fwd_rows<T, fv.lpr>()];
   pdl_trigger();
   const int task = blockIdx.x / nrhs, rk = blockIdx.x % nrhs;
-  fwd_big_body<T, NT>(v, tasks[task], tmeta[task], E, xl + rk * xs, yl + rk * xs, uvec + rk * us,
-                      reinterpret_cast<T *>(smem_raw), red);
+  fwd_big_body<T, fv.nt, fv.un, fv.lpr>(v, tasks[task], tmeta[task], E, xl + rk * xs, yl + rk * xs, uvec + rk * us,
+                                        reinterpret_cast<T *>(smem_raw), red);
 }
 
-// large fronts, backward: task = {front, column block J}; x[32J .. 32J+31] from
-// rows [32J, m) of E
-template <typename T, int NT>
-__device__ __forceinline__ void bwd_big_body(const MfView &v, int2 tk, TaskFront tf, const T *__restrict__ E,
+// Large fronts, backward: task = {front, column block J} of CB columns; x of
+// the block from rows [CB J, m) of E.  LPC lanes per column, NT / LPC columns
+// at once.  Variants as in the forward: threads, loads in flight, columns.
+struct BwdVariant { int nt, un, cb, ctas; };
+constexpr BwdVariant kBwdVariants[4] = {{128, 4, 32, 12}, {256, 8, 32, 4}, {256, 8, 16, 4}, {128, 8, 16, 7}};
+
+template <typename T, int NT, int UN, int CB>
+__device__ __forceinline__ void bwd_big_body(const MfView &v, int2 tk, const SolveFront &f, const T *__restrict__ E,
                                              const T *__restrict__ yl, T *__restrict__ xl, T *w) {
-  constexpr int VN = Vec16<T>::N, LPC = 32 / VN, NCS = NT / LPC, UN = NT == kELeanThreads ? 4 : kEUnroll;
-  const int f = tk.x, J = tk.y;
-  const int m = tf.m, k = tf.k, ld = round4(m);
-  const int c0 = 32 * J, jb = min(32, k - c0);
-  const int64_t xo = v.f_xoff[f] + v.f_p0[f];
-  const T *xb = xl + v.f_xoff[f];
-  const int *rows = v.rows + v.f_rows[f];
+  constexpr int VN = Vec16<T>::N;
+  // lanes per column: a 32-row vector's worth, twice that where the CTA has
+  // more lanes than the block's columns need
+  constexpr int LPC = NT / CB > 32 ? 32 : NT / CB > 32 / VN ? NT / CB : 32 / VN, NCS = NT / LPC, RS = LPC * VN;
+  const int J = tk.y;
+  const int m = f.m, k = f.k, ld = round4(m);
+  const int c0 = CB * J, jb = min(CB, k - c0);
+  const int64_t xo = f.xo;
+  const T *xb = xl + f.xb;
+  const int *rows = v.rows + f.rows;
   const int tid = threadIdx.x;
   const int rq = tid % LPC, cs = tid / LPC;
-  // one batch: rows i + 32u (u < UN) of column c for this lane; a vector
+  // one batch: rows i + RS*u (u < UN) of column c for this lane; a vector
   // wholly above E's diagonal (i + VN <= c) is zero
   T e[UN][VN];
+  const T *E0 = E + f.e_off;
   auto load_batch = [&](int c, int i) {
-    const T *Ec = E + tf.e_off + (int64_t)c * ld;
+    const T *Ec = E0 + (int64_t)c * ld;
 #pragma unroll
     for (int u = 0; u < UN; u++) {
-      const int ii = i + u * 32;
+      const int ii = i + u * RS;
       if (c - c0 < jb && ii < m && ii + VN > c) Vec16<T>::load(Ec + ii, e[u]);
       else {
 #pragma unroll
@@ -1415,6 +1514,7 @@ __device__ __forceinline__ void bwd_big_body(const MfView &v, int2 tk, TaskFront
     rw[q] = (i >= k && i < m) ? rows[i] : 0;
   }
   pdl_wait();
+  const int nrow = ld - c0;
 #pragma unroll
   for (int q = 0; q < kRowsAhead; q++) {
     const int i = c0 + tid + q * NT;
@@ -1423,38 +1523,42 @@ __device__ __forceinline__ void bwd_big_body(const MfView &v, int2 tk, TaskFront
   for (int i = c0 + tid + kRowsAhead * NT; i < ld; i += NT)
     w[i - c0] = i < k ? yl[xo + i] : (i < m ? __ldcg(xb + rows[i]) : T(0));
   __syncthreads();
-  for (int cc = cs; cc < 32; cc += NCS) {  // uniform trip count: the shuffles below need whole groups
+  for (int cc = cs; cc < CB; cc += NCS) {  // uniform trip count: the shuffles below need whole groups
     const int c = c0 + cc;
     T s = T(0);
     if (cc < jb) {
-      for (int i = c0 + rq * VN; i < m; i += UN * 32) {
+      for (int i = c0 + rq * VN; i < m; i += UN * RS) {
         if (i != c0 + rq * VN) load_batch(c, i);  // every column's first batch was loaded ahead
 #pragma unroll
         for (int u = 0; u < UN; u++) {
-          const int ii = i + u * 32;  // w holds rows [c0, ld): rows past m are not read
+          const int ii = i + u * RS;  // w holds rows [c0, ld): rows past m are not read
           if (ii < m) {
+            T x[VN];
+            Vec16<T>::lds(w + ii - c0, x);
 #pragma unroll
-            for (int q = 0; q < VN; q++) s += e[u][q] * w[ii + q - c0];
+            for (int q = 0; q < VN; q++) s += e[u][q] * x[q];
           }
         }
       }
     }
     // the next column's first batch is in flight during this column's reduction
-    if (cc + NCS < 32) load_batch(c + NCS, c0 + rq * VN);
+    if (cc + NCS < CB) load_batch(c + NCS, c0 + rq * VN);
 #pragma unroll
     for (int o = LPC / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (rq == 0 && cc < jb) xl[xo + c] = s;
   }
 }
 
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT, NT == kELeanThreads ? 12 : 4)
-mf_bwd_big(MfView v, const int2 *__restrict__ tasks, const TaskFront *__restrict__ tmeta, const T *__restrict__ E,
+template <typename T, int V>
+__global__ void __launch_bounds__(kBwdVariants[V].nt, kBwdVariants[V].ctas)
+mf_bwd_big(MfView v, const int2 *__restrict__ tasks, const SolveFront *__restrict__ tmeta, const T *__restrict__ E,
            const T *__restrict__ yl, T *__restrict__ xl, int nrhs = 1, int64_t xs = 0) {
+  constexpr BwdVariant bv = kBwdVariants[V];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_trigger();
   const int task = blockIdx.x / nrhs, rk = blockIdx.x % nrhs;
-  bwd_big_body<T, NT>(v, tasks[task], tmeta[task], E, yl + rk * xs, xl + rk * xs, reinterpret_cast<T *>(smem_raw));
+  bwd_big_body<T, bv.nt, bv.un, bv.cb>(v, tasks[task], tmeta[task], E, yl + rk * xs, xl + rk * xs,
+                                       reinterpret_cast<T *>(smem_raw));
 }
 
 // ---------------------------------------------------------------------------
@@ -1515,11 +1619,11 @@ template <typename T>
 __global__ void __launch_bounds__(256, 4)
 mf_fwd_queue(MfView v, QueueView q, const int *__restrict__ small_fronts, const int *__restrict__ lvl_small_off,
              const SmallBuckets *__restrict__ lvl_sb, const int2 *__restrict__ fwd_tasks,
-             const TaskFront *__restrict__ fwd_tmeta, const T *__restrict__ E,
+             const SolveFront *__restrict__ fwd_tmeta, const T *__restrict__ E,
              const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec, int *counter, int *done,
              int *status, int nrhs = 1, int64_t xs = 0, int64_t us = 0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ T red[8][FwdRows<T>::N];
+  __shared__ T red[8 * fwd_rows<T, 32>()];
   __shared__ int s_g;
   T *sm = reinterpret_cast<T *>(smem_raw);
   const int total = q.ntasks * nrhs;
@@ -1539,10 +1643,11 @@ mf_fwd_queue(MfView v, QueueView q, const int *__restrict__ small_fronts, const 
       const int *fr = small_fronts + lvl_small_off[tk.y];
       const int b = tk.z;
       if (b < sb.nb0) fwd_small_body<T, 8>(v, fr, sb.cnt0, E, xk, yk, uk, b, sm);
-      else if (b < sb.nb0 + sb.nb1) fwd_small_body<T, 16>(v, fr + sb.cnt0, sb.cnt1, E, xk, yk, uk, b - sb.nb0, sm);
+      else if (b < sb.nb0 + sb.nb1)
+        fwd_small_body<T, 16>(v, fr + sb.cnt0, sb.cnt1, E, xk, yk, uk, b - sb.nb0, sm);
       else fwd_small_body<T, 32>(v, fr + sb.cnt0 + sb.cnt1, sb.cnt2, E, xk, yk, uk, b - sb.nb0 - sb.nb1, sm);
     } else {
-      fwd_big_body<T, 256>(v, fwd_tasks[tk.z], fwd_tmeta[tk.z], E, xk, yk, uk, sm, red);
+      fwd_big_body<T, 256, 8, 32>(v, fwd_tasks[tk.z], fwd_tmeta[tk.z], E, xk, yk, uk, sm, red);
     }
     __syncthreads();
     if (threadIdx.x == 0) queue_publish<T>(q, done, g);
@@ -1553,7 +1658,7 @@ template <typename T>
 __global__ void __launch_bounds__(256, 4)
 mf_bwd_queue(MfView v, QueueView q, const int *__restrict__ small_fronts, const int *__restrict__ lvl_small_off,
              const SmallBuckets *__restrict__ lvl_sb, const int2 *__restrict__ bwd_tasks,
-             const TaskFront *__restrict__ bwd_tmeta, const T *__restrict__ E,
+             const SolveFront *__restrict__ bwd_tmeta, const T *__restrict__ E,
              const T *__restrict__ yl, T *__restrict__ xl, int *counter, int *done, int *status, int nrhs = 1,
              int64_t xs = 0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1576,10 +1681,11 @@ mf_bwd_queue(MfView v, QueueView q, const int *__restrict__ small_fronts, const 
       const int *fr = small_fronts + lvl_small_off[tk.y];
       const int b = tk.z;
       if (b < sb.nb0) bwd_small_body<T, 8>(v, fr, sb.cnt0, E, yk, xk, b, sm);
-      else if (b < sb.nb0 + sb.nb1) bwd_small_body<T, 16>(v, fr + sb.cnt0, sb.cnt1, E, yk, xk, b - sb.nb0, sm);
+      else if (b < sb.nb0 + sb.nb1)
+        bwd_small_body<T, 16>(v, fr + sb.cnt0, sb.cnt1, E, yk, xk, b - sb.nb0, sm);
       else bwd_small_body<T, 32>(v, fr + sb.cnt0 + sb.cnt1, sb.cnt2, E, yk, xk, b - sb.nb0 - sb.nb1, sm);
     } else {
-      bwd_big_body<T, 256>(v, bwd_tasks[tk.z], bwd_tmeta[tk.z], E, yk, xk, sm);
+      bwd_big_body<T, 256, 8, 32>(v, bwd_tasks[tk.z], bwd_tmeta[tk.z], E, yk, xk, sm);
     }
     __syncthreads();
     if (threadIdx.x == 0) queue_publish<T>(q, done, g);

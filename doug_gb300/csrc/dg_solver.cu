@@ -112,8 +112,10 @@ template <typename T>
 struct MfDevice {
   DBuf<int64_t> f_off, f_rows, f_xoff, f_uoff, f_woff, f_relmap, f_asm, asm_tgt, asm_sp, asm_src, e_off;
   DBuf<ChildEdge> ch_edge;
+  DBuf<SolveFront> sfront;
+  DBuf<unsigned> ctab;
   DBuf<int> f_m, f_k, f_p0, f_child_ptr, f_children, rows, relmap, lvl_fronts, gidx;
-  DBuf<int> pan_fronts, diag_fronts, solve_small;
+  DBuf<int> pan_fronts, diag_fronts;
   int tiny_threads = 64;
   int tensor_update = 1;   // FP32 super-panel updates: 1 tcgen05 + TMEM, 0 mma.sync
   long long q_wait_cycles = kQueueWaitCycles;  // queue schedule: limit of one dependency wait
@@ -140,8 +142,7 @@ struct MfDevice {
   DBuf<SmallBuckets> q_sb;
   int qf_n = 0, qb_n = 0, q_grid = 0, q_k = 0;
   size_t q_smem = 0;
-  DBuf<int2> asm_tasks, upd_tasks, panel_tasks, esc_tasks, etile_tasks, fwd_tasks, bwd_tasks;
-  DBuf<TaskFront> fwd_tmeta, bwd_tmeta;  // each solve task's front (m, k, E offset)
+  DBuf<int2> asm_tasks, upd_tasks, panel_tasks, esc_tasks, etile_tasks;
   DBuf<T> arena, E, xl, yl, u;
   int64_t e_len = 0;
   // per level: small-front range, assembly-task range, steps
@@ -168,10 +169,21 @@ struct MfDevice {
     SmallBuckets sb;
     int fwd_off, fwd_cnt, bwd_off, bwd_cnt;
     size_t fwd_smem, bwd_smem;
-    bool fwd_lean, bwd_lean;      // 128-thread CTAs for levels of small tasks
+    int fwd_v, bwd_v;             // kFwdVariants, kBwdVariants
   };
-  std::vector<SolveLevel> slevels;
-  int nlevels = 0, nfronts = 0;
+  // the solves' work lists: of one right-hand side, of several (planned for
+  // their number)
+  struct SolveLists {
+    std::vector<SolveLevel> levels;
+    DBuf<int> small;
+    DBuf<int2> fwd, bwd;
+    DBuf<SolveFront> fmeta, bmeta;  // each task's front
+  };
+  SolveLists one, many;
+  std::vector<SolveFront> sf;      // per front
+  const MfBatch *batch = nullptr;  // outlives this object
+  MfTune tune_;
+  int nlevels = 0, nfronts = 0, nsm = 1;
   int64_t xlen = 0;
   MfView view{};
 
@@ -214,9 +226,10 @@ struct MfDevice {
     mk = 0;
     view = MfView{f_off.p, f_m.p, f_k.p, f_rows.p, f_xoff.p, f_p0.p, f_uoff.p, f_woff.p,
                   f_child_ptr.p, f_children.p, f_relmap.p, f_asm.p, rows.p, relmap.p,
-                  asm_tgt.p, asm_sp.p, asm_src.p, e_off.p, ch_edge.p};
+                  asm_tgt.p, asm_sp.p, asm_src.p, e_off.p, ch_edge.p, nullptr, nullptr};
     int dev = 0, optin = 0;
     CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     // work lists of the factorisation
     std::vector<int> pn, df;
@@ -328,66 +341,149 @@ struct MfDevice {
     asm_tasks.upload(at);
     upd_tasks.upload(ut);
     etile_tasks.upload(et);
-    // solve work lists: warp kernels for the small fronts; one task per 32-row
-    // block (forward) and per 32-column block (backward) of the others, the
-    // longest first
+    // what the solves read about a front, and its child table
+    sf.assign((size_t)nfronts, SolveFront());
+    std::vector<unsigned> ct;
+    for (int f = 0; f < nfronts; f++) {
+      const int m = B.f_m[(size_t)f], cb = B.f_child_ptr[(size_t)f], nch = B.f_child_ptr[(size_t)f + 1] - cb;
+      SolveFront &S = sf[(size_t)f];
+      S = SolveFront{m, B.f_k[(size_t)f], eo[(size_t)f], B.f_xoff[(size_t)f] + B.f_p0[(size_t)f], B.f_xoff[(size_t)f],
+                     B.f_rows[(size_t)f], B.f_uoff[(size_t)f], (int64_t)ct.size(), 0, 0, nch, cb + 2};
+      if (nch == 0) continue;
+      ct.resize(ct.size() + (size_t)m, ~0u);
+      bool wide = false;  // an update vector beyond 16-bit places: its front's children all go row by row
+      for (int h = 0; h < std::min(nch, 2); h++) {
+        const int c = B.f_children[(size_t)(cb + h)];
+        wide |= B.f_m[(size_t)c] - B.f_k[(size_t)c] >= (int)kNoChild;
+      }
+      if (wide) {
+        S.nch = nch + 2;
+        S.ch2 = cb;
+        continue;
+      }
+      for (int h = 0; h < std::min(nch, 2); h++) {
+        const int c = B.f_children[(size_t)(cb + h)], rc = B.f_m[(size_t)c] - B.f_k[(size_t)c];
+        (h ? S.cu1 : S.cu0) = B.f_uoff[(size_t)c];
+        for (int q = 0; q < rc; q++) {
+          unsigned &t = ct[(size_t)(S.tab + B.relmap[(size_t)(B.f_relmap[(size_t)c] + q)])];
+          t = h ? (t & 0xffffu) | (unsigned)q << 16 : (t & 0xffff0000u) | (unsigned)q;
+        }
+      }
+    }
+    sfront.upload(sf);
+    ctab.upload(ct);
+    view.sfront = sfront.p;
+    view.ctab = ctab.p;
+    queue = tune.schedule == 1;
+    batch = &B;
+    tune_ = tune;
     std::vector<int> ss;
     std::vector<int2> fw, bw;
-    std::vector<TaskFront> fwm, bwm;
-    size_t fwd_smem_max = 0, bwd_smem_max = 0;
-    slevels.assign((size_t)nlevels, SolveLevel());
+    const size_t smem_max = plan_solves(1, one, ss, fw, bw);
+    set_solve_attrs<0>(optin, smem_max);
+    set_solve_attrs<1>(optin, smem_max);
+    set_solve_attrs<2>(optin, smem_max);
+    set_solve_attrs<3>(optin, smem_max);
+    pdl = tune.pdl == 1;
+    overlap = tune.factor_overlap == 1;
+    tiny_threads = tune.tiny_threads;
+    tensor_update = tune.tensor_update;
+    q_wait_cycles = tune.queue_wait_cycles;
+    q_skip_publish = tune.queue_skip_publish;
+    if constexpr (sizeof(T) == 4)
+      if (tensor_update == 1)
+        CK(cudaFuncSetAttribute(mf_update_big_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
+    if (queue) plan_queue(B, ss, fw, bw, smem_max);
+  }
+
+  // Solve work lists for K right-hand sides: warp kernels for the
+  // small fronts; runs of row chunks (forward) and column blocks (backward)
+  // of the others, the longest first.  Returns the shared memory of the
+  // largest front's vector.
+  size_t plan_solves(int K, SolveLists &out, std::vector<int> &ss, std::vector<int2> &fw, std::vector<int2> &bw) {
+    const MfBatch &B = *batch;
+    const MfTune &tune = tune_;
+    size_t smem_max = 0;
+    out.levels.assign((size_t)nlevels, SolveLevel());
     for (int l = 0; l < nlevels; l++) {
-      SolveLevel &L = slevels[(size_t)l];
+      SolveLevel &L = out.levels[(size_t)l];
       std::vector<std::pair<int, int>> sm[3];  // (k, front) per bucket
       L.fwd_off = (int)fw.size();
       L.bwd_off = (int)bw.size();
       L.fwd_smem = L.bwd_smem = 0;
-      std::vector<std::pair<int, int2>> fl, bl;
-      int64_t fwd_bytes = 0, bwd_bytes = 0;
       // a level with few small fronts solves them with the CTA-per-task
       // kernels too: a group of lanes per front leaves the GPU nearly idle
       // while it walks the columns of a large-k front
       int nsmall = 0;
       for (int q = B.lvl_ptr[(size_t)l]; q < B.lvl_ptr[(size_t)l + 1]; q++)
         nsmall += B.f_m[(size_t)B.lvl_fronts[(size_t)q]] <= kSolveSmall;
-      const bool thin = nsmall < tune.small_min_fronts;
+      const bool thin = (int64_t)nsmall * K < tune.small_min_fronts;
+      std::vector<int> large;
       for (int q = B.lvl_ptr[(size_t)l]; q < B.lvl_ptr[(size_t)l + 1]; q++) {
-        int f = B.lvl_fronts[(size_t)q];
-        int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
+        const int f = B.lvl_fronts[(size_t)q], m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
         if (m <= kSolveSmall && !thin) { sm[m <= 32 ? 0 : m <= 64 ? 1 : 2].push_back({k, f}); continue; }
-        // forward tasks: runs of row chunks of at least tune.fwd_task_bytes of E each
-        const int RC = FwdRows<T>::N, nch = (m + RC - 1) / RC;
-        for (int c = 0; c < nch;) {
-          int c1 = c;
-          int64_t bytes = 0;
-          do {
-            const int r0 = c1 * RC, K = r0 < k ? std::min(k, r0 + RC) : k;
-            bytes += (int64_t)RC * K * (int64_t)sizeof(T);
-            c1++;
-          } while (c1 < nch && bytes < tune.fwd_task_bytes);
-          fl.push_back({(int)std::min<int64_t>(bytes, 1 << 30), make_int2(f, (c << 16) | (c1 - c))});
-          fwd_bytes += bytes;
-          c = c1;
-        }
-        for (int J = 0; 32 * J < k; J++) {
-          bl.push_back({m - 32 * J, make_int2(f, J)});
-          bwd_bytes += (int64_t)32 * (m - 32 * J) * (int64_t)sizeof(T);
-        }
+        large.push_back(f);
         L.fwd_smem = std::max(L.fwd_smem, (size_t)round4(m) * sizeof(T));
         L.bwd_smem = std::max(L.bwd_smem, (size_t)round4(m) * sizeof(T));
+      }
+      // tasks of a variant: (size, task), and their bytes of E
+      auto fwd_plan = [&](int v, int64_t task_bytes, int64_t &total) {
+        std::vector<std::pair<int, int2>> t;
+        const int RC = kFwdVariants[v].lpr * Vec16<T>::N;
+        total = 0;
+        for (int f : large) {
+          const int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f], nch = (m + RC - 1) / RC;
+          for (int c = 0; c < nch;) {
+            int c1 = c;
+            int64_t bytes = 0;
+            do {
+              const int r0 = c1 * RC, K = r0 < k ? std::min(k, r0 + RC) : k;
+              bytes += (int64_t)RC * K * (int64_t)sizeof(T);
+              c1++;
+            } while (c1 < nch && bytes < task_bytes);
+            t.push_back({(int)std::min<int64_t>(bytes, 1 << 30), make_int2(f, (c << 16) | (c1 - c))});
+            total += bytes;
+            c = c1;
+          }
+        }
+        return t;
+      };
+      auto bwd_plan = [&](int v, int64_t &total) {
+        std::vector<std::pair<int, int2>> t;
+        const int CB = kBwdVariants[v].cb;
+        total = 0;
+        for (int f : large) {
+          const int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
+          for (int J = 0; CB * J < k; J++) {
+            t.push_back({m - CB * J, make_int2(f, J)});
+            total += (int64_t)CB * (m - CB * J) * (int64_t)sizeof(T);
+          }
+        }
+        return t;
+      };
+      // Which variant: where one wave of short tasks holds the level (four
+      // 256-thread CTAs per SM), the shortest chain of loads per task; else
+      // 256-thread CTAs for long tasks (lean_task_bytes and more on average)
+      // and 128-thread CTAs for short ones, with eight loads in flight while
+      // one wave holds them, four at the highest occupancy beyond.
+      int64_t fb = 0, bb = 0, sb = 0;
+      std::vector<std::pair<int, int2>> fl = fwd_plan(1, tune.fwd_task_bytes, fb), bl = bwd_plan(1, bb);
+      L.fwd_v = L.bwd_v = 1;
+      if (!large.empty() && !queue) {
+        auto sl = fwd_plan(2, 1, sb);
+        if ((int64_t)sl.size() * K <= 4 * nsm) { fl.swap(sl); L.fwd_v = 2; }
+        else if (fb / (int64_t)fl.size() < tune.lean_task_bytes) L.fwd_v = (int64_t)fl.size() * K <= kFwdVariants[3].ctas * nsm ? 3 : 0;
+        sl = bwd_plan(2, sb);
+        if ((int64_t)sl.size() * K <= 4 * nsm) { bl.swap(sl); L.bwd_v = 2; }
+        else if (bb / (int64_t)bl.size() < tune.lean_task_bytes) {
+          if ((int64_t)sl.size() * K <= kBwdVariants[3].ctas * nsm) { bl.swap(sl); L.bwd_v = 3; }
+          else L.bwd_v = 0;
+        }
       }
       std::stable_sort(fl.begin(), fl.end(), [](const std::pair<int, int2> &a, const std::pair<int, int2> &b) { return a.first > b.first; });
       std::stable_sort(bl.begin(), bl.end(), [](const std::pair<int, int2> &a, const std::pair<int, int2> &b) { return a.first > b.first; });
       for (auto &e : fl) fw.push_back(e.second);
       for (auto &e : bl) bw.push_back(e.second);
-      for (auto &e : fl) {
-        const int f = e.second.x;
-        fwm.push_back(TaskFront{B.f_m[(size_t)f], B.f_k[(size_t)f], eo[(size_t)f]});
-      }
-      for (auto &e : bl) {
-        const int f = e.second.x;
-        bwm.push_back(TaskFront{B.f_m[(size_t)f], B.f_k[(size_t)f], eo[(size_t)f]});
-      }
       // fronts of similar pivot counts share a warp
       L.small_off = (int)ss.size();
       int cnt[3];
@@ -402,42 +498,33 @@ struct MfDevice {
       L.small_cta = L.sb.nb0 + L.sb.nb1 + (cnt[2] + 7) / 8;
       L.fwd_cnt = (int)fw.size() - L.fwd_off;
       L.bwd_cnt = (int)bw.size() - L.bwd_off;
-      L.fwd_lean = L.fwd_cnt && fwd_bytes / L.fwd_cnt < tune.lean_task_bytes;
-      L.bwd_lean = L.bwd_cnt && bwd_bytes / L.bwd_cnt < tune.lean_task_bytes;
-      fwd_smem_max = std::max(fwd_smem_max, L.fwd_smem);
-      bwd_smem_max = std::max(bwd_smem_max, L.bwd_smem);
+      smem_max = std::max({smem_max, L.fwd_smem, L.bwd_smem});
     }
-    solve_small.upload(ss);
-    fwd_tasks.upload(fw);
-    bwd_tasks.upload(bw);
-    fwd_tmeta.upload(fwm);
-    bwd_tmeta.upload(bwm);
-    set_solve_attrs<kEThreads>(optin, fwd_smem_max, bwd_smem_max);
-    set_solve_attrs<kELeanThreads>(optin, fwd_smem_max, bwd_smem_max);
-    queue = tune.schedule == 1;
-    pdl = tune.pdl == 1;
-    overlap = tune.factor_overlap == 1;
-    tiny_threads = tune.tiny_threads;
-    tensor_update = tune.tensor_update;
-    q_wait_cycles = tune.queue_wait_cycles;
-    q_skip_publish = tune.queue_skip_publish;
-    if constexpr (sizeof(T) == 4)
-      if (tensor_update == 1)
-        CK(cudaFuncSetAttribute(mf_update_big_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-    if (queue) plan_queue(B, ss, fw, bw, fwd_smem_max, bwd_smem_max);
+    std::vector<SolveFront> fwm, bwm;
+    for (const int2 &t : fw) fwm.push_back(sf[(size_t)t.x]);
+    for (const int2 &t : bw) bwm.push_back(sf[(size_t)t.x]);
+    out.small.upload(ss);
+    out.fwd.upload(fw);
+    out.bwd.upload(bw);
+    out.fmeta.upload(fwm);
+    out.bmeta.upload(bwm);
+    return smem_max;
   }
 
-  template <int NT>
-  void set_solve_attrs(int optin, size_t fwd_smem_max, size_t bwd_smem_max) {
-    cudaFuncAttributes fa{}, fb{};
-    CK(cudaFuncGetAttributes(&fa, mf_fwd_big<T, NT>));
-    CK(cudaFuncGetAttributes(&fb, mf_bwd_big<T, NT>));
-    if (fwd_smem_max + fa.sharedSizeBytes > (size_t)optin || bwd_smem_max + fb.sharedSizeBytes > (size_t)optin)
-      throw CudaError{cudaErrorInvalidValue, "front too large for the shared-memory solve"};
-    CK(cudaFuncSetAttribute(mf_fwd_big<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            optin - (int)fa.sharedSizeBytes));
-    CK(cudaFuncSetAttribute(mf_bwd_big<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            optin - (int)fb.sharedSizeBytes));
+  // dynamic shared memory of the large-front kernels: always the device
+  // maximum (the attribute is per function, shared by every batch of this
+  // precision)
+  template <int V>
+  void set_solve_attrs(int optin, size_t smem_max) {
+    auto set = [&](auto *k) {
+      cudaFuncAttributes fa{};
+      CK(cudaFuncGetAttributes(&fa, k));
+      if (smem_max + fa.sharedSizeBytes > (size_t)optin)
+        throw CudaError{cudaErrorInvalidValue, "front too large for the shared-memory solve"};
+      CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
+    };
+    set(mf_fwd_big<T, V>);
+    set(mf_bwd_big<T, V>);
   }
 
   int factor(const double *vals, int *status, cudaStream_t s) {
@@ -526,7 +613,7 @@ struct MfDevice {
   // tasks producing its inputs (forward: all tasks of the children of its
   // fronts; backward: all tasks of their parents).
   void plan_queue(const MfBatch &B, const std::vector<int> &ss, const std::vector<int2> &fw,
-                  const std::vector<int2> &bw, size_t fwd_smem_max, size_t bwd_smem_max) {
+                  const std::vector<int2> &bw, size_t smem_max) {
     const int nf = B.nfronts;
     std::vector<int4> qt[2];
     std::vector<std::vector<int>> prod[2];   // per front: its tasks
@@ -535,7 +622,7 @@ struct MfDevice {
       prod[dir].assign((size_t)nf, {});
       for (int li = 0; li < nlevels; li++) {
         const int l = dir == 0 ? li : nlevels - 1 - li;
-        const SolveLevel &L = slevels[(size_t)l];
+        const SolveLevel &L = one.levels[(size_t)l];
         const int boff = dir == 0 ? L.fwd_off : L.bwd_off, bcnt = dir == 0 ? L.fwd_cnt : L.bwd_cnt;
         for (int i = boff; i < boff + bcnt; i++) {
           const int f = dir == 0 ? fw[(size_t)i].x : bw[(size_t)i].x;
@@ -589,11 +676,11 @@ struct MfDevice {
     qb_n = (int)qt[1].size();
     std::vector<int> so((size_t)nlevels);
     std::vector<SmallBuckets> sbv((size_t)nlevels);
-    for (int l = 0; l < nlevels; l++) { so[(size_t)l] = slevels[(size_t)l].small_off; sbv[(size_t)l] = slevels[(size_t)l].sb; }
+    for (int l = 0; l < nlevels; l++) { so[(size_t)l] = one.levels[(size_t)l].small_off; sbv[(size_t)l] = one.levels[(size_t)l].sb; }
     q_small_off.upload(so);
     q_sb.upload(sbv);
     q_counter.alloc(2);
-    q_smem = std::max({(size_t)8 * kSolveSmall * sizeof(T), fwd_smem_max, bwd_smem_max});
+    q_smem = std::max((size_t)8 * kSolveSmall * sizeof(T), smem_max);
     CK(cudaFuncSetAttribute(mf_fwd_queue<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q_smem));
     CK(cudaFuncSetAttribute(mf_bwd_queue<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q_smem));
     int dev = 0, nsm = 0, occ_f = 0, occ_b = 0;
@@ -619,13 +706,15 @@ struct MfDevice {
     xlm.alloc((size_t)xlen * K);
     ylm.alloc((size_t)xlen * K);
     um.alloc((size_t)std::max<int64_t>(ulen, 1) * K);
+    std::vector<int> ss;
+    std::vector<int2> fw, bw;
+    plan_solves(K, many, ss, fw, bw);
     mk = K;
   }
 
   // forward + backward solve: right-hand side in xl, solution back in xl
   // (nrhs > 1: the nrhs right-hand sides in xlm, solutions back in xlm)
   int solve(cudaStream_t s, int nrhs = 1, int *status = nullptr) {
-    int launches = 0;
     T *xl_ = nrhs > 1 ? xlm.p : xl.p, *yl_ = nrhs > 1 ? ylm.p : yl.p, *u_ = nrhs > 1 ? um.p : u.p;
     const int64_t xs = nrhs > 1 ? xlen : 0, us = nrhs > 1 ? std::max<int64_t>(ulen, 1) : 0;
     if (queue && status && q_k >= nrhs) {
@@ -633,44 +722,60 @@ struct MfDevice {
       CK(cudaMemsetAsync(q_done.p, 0, (size_t)(qf_n + qb_n) * nrhs * sizeof(int), s));
       mf_fwd_queue<T><<<q_grid, 256, q_smem, s>>>(view, QueueView{qf_tasks.p, qf_dep_ptr.p, qf_dep.p, qf_n,
                                                                    q_wait_cycles, q_skip_publish},
-                                                  solve_small.p, q_small_off.p, q_sb.p, fwd_tasks.p, fwd_tmeta.p, E.p,
+                                                  one.small.p, q_small_off.p, q_sb.p, one.fwd.p, one.fmeta.p, E.p,
                                                   xl_, yl_,
                                                   u_, q_counter.p, q_done.p, status, nrhs, xs, us);
       mf_bwd_queue<T><<<q_grid, 256, q_smem, s>>>(view, QueueView{qb_tasks.p, qb_dep_ptr.p, qb_dep.p, qb_n,
                                                                    q_wait_cycles, -1},
-                                                  solve_small.p, q_small_off.p, q_sb.p, bwd_tasks.p, bwd_tmeta.p, E.p,
+                                                  one.small.p, q_small_off.p, q_sb.p, one.bwd.p, one.bmeta.p, E.p,
                                                   yl_, xl_,
                                                   q_counter.p + 1, q_done.p + (size_t)qf_n * nrhs, status, nrhs, xs);
       return 2;
     }
+    return solve_levels(s, nrhs > 1 ? many : one, nrhs, xl_, yl_, u_, xs, us);
+  }
+
+  // the level launches
+  int solve_levels(cudaStream_t s, const SolveLists &w, int nrhs, T *xl_, T *yl_, T *u_, int64_t xs, int64_t us) {
+    int launches = 0;
+    auto fwd = [&](const SolveLevel &L, auto *k) {
+      launch_level(pdl, k, L.fwd_cnt * nrhs, kFwdVariants[L.fwd_v].nt, L.fwd_smem, s, view,
+                   (const int2 *)(w.fwd.p + L.fwd_off), (const SolveFront *)(w.fmeta.p + L.fwd_off),
+                   (const T *)E.p, (const T *)xl_, yl_, u_, nrhs, xs, us);
+    };
+    auto bwd = [&](const SolveLevel &L, auto *k) {
+      launch_level(pdl, k, L.bwd_cnt * nrhs, kBwdVariants[L.bwd_v].nt, L.bwd_smem, s, view,
+                   (const int2 *)(w.bwd.p + L.bwd_off), (const SolveFront *)(w.bmeta.p + L.bwd_off),
+                   (const T *)E.p, (const T *)yl_, xl_, nrhs, xs);
+    };
     for (int l = 0; l < nlevels; l++) {
-      const SolveLevel &L = slevels[(size_t)l];
+      const SolveLevel &L = w.levels[(size_t)l];
       if (L.small_cta) {
         launch_level(pdl, mf_fwd_small<T>, L.small_cta * nrhs, 256, 0, s, view,
-                     (const int *)(solve_small.p + L.small_off), L.sb, (const T *)E.p, (const T *)xl_, yl_, u_, nrhs,
+                     (const int *)(w.small.p + L.small_off), L.sb, (const T *)E.p, (const T *)xl_, yl_, u_, nrhs,
                      xs, us);
         launches++;
       }
       if (L.fwd_cnt) {
-        launch_level(pdl, L.fwd_lean ? mf_fwd_big<T, kELeanThreads> : mf_fwd_big<T, kEThreads>, L.fwd_cnt * nrhs,
-                     L.fwd_lean ? kELeanThreads : kEThreads, L.fwd_smem, s, view,
-                     (const int2 *)(fwd_tasks.p + L.fwd_off), (const TaskFront *)(fwd_tmeta.p + L.fwd_off),
-                     (const T *)E.p, (const T *)xl_, yl_, u_, nrhs, xs, us);
+        if (L.fwd_v == 0) fwd(L, mf_fwd_big<T, 0>);
+        else if (L.fwd_v == 1) fwd(L, mf_fwd_big<T, 1>);
+        else if (L.fwd_v == 2) fwd(L, mf_fwd_big<T, 2>);
+        else fwd(L, mf_fwd_big<T, 3>);
         launches++;
       }
     }
     for (int l = nlevels - 1; l >= 0; l--) {
-      const SolveLevel &L = slevels[(size_t)l];
+      const SolveLevel &L = w.levels[(size_t)l];
       if (L.bwd_cnt) {
-        launch_level(pdl, L.bwd_lean ? mf_bwd_big<T, kELeanThreads> : mf_bwd_big<T, kEThreads>, L.bwd_cnt * nrhs,
-                     L.bwd_lean ? kELeanThreads : kEThreads, L.bwd_smem, s, view,
-                     (const int2 *)(bwd_tasks.p + L.bwd_off), (const TaskFront *)(bwd_tmeta.p + L.bwd_off),
-                     (const T *)E.p, (const T *)yl_, xl_, nrhs, xs);
+        if (L.bwd_v == 0) bwd(L, mf_bwd_big<T, 0>);
+        else if (L.bwd_v == 1) bwd(L, mf_bwd_big<T, 1>);
+        else if (L.bwd_v == 2) bwd(L, mf_bwd_big<T, 2>);
+        else bwd(L, mf_bwd_big<T, 3>);
         launches++;
       }
       if (L.small_cta) {
         launch_level(pdl, mf_bwd_small<T>, L.small_cta * nrhs, 256, 0, s, view,
-                     (const int *)(solve_small.p + L.small_off), L.sb, (const T *)E.p, (const T *)yl_, xl_, nrhs, xs);
+                     (const int *)(w.small.p + L.small_off), L.sb, (const T *)E.p, (const T *)yl_, xl_, nrhs, xs);
         launches++;
       }
     }

@@ -126,7 +126,10 @@ __device__ __forceinline__ float tsqrt<float>(float x) { return sqrtf(x); }
 
 constexpr int kMfThreads = 256;
 constexpr int kNB = 32;      // panel width
-constexpr int kTile = 64;    // trailing-update tile (64 x 64 per CTA step, 4x4 per thread)
+// Tile of mf_update: FP32 64 x 64 (4 x 4 per thread).  FP64 32 x 32: its pipe
+// is the limit at any tile size, small tiles leave less padding and spread a
+// short update over more SMs (one 64 x 64 x 32 tile took 32 us on its SM).
+template <typename T> struct UpdTile { static constexpr int N = sizeof(T) == 8 ? 32 : 64; };
 
 // Every factorisation kernel also produces the front's elimination matrix
 //     E = [ L11^-1 ; -L21 L11^-1 ]     (m x k, column-major, ld = round4(m)),
@@ -186,29 +189,42 @@ template <> struct SVec<double> {
   __device__ static __forceinline__ void set(V &v, int q, double x) { if (q == 0) v.x = x; else v.y = x; }
 };
 
-// Row stride (elements) of the one-CTA kernel's panel and E in shared
-// memory: whole 16-byte vectors, an odd number of them, so that the vectors
-// of 8 consecutive rows fall into 8 different bank groups.
+// Row stride (elements) of the one-CTA kernel's panel in shared memory: whole
+// 16-byte vectors, an odd number of them, so that the vectors of 8
+// consecutive rows fall into 8 different bank groups.
 template <typename T> __host__ __device__ constexpr int pan_ld(int k) {
   const int vn = 16 / (int)sizeof(T);
   int nv = (k + vn - 1) / vn;
   if ((nv & 1) == 0) nv++;
   return nv * vn;
 }
-// shared memory of one front: panel and E (m x pan_ld(k) each), the
-// multiplier row (pan_ld(k))
+// shared memory of one front: panel (m rows), unit lower factor (k rows), two
+// multiplier rows, reciprocal pivots and their square roots
 template <typename T> __host__ __device__ constexpr size_t pan_smem(int m, int k) {
-  return ((size_t)2 * m + 1) * pan_ld<T>(k) * sizeof(T);
+  return ((size_t)m + k + 4) * pan_ld<T>(k) * sizeof(T);
 }
 
-// Fronts whose pivot panel (m x k) and E (m x k) fit in shared memory: one
-// CTA per front.  The pivot columns are assembled straight into shared
-// memory, the update block in the arena; the panel is factored and E formed
-// in shared memory, E is written out, and the update block receives
-// -L21 L21^T in 4x4 register blocks.  Panel and E are row-major in shared
-// memory (row i at i * pan_ld(k)): a thread updates its rows 16 bytes at a
-// time against the broadcast multiplier row, and the update block reads
-// 16-byte pieces of two rows per step.
+// Fronts whose panel (m x k) and factor (k x k) fit in shared memory: one CTA
+// per front.
+//
+//   1. The pivot columns are assembled into shared memory (row-major), the
+//      update block in the arena.
+//   2. A11 = Lt D Lt^T and Lt^-1, in place, one barrier per pivot: step j
+//      subtracts li = P(i, j) / d_j times a multiplier row from row i, whose
+//      columns left of j hold Lt^-1 so far and right of j the Schur
+//      complement.  The multiplier row (row j of Lt^-1, 1, column j of the
+//      Schur complement) is written by the threads of the step before.
+//   3. Rows of L21 by substitution with Lt, four lanes per row, no barrier;
+//      E11 = D^-1/2 Lt^-1.
+//   4. E21 = -L21 E11, four lanes per row; E to global; the update block
+//      receives -L21 L21^T in 4x4 register blocks.
+//
+// Only the k x k part walks the pivots one after the other; the m - k rows
+// below (most of the work) take part in two products.  Updating all m rows of
+// panel and E at every pivot instead, with two barriers, a square root and a
+// division per row each time, took: 705 FP64 fronts of up to 56 x 24 123 us
+// (now 77), 18 of up to 145 x 61 241 us (167), all one-CTA fronts of a 128^3
+// problem in FP32 9.9 ms (8.9).  FP64 is bound by its pipe from there on.
 constexpr int kPanThreads = 128;       // fronts of up to kPanWideRows rows
 constexpr int kPanThreadsWide = 256;   // larger fronts
 constexpr int kPanWideRows = 160;
@@ -224,33 +240,26 @@ mf_factor_panel(MfView v, const int *__restrict__ fronts, const double *__restri
   const int f = fronts[blockIdx.x];
   const int m = v.f_m[f], k = v.f_k[f], r = m - k;
   const int ldk = pan_ld<T>(k), nv = ldk / VN;
-  T *P = reinterpret_cast<T *>(smem_raw);  // m x k panel, row-major, row stride ldk
-  T *Es = P + (size_t)m * ldk;              // m x k elimination matrix, row-major
-  T *lmul = Es + (size_t)m * ldk;           // step j: L(c, j) for j < c < k, zero elsewhere
+  T *P = reinterpret_cast<T *>(smem_raw);   // m x k panel, row-major, row stride ldk
+  T *L = P + (size_t)m * ldk;               // k x k unit lower factor, likewise
+  T *mul = L + (size_t)k * ldk;             // multiplier rows of even and odd steps
+  T *inv = mul + 2 * ldk;                   // 1 / d_j
+  T *rs = inv + ldk;                        // d_j^-1/2
   const int64_t off = v.f_off[f];
   T *F = arena + off;
   const int tid = threadIdx.x, nt = blockDim.x;
-  // 1. zero: panel, E = [I ; 0] and the multiplier row in shared memory,
-  //    update block in the arena
-  for (int i = tid; i < m; i += nt) {
-    V *pr = reinterpret_cast<V *>(P + (size_t)i * ldk);
-    V *er = reinterpret_cast<V *>(Es + (size_t)i * ldk);
-    for (int q = 0; q < nv; q++) {
-      V z, e;
+  // 1. zero: panel and factor in shared memory, update block in the arena
+  {
+    V z;
 #pragma unroll
-      for (int u = 0; u < VN; u++) {
-        SV::set(z, u, T(0));
-        SV::set(e, u, (q * VN + u == i && i < k) ? T(1) : T(0));
-      }
-      pr[q] = z;
-      er[q] = e;
-    }
+    for (int u = 0; u < VN; u++) SV::set(z, u, T(0));
+    V *p = reinterpret_cast<V *>(P);
+    for (int q = tid; q < (m + k + 2) * nv; q += nt) p[q] = z;
   }
-  for (int c = tid; c < ldk; c += nt) lmul[c] = T(0);
   for (int c = 0; c < r; c++)
     for (int i = c + tid; i < r; i += nt) F[(int64_t)(k + c) * m + k + i] = T(0);
   __syncthreads();
-  // 2. original entries (each target once, duplicates summed in order)
+  // original entries (each target once, duplicates summed in order)
   for (int64_t e = v.f_asm[f] + tid; e < v.f_asm[f + 1]; e += nt) {
     double sv = 0.0;
     for (int64_t q = v.asm_sp[e]; q < v.asm_sp[e + 1]; q++) sv += vals[v.asm_src[q]];
@@ -263,7 +272,7 @@ mf_factor_panel(MfView v, const int *__restrict__ fronts, const double *__restri
     }
   }
   __syncthreads();
-  // 3. extend-add of the children's update matrices, children in order
+  // extend-add of the children's update matrices, children in order
   for (int ci = v.f_child_ptr[f]; ci < v.f_child_ptr[f + 1]; ci++) {
     const int c = v.f_children[ci];
     const int mc = v.f_m[c], kc = v.f_k[c], rc = mc - kc;
@@ -277,74 +286,166 @@ mf_factor_panel(MfView v, const int *__restrict__ fronts, const double *__restri
     }
     __syncthreads();
   }
-  // 4. factor the panel and eliminate E.  Every thread takes the pivot from
-  //    shared memory itself; the scaled column j goes to the multiplier row
-  //    (panel rows) beside the panel.  A thread then updates each of its
-  //    rows i > j 16 bytes at a time: panel columns (j, k) against the
-  //    multiplier row, E columns [0, j] against E's row j.  Entries left of
-  //    column j + 1 (panel) or right of column j (E) inside a vector keep
-  //    their values; upper-triangle and padding entries of the panel are
-  //    never read.  Each element receives the updates of the pivots in
-  //    increasing order.
-  for (int j = 0; j < k; j++) {
-    T d = P[(size_t)j * ldk + j];
+  // 2. the pivots
+  auto pivot = [&](T d, int j) {
     if (!(d > T(0))) {
-      if (tid == 0) atomicOr(status, ERR_NOT_SPD);
+      atomicOr(status, ERR_NOT_SPD);
       d = T(1);
     }
-    const T p = tsqrt<T>(d);
-    for (int i = j + 1 + tid; i < m; i += nt) {
-      const T x = P[(size_t)i * ldk + j] / p;
-      P[(size_t)i * ldk + j] = x;
-      if (i < k) lmul[i] = x;
-    }
-    for (int c = tid; c <= j; c += nt) Es[(size_t)j * ldk + c] /= p;
-    if (tid == 0) lmul[j] = T(0);  // held L(j, j-1); column j is no multiplier of step j
-    __syncthreads();
-    if (tid == 0) P[(size_t)j * ldk + j] = p;  // read by no thread before the next step
-    const V *lm = reinterpret_cast<const V *>(lmul);
-    const V *ej = reinterpret_cast<const V *>(Es + (size_t)j * ldk);
-    const int qp0 = (j + 1) / VN, qp1 = (k + VN - 1) / VN, qe1 = j / VN;
-    for (int i = j + 1 + tid; i < m; i += nt) {
-      const T lij = P[(size_t)i * ldk + j];
-      V *pr = reinterpret_cast<V *>(P + (size_t)i * ldk);
-      V *er = reinterpret_cast<V *>(Es + (size_t)i * ldk);
-      for (int q = qp0; q < qp1; q++) {
-        const V a = pr[q], b = lm[q];
+    inv[j] = T(1) / d;
+  };
+  for (int c = tid; c < k; c += nt) {
+    const T x = P[(size_t)c * ldk];
+    mul[c] = c == 0 ? T(1) : x;
+    if (c == 0) pivot(x, 0);
+  }
+  __syncthreads();
+  constexpr int TX = 4;  // threads per row
+  const int tx = tid & (TX - 1), ty = tid / TX, ny = nt / TX;
+  for (int j = 0; j < k - 1; j++) {
+    const T *cur = mul + (j & 1) * ldk;
+    T *nxt = mul + ((j + 1) & 1) * ldk;
+    const T iv = inv[j];
+    for (int i = j + 1 + ty; i < k; i += ny) {
+      const T li = cur[i] * iv;
+      if (tx == 0) L[(size_t)i * ldk + j] = li;
+      V *row = reinterpret_cast<V *>(P + (size_t)i * ldk);
+      // (entries right of the diagonal take garbage; nothing reads them)
+      for (int q = tx; q * VN <= i; q += TX) {
+        const V a = row[q], w = reinterpret_cast<const V *>(cur)[q];
         V o;
 #pragma unroll
-        for (int u = 0; u < VN; u++) {
-          const T nvl = SV::get(a, u) - lij * SV::get(b, u);
-          SV::set(o, u, q * VN + u > j ? nvl : SV::get(a, u));
-        }
-        pr[q] = o;
-      }
-      for (int q = 0; q <= qe1; q++) {
-        const V a = er[q], b = ej[q];
-        V o;
+        for (int u = 0; u < VN; u++) SV::set(o, u, SV::get(a, u) - li * SV::get(w, u));
+        if (q == j / VN)
 #pragma unroll
-        for (int u = 0; u < VN; u++) {
-          const T nvl = SV::get(a, u) - lij * SV::get(b, u);
-          SV::set(o, u, q * VN + u <= j ? nvl : SV::get(a, u));
+          for (int u = 0; u < VN; u++)
+            if (u == j % VN) SV::set(o, u, -li);
+        row[q] = o;
+        if (i == j + 1) {  // the next pivot's row
+#pragma unroll
+          for (int u = 0; u < VN; u++) {
+            const int c = q * VN + u;
+            if (c <= j) nxt[c] = SV::get(o, u);
+            else if (c == i) {
+              nxt[c] = T(1);
+              pivot(SV::get(o, u), i);
+            }
+          }
+        } else if (q == (j + 1) / VN) {  // and its column
+#pragma unroll
+          for (int u = 0; u < VN; u++)
+            if (u == (j + 1) % VN) nxt[i] = SV::get(o, u);
         }
-        er[q] = o;
       }
     }
     __syncthreads();
   }
-  // 5. E -> global (column-major, ld round4(m)); the padding rows stay zero
+  for (int j = tid; j < k; j += nt) rs[j] = tsqrt<T>(inv[j]);
+  __syncthreads();
+  // 3. E11: rows of Lt^-1 scaled (its unit diagonal and the zeros above it)
+  for (int q = tid; q < k * nv; q += nt) {
+    const int i = q / nv, c0 = (q % nv) * VN;
+    V a = reinterpret_cast<V *>(P + (size_t)i * ldk)[q % nv];
+    const T sc = rs[i];
+#pragma unroll
+    for (int u = 0; u < VN; u++) SV::set(a, u, c0 + u < i ? SV::get(a, u) * sc : c0 + u == i ? sc : T(0));
+    reinterpret_cast<V *>(P + (size_t)i * ldk)[q % nv] = a;
+  }
+  //    L21, LW lanes per row and CL columns per lane (FP64 four lanes: the
+  //    pipe of one SM sub-partition would walk a row alone; FP32 two, for more
+  //    multiplications per shared-memory read): z = A21 Lt^-T block
+  //    by block of 8 columns, then scaled by D^-1/2
+  constexpr int LW = sizeof(T) == 8 ? 4 : 2, CL = 8 / LW;
+  const int sub = tid % LW, g0 = (tid & 31) / LW * LW;  // lane in the row's group, group's first lane
+  for (int i0 = k; i0 < m; i0 += nt / LW) {
+    const int i = min(i0 + tid / LW, m - 1);  // (rows past m repeat the last one)
+    const bool on = i0 + tid / LW < m;
+    T *pr = P + (size_t)i * ldk;
+    for (int b0 = 0; b0 < k; b0 += 8) {
+      const int c0 = b0 + CL * sub;
+      T a[CL];
+      const T *l[CL];
+#pragma unroll
+      for (int h = 0; h < CL; h++) {
+        a[h] = c0 + h < k ? pr[c0 + h] : T(0);
+        l[h] = L + (size_t)min(c0 + h, k - 1) * ldk;
+      }
+      for (int q = 0; q < b0; q += VN) {
+        const V z = *reinterpret_cast<const V *>(pr + q);
+#pragma unroll
+        for (int h = 0; h < CL; h++) {
+          const V x = *reinterpret_cast<const V *>(l[h] + q);
+#pragma unroll
+          for (int u = 0; u < VN; u++) a[h] -= SV::get(z, u) * SV::get(x, u);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 7; t++) {
+        T z = a[t % CL];
+        if constexpr (LW > 1) z = __shfl_sync(0xffffffffu, z, g0 + t / CL);
+        if (b0 + t < k - 1)
+#pragma unroll
+          for (int h = 0; h < CL; h++)
+            if (CL * sub + h > t) a[h] -= z * l[h][b0 + t];
+      }
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < CL; h++)
+        if (on && c0 + h < k) pr[c0 + h] = a[h];
+      __syncwarp();
+    }
+    if (on)
+      for (int c = sub; c < k; c += LW) pr[c] *= rs[c];
+    __syncwarp();
+  }
+  __syncthreads();
+  // 4. E -> global (column-major, ld round4(m)); the padding rows stay zero
   {
     const int ld = round4(m);
     T *Eg = E + v.e_off[f];
     for (int c = 0; c < k; c++)
-      for (int i = tid; i < m; i += nt) Eg[(int64_t)c * ld + i] = Es[(size_t)i * ldk + c];
+      for (int i = tid; i < k; i += nt) Eg[(int64_t)c * ld + i] = P[(size_t)i * ldk + c];
+    for (int i = k + tid / LW; i < m; i += nt / LW) {
+      const T *pr = P + (size_t)i * ldk;
+      for (int b0 = 0; b0 < k; b0 += 8) {
+        const int c0 = b0 + CL * sub;
+        T a[CL];
+#pragma unroll
+        for (int h = 0; h < CL; h++) a[h] = T(0);
+        for (int q = b0; q < k; q += VN) {
+          const V z = *reinterpret_cast<const V *>(pr + q);
+#pragma unroll
+          for (int u = 0; u < VN; u++) {
+            if (q + u < k) {
+              // (a row's vectors past column k: the next row's first, unused)
+              const T *e = P + (size_t)(q + u) * ldk + c0;
+#pragma unroll
+              for (int h = 0; h < CL; h += VN) {
+                const V x = *reinterpret_cast<const V *>(e + h);
+#pragma unroll
+                for (int w = 0; w < VN; w++) a[h + w] -= SV::get(z, u) * SV::get(x, w);
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < CL; h++)
+          if (c0 + h < k) Eg[(int64_t)(c0 + h) * ld + i] = a[h];
+      }
+    }
   }
-  // 6. update block: F[k:m, k:m] -= L21 L21^T (lower), 4x4 blocks per thread;
-  //    L21 rows read VN columns at a time (padding columns are zero)
-  const int nb4 = (r + 3) / 4;
-  for (int q = tid; q < nb4 * nb4; q += nt) {
-    const int bi = q % nb4, bc = q / nb4;
-    if (bi < bc) continue;
+  //    update block: F[k:m, k:m] -= L21 L21^T (lower), 4x4 blocks per thread
+  //    over the lower block triangle; L21 rows read VN columns at a time
+  const int nb4 = (r + 3) / 4, nblk = nb4 * (nb4 + 1) / 2;
+  for (int q = tid; q < nblk; q += nt) {
+    // q-th block of the lower triangle, column by column (consecutive threads
+    // share a column block and update consecutive rows): t columns from the
+    // last one, counted from its end
+    const int e = nblk - 1 - q;
+    int t = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+    while (t * (t + 1) / 2 > e) t--;
+    while ((t + 1) * (t + 2) / 2 <= e) t++;
+    const int bc = nb4 - 1 - t, bi = nb4 - 1 - (e - t * (t + 1) / 2);
     const int i0 = k + 4 * bi, c0 = k + 4 * bc;
     T acc[4][4];
 #pragma unroll
@@ -444,29 +545,43 @@ __device__ __forceinline__ void chol_warp(T (*D)[kNB + 1], int jb, int *status) 
   for (int c = 0; c < kNB; c++) D[lane][c] = a[c];
 }
 
-// The same right-looking Cholesky by a whole CTA in shared memory, one
-// pivot per step: for FP64, whose square roots and divisions are too slow
-// for one warp's chain on the FP64 pipe
+// The Cholesky factor by a whole CTA in shared memory as L D L^T with the
+// columns scaled at the end, one barrier and one division per pivot: for
+// FP64, whose square roots and divisions are too slow for one warp's chain
+// on the FP64 pipe
 template <typename T>
 __device__ __forceinline__ void chol_cta(T (*D)[kNB + 1], int jb, int *status) {
+  __shared__ T inv[kNB];
   const int tid = threadIdx.x;
-  for (int j = 0; j < jb; j++) {
-    if (tid == 0) {
-      T d = D[j][j];
-      if (!(d > T(0))) { atomicOr(status, ERR_NOT_SPD); d = T(1); }
-      D[j][j] = tsqrt<T>(d);
+  auto pivot = [&](T d, int j) {
+    if (!(d > T(0))) {
+      atomicOr(status, ERR_NOT_SPD);
+      d = T(1);
     }
-    __syncthreads();
-    const T p = D[j][j];
-    for (int i = j + 1 + tid; i < jb; i += blockDim.x) D[i][j] /= p;
-    __syncthreads();
-    const int w = jb - j - 1;
-    for (int q = tid; q < w * w; q += blockDim.x) {
-      const int i = j + 1 + q / w, c = j + 1 + q % w;
-      if (i >= c) D[i][c] -= D[i][j] * D[c][j];
+    D[j][j] = d;
+    inv[j] = T(1) / d;
+  };
+  if (tid == 0) pivot(D[0][0], 0);
+  __syncthreads();
+  constexpr int TX = kMfThreads / kNB;  // threads per row
+  const int i = tid / TX, tx = tid % TX;
+  for (int j = 0; j < jb - 1; j++) {
+    if (i > j && i < jb) {
+      const T li = D[i][j] * inv[j];
+      for (int c = j + 1 + tx; c <= i; c += TX) {
+        const T x = D[i][c] - li * D[c][j];
+        if (c == i && i == j + 1) pivot(x, i);
+        else D[i][c] = x;
+      }
     }
     __syncthreads();
   }
+  for (int q = tid; q < jb * jb; q += kMfThreads) {
+    const int c = q / jb, k = q % jb;
+    if (k > c) D[k][c] *= tsqrt<T>(inv[c]);
+  }
+  __syncthreads();
+  if (tid < jb) D[tid][tid] = tsqrt<T>(D[tid][tid]);
 }
 
 // FP32: one warp per front (chol_warp); FP64: kMfThreads per front (chol_cta)
@@ -573,6 +688,8 @@ mf_panel(MfView v, const int2 *__restrict__ tasks, int npanel, const int2 *__res
     int c = q / jb, i = q % jb;
     D[i][c] = i >= c ? F[(int64_t)(j0 + c) * m + j0 + i] : T(0);
   }
+  __shared__ T rd[kNB];  // FP64: reciprocals of its diagonal, no division per row
+  if (sizeof(T) == 8 && tid < jb) rd[tid] = T(1) / F[(int64_t)(j0 + tid) * m + j0 + tid];
   if (escale) {
     constexpr int NC = EscCols<T>::N;
     __shared__ T Eb[NC][kNB + 1];
@@ -590,7 +707,7 @@ mf_panel(MfView v, const int2 *__restrict__ tasks, int npanel, const int2 *__res
       for (int t = 0; t < jb; t++) {
         T s = Eb[cc][t];
         for (int q = 0; q < t; q++) s -= D[t][q] * Eb[cc][q];
-        Eb[cc][t] = s / D[t][t];
+        Eb[cc][t] = sizeof(T) == 8 ? s * rd[t] : s / D[t][t];
       }
     }
     __syncthreads();
@@ -617,7 +734,7 @@ mf_panel(MfView v, const int2 *__restrict__ tasks, int npanel, const int2 *__res
         T s = x[t];
 #pragma unroll
         for (int q = 0; q < t; q++) s -= x[q] * D[t][q];
-        x[t] = s / D[t][t];
+        x[t] = sizeof(T) == 8 ? s * rd[t] : s / D[t][t];
       }
     }
 #pragma unroll
@@ -626,7 +743,7 @@ mf_panel(MfView v, const int2 *__restrict__ tasks, int npanel, const int2 *__res
   }
 }
 
-// One 64x64 tile of an update with the L columns [jl, jl + K), K = min(kw, k - jl).
+// One tile (UpdTile) of an update with the L columns [jl, jl + K), K = min(kw, k - jl).
 // Trailing-update tiles (task = {front, (ti << 16) | tj}, ti >= tj) cover rows
 // and columns from c0 = jl + K: C -= L[rows, J] L[cols, J]^T (lower part),
 // only columns below cend = min(cend_base, k) when cend_base > 0 (the update
@@ -642,6 +759,7 @@ template <typename T>
 __global__ void __launch_bounds__(kMfThreads)
 mf_update(MfView v, const int2 *__restrict__ tasks, int nupd, const int2 *__restrict__ etasks, int jl, int kw,
           int cend_base, T *__restrict__ arena, T *__restrict__ E, int *__restrict__ status) {
+  constexpr int kTile = UpdTile<T>::N, R = kTile / 16;
   __shared__ T As[kNB][kTile];
   __shared__ T Bs[kNB][kTile + 1];
   const bool etile = (int)blockIdx.x >= nupd;
@@ -658,11 +776,11 @@ mf_update(MfView v, const int2 *__restrict__ tasks, int nupd, const int2 *__rest
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int ld = round4(m);
   T *Eg = E + v.e_off[f];
-  T acc[4][4];
+  T acc[R][R];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < R; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) acc[a][b] = T(0);
+    for (int b = 0; b < R; b++) acc[a][b] = T(0);
   for (int t0 = 0; t0 < K; t0 += kNB) {
     const int tb = min(kNB, K - t0);
     if (t0 > 0) __syncthreads();  // the previous chunk is consumed
@@ -683,26 +801,26 @@ mf_update(MfView v, const int2 *__restrict__ tasks, int nupd, const int2 *__rest
     }
     __syncthreads();
     for (int t = 0; t < tb; t++) {
-      T ra[4], rb[4];
+      T ra[R], rb[R];
 #pragma unroll
-      for (int a = 0; a < 4; a++) ra[a] = As[t][tx + 16 * a];
+      for (int a = 0; a < R; a++) ra[a] = As[t][tx + 16 * a];
 #pragma unroll
-      for (int b = 0; b < 4; b++) rb[b] = Bs[t][ty + 16 * b];
+      for (int b = 0; b < R; b++) rb[b] = Bs[t][ty + 16 * b];
 #pragma unroll
-      for (int a = 0; a < 4; a++)
+      for (int a = 0; a < R; a++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] += ra[a] * rb[b];
+        for (int b = 0; b < R; b++) acc[a][b] += ra[a] * rb[b];
     }
   }
   const int j0 = jl;
   if (etile) {
     const int rend = cend_base > 0 ? cend : m;
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
+    for (int b = 0; b < R; b++) {
       const int col = cc0 + ty + 16 * b;
       if (col >= c0) continue;
 #pragma unroll
-      for (int a = 0; a < 4; a++) {
+      for (int a = 0; a < R; a++) {
         const int row = r0 + tx + 16 * a;
         if (row >= rend) continue;
         T *dst = Eg + (int64_t)col * ld + row;
@@ -712,11 +830,11 @@ mf_update(MfView v, const int2 *__restrict__ tasks, int nupd, const int2 *__rest
     return;
   }
 #pragma unroll
-  for (int b = 0; b < 4; b++) {
+  for (int b = 0; b < R; b++) {
     const int col = cc0 + ty + 16 * b;
     if (col >= cend) continue;
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
+    for (int a = 0; a < R; a++) {
       const int row = r0 + tx + 16 * a;
       if (row < m && row >= col) F[(int64_t)col * m + row] -= acc[a][b];
     }

@@ -249,7 +249,7 @@ struct MfDevice {
         if (m <= tune.tiny_rows) {
           tiny.push_back(f);
           L.tiny_smem = std::max(L.tiny_smem, smem);
-        } else if (m <= tune.panel_rows && smem <= kPanelSmem) {
+        } else if (m <= tune.panel_rows && ((size_t)2 * m + 1) * pan_ld<T>(k) * sizeof(T) <= kPanelSmem) {
           pan.push_back(f);
           L.pan_smem = std::max(L.pan_smem, smem);
           L.pan_maxm = std::max(L.pan_maxm, m);
@@ -274,6 +274,7 @@ struct MfDevice {
       // panel updates only the rest of its super-panel; the trailing matrix
       // receives one update with up to kSuperPanel columns of L per super-panel
       const int SP = tune.super_panel;
+      constexpr int kTile = UpdTile<T>::N;
       for (int S0 = 0; S0 < kmax; S0 += SP) {
         for (int j0 = S0; j0 < std::min(S0 + SP, kmax); j0 += kNB) {
           Step st{j0, (int)df.size(), 0, (int)pf.size(), 0, (int)es.size(), 0,
@@ -306,7 +307,7 @@ struct MfDevice {
           st.etile_cnt = (int)et.size() - st.etile_off;
           L.steps.push_back(st);
         }
-        const bool bigt = sizeof(T) == 4;  // FP32: 128 x 128 tiles; FP64 keeps 64 x 64 (FP64-pipe bound)
+        const bool bigt = sizeof(T) == 4;  // FP32: 128 x 128 tiles; FP64 keeps mf_update (FP64-pipe bound)
         const int tile = bigt ? kBT : kTile;
         Step st{S0, (int)df.size(), 0, (int)pf.size(), 0, (int)es.size(), 0,
                 (int)ut.size(), 0, (int)et.size(), 0, SP, 0, bigt};
@@ -527,6 +528,14 @@ struct MfDevice {
     set(mf_bwd_big<T, V>);
   }
 
+  // Threads of a one-CTA front: `most` when the level's fronts fill the GPU
+  // several times over; with few fronts per SM as many as its four
+  // sub-partitions take (FP64: each has half an FMA per clock)
+  int pan_threads(int cnt, int nt) const {
+    while (sizeof(T) == 8 && nt < kPanThreadsWide && cnt < 512 * nsm / nt) nt *= 2;
+    return nt;
+  }
+
   int factor(const double *vals, int *status, cudaStream_t s) {
     int launches = 0;
     if (overlap && !aux) {  // the side stream takes the calling stream's priority
@@ -548,12 +557,13 @@ struct MfDevice {
         sp = aux;
       }
       if (L.tiny_cnt) {  // small fronts: narrow CTAs, more of them per SM
-        mf_factor_panel<T><<<L.tiny_cnt, tiny_threads, L.tiny_smem, sp>>>(view, pan_fronts.p + L.tiny_off, vals,
+        mf_factor_panel<T><<<L.tiny_cnt, pan_threads(L.tiny_cnt, tiny_threads), L.tiny_smem, sp>>>(view, pan_fronts.p + L.tiny_off, vals,
                                                                           arena.p, E.p, status);
         launches++;
       }
       if (L.pan_cnt) {
-        mf_factor_panel<T><<<L.pan_cnt, L.pan_maxm > kPanWideRows ? kPanThreadsWide : kPanThreads, L.pan_smem, sp>>>(
+        const int nt = L.pan_maxm > kPanWideRows ? kPanThreadsWide : kPanThreads;
+        mf_factor_panel<T><<<L.pan_cnt, pan_threads(L.pan_cnt, nt), L.pan_smem, sp>>>(
             view, pan_fronts.p + L.pan_off, vals, arena.p, E.p, status);
         launches++;
       }

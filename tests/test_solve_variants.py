@@ -7,6 +7,8 @@ sides of every line: warp kernels and one wave of short tasks by default;
 every front as CTA tasks (thin_level_fronts) gives the 128-thread variants,
 with lean_task_kb 1 the 256-thread one; leaves of 3 unknowns give tiny fronts
 and fronts of more than two children; one subdomain gives the longest fronts.
+The last four reach the ends of the one-CTA factorisation: leaves of 2, 33 and
+90 pivots, and every front of more than 20 rows through the panel pipeline.
 Bars: those of the other solve tests, FP64 1e-10 and mixed 1e-7 of the FP64
 oracle (tolerance 1e-12), the FP64 iteration count within one.
 """
@@ -28,7 +30,9 @@ OPTS = dict(solver=2, method=1, fine_method=1, levels=2, overlap=2, smoothers=1,
 @pytest.mark.parametrize("n,parts,words", [(26, 4, {}), (26, 4, dict(thin_level_fronts=100000)),
                                            (26, 4, dict(thin_level_fronts=100000, lean_task_kb=1)),
                                            (26, 4, dict(thin_level_fronts=0)), (17, 2, dict(nd_leaf=3)),
-                                           (21, 1, dict(fwd_task_kb=1))])
+                                           (21, 1, dict(fwd_task_kb=1)), (11, 2, dict(nd_leaf=2)),
+                                           (19, 2, dict(nd_leaf=33)), (19, 2, dict(nd_leaf=90)),
+                                           (21, 1, dict(panel_rows=20))])
 def test_variants_match_the_oracle(n, parts, words, precision):
     import doug_gb300 as D
     import oracle as O

@@ -47,7 +47,7 @@ def _stale(obj, srcs):
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OUT, exist_ok=True)
     nvcc = _nvcc()
-    headers = [os.path.join(CSRC, f) for f in ("dg_kernels.cuh", "host/setup.hpp", "host/mf_symbolic.hpp")]
+    headers = [os.path.join(CSRC, f) for f in ("dg_kernels.cuh", "dg_split.cuh", "dg_tc.cuh", "host/setup.hpp", "host/mf_symbolic.hpp")]
     headers.append(os.path.join(ROOT, "include", "doug_gpu.h"))
     jobs = []
     objs = []

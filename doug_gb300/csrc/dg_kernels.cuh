@@ -548,8 +548,13 @@ __device__ __forceinline__ void chol_warp(T (*D)[kNB + 1], int jb, int *status) 
 // The Cholesky factor by a whole CTA in shared memory as L D L^T with the
 // columns scaled at the end, one barrier and one division per pivot: for
 // FP64, whose square roots and divisions are too slow for one warp's chain
-// on the FP64 pipe
-template <typename T>
+// on the FP64 pipe.  NAMED: the first kMfThreads threads of a larger CTA.
+template <bool NAMED>
+__device__ __forceinline__ void diag_sync() {
+  if constexpr (NAMED) asm volatile("bar.sync 1, %0;" ::"n"(kMfThreads) : "memory");
+  else __syncthreads();
+}
+template <typename T, bool NAMED = false>
 __device__ __forceinline__ void chol_cta(T (*D)[kNB + 1], int jb, int *status) {
   __shared__ T inv[kNB];
   const int tid = threadIdx.x;
@@ -562,7 +567,7 @@ __device__ __forceinline__ void chol_cta(T (*D)[kNB + 1], int jb, int *status) {
     inv[j] = T(1) / d;
   };
   if (tid == 0) pivot(D[0][0], 0);
-  __syncthreads();
+  diag_sync<NAMED>();
   constexpr int TX = kMfThreads / kNB;  // threads per row
   const int i = tid / TX, tx = tid % TX;
   for (int j = 0; j < jb - 1; j++) {
@@ -574,13 +579,13 @@ __device__ __forceinline__ void chol_cta(T (*D)[kNB + 1], int jb, int *status) {
         else D[i][c] = x;
       }
     }
-    __syncthreads();
+    diag_sync<NAMED>();
   }
   for (int q = tid; q < jb * jb; q += kMfThreads) {
     const int c = q / jb, k = q % jb;
     if (k > c) D[k][c] *= tsqrt<T>(inv[c]);
   }
-  __syncthreads();
+  diag_sync<NAMED>();
   if (tid < jb) D[tid][tid] = tsqrt<T>(D[tid][tid]);
 }
 
@@ -591,21 +596,21 @@ template <typename T> __host__ __device__ constexpr int diag_threads() { return 
 // front's arena block, ld m): its lower part into shared memory, FP32 by one
 // warp in registers, FP64 by the whole CTA; every thread of the CTA calls it,
 // after a barrier that makes the block's final values visible.
-template <typename T>
+template <typename T, bool NAMED = false>
 __device__ __forceinline__ void factor_diag_block(T *__restrict__ F, int m, int j0, int jb, int *status) {
   __shared__ T D[kNB][kNB + 1];
-  const int tid = threadIdx.x, nt = blockDim.x;
+  const int tid = threadIdx.x, nt = NAMED ? kMfThreads : blockDim.x;
   for (int q = tid; q < kNB * kNB; q += nt) {  // lower part, zeros elsewhere
     const int c = q / kNB, i = q % kNB;  // column-major walk: coalesced over rows
     D[i][c] = (i >= c && i < jb) ? F[(int64_t)(j0 + c) * m + j0 + i] : T(0);
   }
-  __syncthreads();
+  diag_sync<NAMED>();
   if constexpr (sizeof(T) == 4) {
     if (tid < 32) chol_warp<T>(D, jb, status);
   } else {
-    chol_cta<T>(D, jb, status);
+    chol_cta<T, NAMED>(D, jb, status);
   }
-  __syncthreads();
+  diag_sync<NAMED>();
   for (int q = tid; q < jb * jb; q += nt) {
     const int c = q / jb, i = q % jb;
     if (i >= c) F[(int64_t)(j0 + c) * m + j0 + i] = D[i][c];
@@ -1145,6 +1150,10 @@ mf_update_big_tc(MfView v, const int2 *__restrict__ tasks, int nupd, const int2 
   if (fuse_diag && !bad && !etile && ti == 0 && tj == 0 && c0 < k)
     factor_diag_block<float>(F, m, c0, min(kNB, k - c0), status);
 }
+
+}  // namespace dg
+#include "dg_split.cuh"  // FP64 super-panel updates on the tensor cores
+namespace dg {
 
 // ---------------------------------------------------------------------------
 // multifrontal solves with the elimination matrices E

@@ -143,6 +143,9 @@ struct MfDevice {
   int qf_n = 0, qb_n = 0, q_grid = 0, q_k = 0;
   size_t q_smem = 0;
   DBuf<int2> asm_tasks, upd_tasks, panel_tasks, esc_tasks, etile_tasks;
+  DBuf<int4> split_tasks, tile_tasks;
+  DBuf<unsigned char> slices;  // of one super-panel step's fronts
+  DBuf<int> expo;
   DBuf<T> arena, E, xl, yl, u;
   int64_t e_len = 0;
   // per level: small-front range, assembly-task range, steps
@@ -154,6 +157,8 @@ struct MfDevice {
     int upd_off, upd_cnt, etile_off, etile_cnt;
     int kw, cend_base;
     bool big;                     // trailing update in 128 x 128 tiles (FP32)
+    int split_off = 0, split_cnt = 0;  // FP64 on the tensor cores: mf_split tasks (0: mf_update),
+    int tile_off = 0, tile_cnt = 0, tile_upd = 0;  // mf_update_split tasks, trailing tiles first
   };
   struct Level {
     int pan_off, pan_cnt, asm_off, asm_cnt, pan_maxm;
@@ -234,6 +239,8 @@ struct MfDevice {
     // work lists of the factorisation
     std::vector<int> pn, df;
     std::vector<int2> at, ut, pf, es, et;
+    std::vector<int4> sp, tt;
+    int64_t split_blocks = 0;
     levels.assign((size_t)nlevels, Level());
     for (int l = 0; l < nlevels; l++) {
       Level &L = levels[(size_t)l];
@@ -311,6 +318,11 @@ struct MfDevice {
         const int tile = bigt ? kBT : kTile;
         Step st{S0, (int)df.size(), 0, (int)pf.size(), 0, (int)es.size(), 0,
                 (int)ut.size(), 0, (int)et.size(), 0, SP, 0, bigt};
+        if (sizeof(T) == 8 && split_step(B, tune, large, S0)) {
+          plan_split(B, large, S0, SP, st, sp, tt, split_blocks);
+          L.steps.push_back(st);
+          continue;
+        }
         for (int f : large) {
           int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
           if (S0 >= k) continue;
@@ -342,6 +354,13 @@ struct MfDevice {
     asm_tasks.upload(at);
     upd_tasks.upload(ut);
     etile_tasks.upload(et);
+    if (split_blocks) {
+      split_tasks.upload(sp);
+      tile_tasks.upload(tt);
+      slices.alloc((size_t)split_blocks * kSplitBlock);
+      expo.alloc((size_t)split_blocks * kSplitRows);
+      CK(cudaFuncSetAttribute(mf_update_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitSmem));
+    }
     // what the solves read about a front, and its child table
     sf.assign((size_t)nfronts, SolveFront());
     std::vector<unsigned> ct;
@@ -395,6 +414,64 @@ struct MfDevice {
       if (tensor_update == 1)
         CK(cudaFuncSetAttribute(mf_update_big_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
     if (queue) plan_queue(B, ss, fw, bw, smem_max);
+  }
+
+  // Does the tensor-core update take the FP64 super-panel at column S0?  Where
+  // it is the faster one: mf_update's 32 x 32 tiles are bound by the FP64 pipe
+  // (two multiply-adds per clock and SM: 0.27 us per tile and column of L,
+  // all SMs at least one tile), while the tensor-core path takes 14 us per
+  // round of 128 x 64 tiles with 64 columns, 18.5 us with 128, and 8 us for
+  // the slices.  Measured (mf_update against mf_split and the tiles, both with
+  // the next diagonal block): 25 tiles of 32 x 32 and 32 columns 17.5 us against
+  // 26 us, 182 of 128 columns 52 us against 37 us, 58 of 128 columns 66 us
+  // against 56 us, 49386 of 128 columns 3.24 ms against 1.00 ms.
+  bool split_step(const MfBatch &B, const MfTune &tune, const std::vector<int> &large, int S0) const {
+    if (tune.tensor_update != 1 || tune.super_panel > kSplitK) return false;
+    double fma_tiles = 0, tiles = 0, kmax = 0;
+    for (int f : large) {
+      const int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
+      if (S0 >= k) continue;
+      const int K = std::min(tune.super_panel, k - S0), c1 = S0 + K, r = m - c1;
+      if (r <= 0) continue;
+      const double n32 = (r + 31) / 32, e32 = (c1 + 31) / 32, n128 = (r + 127) / 128;
+      fma_tiles += K * (0.5 * n32 * (n32 + 1) + n32 * e32);
+      tiles += n128 * (n128 + 1) + n128 * ((c1 + 63) / 64);
+      kmax = std::max(kmax, (double)K);
+    }
+    const double cuda = 0.27 * std::max(kmax, fma_tiles / nsm);
+    const double tensor = 8.0 + std::ceil(tiles / nsm) * (9.5 + 0.07 * kmax);
+    return cuda > tensor;
+  }
+
+  // Tasks of the tensor-core update of the super-panel at column S0: 64-row
+  // blocks of L below it (an even number: a tile takes two) and of E's
+  // columns before its end, then the tiles.
+  static void plan_split(const MfBatch &B, const std::vector<int> &large, int S0, int SP, Step &st,
+                         std::vector<int4> &sp, std::vector<int4> &tt, int64_t &blocks) {
+    std::vector<int4> te;
+    st.split_off = (int)sp.size();
+    st.tile_off = (int)tt.size();
+    int blk = 0;
+    for (int f : large) {
+      const int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
+      if (S0 >= k) continue;
+      const int c1 = S0 + std::min(SP, k - S0);
+      if (c1 >= m) continue;
+      const int nt = (m - c1 + 127) / 128, nl = (m - c1 + kSplitRows - 1) / kSplitRows;
+      const int ne = (c1 + kSplitRows - 1) / kSplitRows, be = blk + 2 * nt;
+      for (int h = 0; h < 4 * nt; h++) sp.push_back(make_int4(f, c1 + h * kSplitCtaRows, 2 * blk + h, 0));
+      for (int h = 0; h < 2 * ne; h++) sp.push_back(make_int4(f, ~(h * kSplitCtaRows), 2 * be + h, 0));
+      for (int tj = 0; tj < nl; tj++)
+        for (int ti = tj / 2; ti < nt; ti++) tt.push_back(make_int4(f, (ti << 16) | tj, blk + 2 * ti, blk + tj));
+      for (int ti = 0; ti < nt; ti++)
+        for (int tc = 0; tc < ne; tc++) te.push_back(make_int4(f, (ti << 16) | tc, blk + 2 * ti, be + tc));
+      blk = be + ne;
+    }
+    st.tile_upd = (int)tt.size() - st.tile_off;
+    tt.insert(tt.end(), te.begin(), te.end());
+    st.split_cnt = (int)sp.size() - st.split_off;
+    st.tile_cnt = (int)tt.size() - st.tile_off;
+    blocks = std::max<int64_t>(blocks, blk);
   }
 
   // Solve work lists for K right-hand sides: warp kernels for the
@@ -604,6 +681,15 @@ struct MfDevice {
                                                                arena.p, E.p, status);
               launches++;
             }
+          }
+        } else if (st.split_cnt) {
+          if constexpr (sizeof(T) == 8) {  // planned for FP64 batches only
+            mf_split<<<st.split_cnt, 256, 0, s>>>(view, split_tasks.p + st.split_off, st.j0, st.kw, arena.p, E.p,
+                                                  slices.p, expo.p);
+            mf_update_split<<<std::min(st.tile_cnt, nsm), kSplitThreads, kSplitSmem, s>>>(
+                view, tile_tasks.p + st.tile_off, st.tile_cnt, st.tile_upd, st.j0, st.kw, slices.p, expo.p, arena.p,
+                E.p, status);
+            launches += 2;
           }
         } else if (st.upd_cnt + st.etile_cnt) {
           mf_update<T><<<st.upd_cnt + st.etile_cnt, kMfThreads, 0, s>>>(

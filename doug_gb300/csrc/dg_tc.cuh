@@ -45,6 +45,29 @@ __host__ __device__ constexpr uint32_t idesc_tf32(int M, int N) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// instruction descriptor of kind::f16 with F16 operands: D F32, both K-major
+__host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// byte offset of the 16-byte chunk c (8 F16 values of K) of row r in a
+// SWIZZLE_128B K-major tile of R rows x 64 F16 values
+__host__ __device__ constexpr uint32_t sw128_chunk_f16(int r, int c) {
+  return (uint32_t)(r >> 3) * 1024u + (uint32_t)(r & 7) * 128u + (uint32_t)((c ^ r) & 7) * 16u;
+}
+
+// D[tmem] (+)= A B^T for one K step of 16 F16 values
+__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
+                                        uint32_t accumulate) {
+#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 1000)
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+#endif
+}
+
 // D[tmem] (+)= A B^T for one K step; accumulate = 0 overwrites D
 __device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
                                          uint32_t accumulate) {
@@ -135,9 +158,57 @@ __device__ __forceinline__ void tmem_load16(uint32_t taddr, float (&v)[16]) {
 #endif
 }
 
+// 2 consecutive columns of this thread's TMEM lane in each of eight 64-column
+// accumulators: v[2 s + c] = column c of accumulator s
+__device__ __forceinline__ void tmem_load_8x2(uint32_t taddr, float (&v)[16]) {
+#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 1000)
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%16];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%2,%3}, [%17];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%4,%5}, [%18];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%6,%7}, [%19];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%8,%9}, [%20];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%10,%11}, [%21];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%12,%13}, [%22];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%14,%15}, [%23];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+        "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15])
+      : "r"(taddr + 0), "r"(taddr + 64), "r"(taddr + 128), "r"(taddr + 192), "r"(taddr + 256), "r"(taddr + 320), "r"(taddr + 384), "r"(taddr + 448)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+#else
+#pragma unroll
+  for (int i = 0; i < 16; i++) v[i] = 0.f;
+#endif
+}
+
+// initialises several mbarriers (no fence: mbar_init_fence after the last)
+__device__ __forceinline__ void mbar_init_nofence(uint64_t *bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_init_fence() {
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+// announces bytes to come with bulk copies, and arrives
+__device__ __forceinline__ void mbar_expect(uint64_t *bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// bulk copy of bytes (a multiple of 16, both addresses 16-byte aligned) to shared memory
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 
 // waits for the phase with the given parity to complete, at most max_polls

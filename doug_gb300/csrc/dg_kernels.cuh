@@ -142,6 +142,26 @@ template <typename T> struct UpdTile { static constexpr int N = sizeof(T) == 8 ?
 // once E is formed; the update (Schur complement) block stays in the arena
 // for the parent's extend-add.
 
+// 1 / d of a pivot d > 0.  FP64: the division of the language is a chain of
+// some ten dependent FP64 operations, each 64 clocks and more on this pipe,
+// between one pivot and the next.  Here the single-precision reciprocal of the
+// significand (relative error below 2^-21) and one step of Chebyshev's
+// third-order iteration (r (1 + e + e^2), e = 1 - x r; Traub, Iterative Methods
+// for the Solution of Equations, 1964): three dependent FP64 operations,
+// error e^3 < 2^-63 before the last rounding.
+__device__ __forceinline__ float pivot_inverse(float d) { return 1.0f / d; }
+__device__ __forceinline__ double pivot_inverse(double d) {
+  const int hi = __double2hiint(d), lo = __double2loint(d), ex = hi >> 20;
+  if (ex < 1 || ex > 2043) return 1.0 / d;  // subnormal, or the result is, or not finite
+  const double x = __hiloint2double((hi & 0xfffff) | 0x3ff00000, lo);  // in [1, 2)
+  const float f = __int_as_float(0x3f800000 | (hi & 0xfffff) << 3 | (int)((unsigned)lo >> 29));
+  const unsigned g = (unsigned)__float_as_int(__frcp_rn(f));  // in (1/2, 1]
+  const double r = __hiloint2double((int)(g >> 3) + (896 << 20), (int)(g << 29));
+  const double e = __fma_rn(-x, r, 1.0);
+  const double y = __fma_rn(r, __fma_rn(e, e, e), r);
+  return __hiloint2double(__double2hiint(y) + ((1023 - ex) << 20), __double2loint(y));
+}
+
 // Extend-add of column b of a child's update block into column pb of the
 // parent (Dst = the parent's column base; row r of the column at
 // Dst[r * stride]): rows a >= b, by the lanes of one warp.  kEaBatch rows
@@ -292,7 +312,7 @@ mf_factor_panel(MfView v, const int *__restrict__ fronts, const double *__restri
       atomicOr(status, ERR_NOT_SPD);
       d = T(1);
     }
-    inv[j] = T(1) / d;
+    inv[j] = pivot_inverse(d);
   };
   for (int c = tid; c < k; c += nt) {
     const T x = P[(size_t)c * ldk];
@@ -564,7 +584,7 @@ __device__ __forceinline__ void chol_cta(T (*D)[kNB + 1], int jb, int *status) {
       d = T(1);
     }
     D[j][j] = d;
-    inv[j] = T(1) / d;
+    inv[j] = pivot_inverse(d);
   };
   if (tid == 0) pivot(D[0][0], 0);
   diag_sync<NAMED>();
@@ -694,7 +714,7 @@ mf_panel(MfView v, const int2 *__restrict__ tasks, int npanel, const int2 *__res
     D[i][c] = i >= c ? F[(int64_t)(j0 + c) * m + j0 + i] : T(0);
   }
   __shared__ T rd[kNB];  // FP64: reciprocals of its diagonal, no division per row
-  if (sizeof(T) == 8 && tid < jb) rd[tid] = T(1) / F[(int64_t)(j0 + tid) * m + j0 + tid];
+  if (sizeof(T) == 8 && tid < jb) rd[tid] = pivot_inverse(F[(int64_t)(j0 + tid) * m + j0 + tid]);
   if (escale) {
     constexpr int NC = EscCols<T>::N;
     __shared__ T Eb[NC][kNB + 1];
@@ -748,6 +768,60 @@ mf_panel(MfView v, const int2 *__restrict__ tasks, int npanel, const int2 *__res
   }
 }
 
+// The same for levels with few rows: four lanes per row (of L21, or column of
+// E), eight columns each, kThinRows rows per CTA.  One thread per row walks
+// 528 multiply-adds on its own, and a warp's FP64 multiply-add takes its
+// sub-partition 64 clocks: 18 us at least, 35 us for the eight warps of a
+// 256-row CTA, however few CTAs there are; this way 16 us (33 rows), with the
+// columns in the order as above.
+constexpr int kThinRows = 32, kThinLanes = 4;
+
+template <typename T>
+__global__ void __launch_bounds__(kThinRows * kThinLanes)
+mf_panel_thin(MfView v, const int2 *__restrict__ tasks, int npanel, const int2 *__restrict__ esc, int j0,
+              T *__restrict__ arena, T *__restrict__ E) {
+  constexpr int LW = kThinLanes, NC = kNB / LW, NT = kThinRows * LW;
+  __shared__ T D[kNB][kNB + 1], rd[kNB];
+  const bool escale = (int)blockIdx.x >= npanel;
+  const int2 task = escale ? esc[blockIdx.x - npanel] : tasks[blockIdx.x];
+  const int f = task.x, m = v.f_m[f], k = v.f_k[f], jb = min(kNB, k - j0);
+  T *F = arena + v.f_off[f];
+  const int tid = threadIdx.x, lane = tid & 31;
+  // eight rows per warp, a row's lanes eight apart: consecutive lanes read consecutive rows
+  const int g = lane & 7, l = lane >> 3, i = task.y + (tid >> 5) * 8 + g;
+  const bool on = escale ? i < j0 + jb : i < m;
+  // entry t of the row at p[t * st]
+  T *p = escale ? E + v.e_off[f] + (int64_t)i * round4(m) + j0 : F + (int64_t)j0 * m + i;
+  const int64_t st = escale ? 1 : m;
+  T x[NC];  // entries LW * q + l
+#pragma unroll
+  for (int q = 0; q < NC; q++) {
+    const int t = LW * q + l;
+    x[q] = T(0);
+    if (on && t < jb) x[q] = escale && i >= j0 ? (i - j0 == t ? T(1) : T(0)) : p[t * st];
+  }
+  for (int q = tid; q < kNB * kNB; q += NT) {
+    const int c = q / kNB, r = q % kNB;
+    D[r][c] = r >= c && r < jb ? F[(int64_t)(j0 + c) * m + j0 + r] : T(0);
+  }
+  __syncthreads();
+  if (tid < jb) rd[tid] = sizeof(T) == 8 ? pivot_inverse(D[tid][tid]) : D[tid][tid];
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < kNB; t++) {
+    if (t >= jb) break;
+    const T own = sizeof(T) == 8 ? x[t / LW] * rd[t] : x[t / LW] / rd[t];
+    const T xt = __shfl_sync(0xffffffffu, own, t % LW * 8 + g);
+    if (l == t % LW) x[t / LW] = xt;
+#pragma unroll
+    for (int q = t / LW; q < NC; q++)
+      if (LW * q + l > t) x[q] -= xt * D[LW * q + l][t];
+  }
+#pragma unroll
+  for (int q = 0; q < NC; q++)
+    if (on && LW * q + l < jb) p[(LW * q + l) * st] = x[q];
+}
+
 // One tile (UpdTile) of an update with the L columns [jl, jl + K), K = min(kw, k - jl).
 // Trailing-update tiles (task = {front, (ti << 16) | tj}, ti >= tj) cover rows
 // and columns from c0 = jl + K: C -= L[rows, J] L[cols, J]^T (lower part),
@@ -777,6 +851,7 @@ mf_update(MfView v, const int2 *__restrict__ tasks, int nupd, const int2 *__rest
   const int c0 = jl + K;
   const int r0 = c0 + ti * kTile;
   const int cc0 = etile ? tj * kTile : c0 + tj * kTile;
+  const bool diag = !etile && ti == tj;
   const int cend = cend_base > 0 ? min(cend_base, k) : m;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int ld = round4(m);
@@ -811,10 +886,12 @@ mf_update(MfView v, const int2 *__restrict__ tasks, int nupd, const int2 *__rest
       for (int a = 0; a < R; a++) ra[a] = As[t][tx + 16 * a];
 #pragma unroll
       for (int b = 0; b < R; b++) rb[b] = Bs[t][ty + 16 * b];
+      // (16-row blocks above the diagonal of a diagonal tile are not stored)
 #pragma unroll
       for (int a = 0; a < R; a++)
 #pragma unroll
-        for (int b = 0; b < R; b++) acc[a][b] += ra[a] * rb[b];
+        for (int b = 0; b < R; b++)
+          if (a >= b || !diag) acc[a][b] += ra[a] * rb[b];
     }
   }
   const int j0 = jl;

@@ -157,6 +157,7 @@ struct MfDevice {
     int upd_off, upd_cnt, etile_off, etile_cnt;
     int kw, cend_base;
     bool big;                     // trailing update in 128 x 128 tiles (FP32)
+    bool thin = false;            // mf_panel_thin
     int split_off = 0, split_cnt = 0;  // FP64 on the tensor cores: mf_split tasks (0: mf_update),
     int tile_off = 0, tile_cnt = 0, tile_upd = 0;  // mf_update_split tasks, trailing tiles first
   };
@@ -249,6 +250,21 @@ struct MfDevice {
       L.tiny_smem = 0;
       L.asm_off = (int)at.size();
       std::vector<int> large, tiny, pan;
+      auto one_cta = [&](int m, int k) {
+        return m <= tune.panel_rows && ((size_t)2 * m + 1) * pan_ld<T>(k) * sizeof(T) <= kPanelSmem;
+      };
+      // One CTA per front (of more than tiny_rows rows) only where at least eight
+      // per SM keep the FP64 pipes busy: a CTA alone walks its pivots and
+      // products in 100 to 300 us, which the panel pipeline spreads over the
+      // SMs.  Factorisations with the line at none, 4, 8 and 32 per SM:
+      // Poisson 129^2 1.56, 1.12, 1.11, 1.12 ms, 48 grids of 2-D cells 3.36, 2.43,
+      // 2.39, 2.42 ms, diffusion 96^3 39.1, 39.0, 39.0, 40.1 ms.
+      int npan = 0;
+      for (int q = B.lvl_ptr[(size_t)l]; q < B.lvl_ptr[(size_t)l + 1]; q++) {
+        const int f = B.lvl_fronts[(size_t)q], m = B.f_m[(size_t)f];
+        npan += one_cta(m, B.f_k[(size_t)f]);
+      }
+      const bool many = npan >= 8 * nsm;
       for (int q = B.lvl_ptr[(size_t)l]; q < B.lvl_ptr[(size_t)l + 1]; q++) {
         int f = B.lvl_fronts[(size_t)q];
         int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
@@ -256,7 +272,7 @@ struct MfDevice {
         if (m <= tune.tiny_rows) {
           tiny.push_back(f);
           L.tiny_smem = std::max(L.tiny_smem, smem);
-        } else if (m <= tune.panel_rows && ((size_t)2 * m + 1) * pan_ld<T>(k) * sizeof(T) <= kPanelSmem) {
+        } else if (many && one_cta(m, k)) {
           pan.push_back(f);
           L.pan_smem = std::max(L.pan_smem, smem);
           L.pan_maxm = std::max(L.pan_maxm, m);
@@ -286,6 +302,17 @@ struct MfDevice {
         for (int j0 = S0; j0 < std::min(S0 + SP, kmax); j0 += kNB) {
           Step st{j0, (int)df.size(), 0, (int)pf.size(), 0, (int)es.size(), 0,
                   (int)ut.size(), 0, (int)et.size(), 0, kNB, S0 + SP, false};
+          // With fewer than four of mf_panel's CTAs per SM the thin kernel's
+          // shorter chains win (45^3, all super-panels: mf_panel 34 us a step,
+          // mf_panel_thin 20 us); beyond, one thread per row has the fewer FP64
+          // operations (96^3: thin everywhere 39.3 ms, this line 39.0 ms).
+          int wide = 0;
+          for (int f : large) {
+            const int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f], c0 = j0 + std::min(kNB, k - j0);
+            if (j0 < k) wide += (m - c0 + kPanelRows - 1) / kPanelRows + (c0 + EscCols<T>::N - 1) / EscCols<T>::N;
+          }
+          st.thin = wide < 4 * nsm;
+          const int prow = st.thin ? kThinRows : kPanelRows, ecol = st.thin ? kThinRows : EscCols<T>::N;
           for (int f : large) {
             int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
             if (j0 >= k) continue;
@@ -293,8 +320,8 @@ struct MfDevice {
             // except after the mma.sync trailing update (tensor_update 0)
             if (j0 > 0 && j0 == S0 && sizeof(T) == 4 && tune.tensor_update != 1) df.push_back(f);
             const int c0 = j0 + std::min(kNB, k - j0);
-            for (int r0 = c0; r0 < m; r0 += kPanelRows) pf.push_back(make_int2(f, r0));
-            for (int e0 = 0; e0 < c0; e0 += EscCols<T>::N) es.push_back(make_int2(f, e0));
+            for (int r0 = c0; r0 < m; r0 += prow) pf.push_back(make_int2(f, r0));
+            for (int e0 = 0; e0 < c0; e0 += ecol) es.push_back(make_int2(f, e0));
             const int nt = (m - c0 + kTile - 1) / kTile;
             const int cend = std::min(S0 + SP, k);
             const int ntc = cend > c0 ? (cend - c0 + kTile - 1) / kTile : 0;
@@ -657,7 +684,8 @@ struct MfDevice {
           launches++;
         }
         if (st.panel_cnt + st.esc_cnt) {
-          mf_panel<T><<<st.panel_cnt + st.esc_cnt, kMfThreads, 0, s>>>(
+          auto *kern = st.thin ? mf_panel_thin<T> : mf_panel<T>;
+          kern<<<st.panel_cnt + st.esc_cnt, st.thin ? kThinRows * kThinLanes : kMfThreads, 0, s>>>(
               view, panel_tasks.p + st.panel_off, st.panel_cnt, esc_tasks.p + st.esc_off, st.j0, arena.p, E.p);
           launches++;
         }

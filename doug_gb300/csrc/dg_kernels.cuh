@@ -40,9 +40,10 @@ struct ChildEdge {
 
 // What a solve reads about a front, in one load: beside each large-front
 // task, and per front for the small ones.  tab: per row of the front its
-// place in the first two children's update vectors (16 bits each, kNoChild:
-// none), so that the right-hand side is gathered in one round of loads; cu0,
-// cu1: those vectors.  Children beyond the second: ch_edge[ch2 .. ch2 + nch - 2).
+// place in two children's update vectors (16 bits each, kNoChild: none), m
+// words per pair of children, so that the right-hand side is gathered in one
+// round of loads; cu0, cu1: the first two children's vectors, ch_edge[ch ..]:
+// all nch children.  nch < 0: -nch children without a table.
 struct __align__(16) SolveFront {
   int m, k;
   int64_t e_off;
@@ -51,7 +52,7 @@ struct __align__(16) SolveFront {
   int64_t uoff;            // update vector
   int64_t tab;             // offset into the child table
   int64_t cu0, cu1;
-  int nch, ch2;
+  int nch, ch;
 };
 static_assert(sizeof(SolveFront) == 80, "five 16-byte loads");
 constexpr unsigned kNoChild = 0xffffu;
@@ -1336,9 +1337,20 @@ __device__ __forceinline__ T add_children(T x, unsigned t, const T *__restrict__
   return x;
 }
 
+// and the children from the pair cp on (w: the row's table entry of pair 0)
+template <typename T>
+__device__ __forceinline__ T add_more_children(T x, const MfView &v, int64_t w, int m, int nch, int ch, int cp,
+                                               const T *__restrict__ u) {
+  for (; 2 * cp < nch; cp++)
+    x = add_children(x, v.ctab[w + (int64_t)cp * m], u, v.ch_edge[ch + 2 * cp].uoff,
+                     2 * cp + 1 < nch ? v.ch_edge[ch + 2 * cp + 1].uoff : 0);
+  return x;
+}
+
 // small fronts, forward: the first batch of E is loaded before the
 // right-hand side is assembled.  cta: this CTA's index within its bucket.
-template <typename T, int G>
+// MORE: fronts of more than two children (or without a child table) as well
+template <typename T, int G, bool MORE>
 __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__restrict__ fronts, int nf,
                                                const T *__restrict__ E, const T *__restrict__ xl,
                                                T *__restrict__ yl, T *__restrict__ uvec, int cta,
@@ -1359,7 +1371,7 @@ __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__res
   // the child table is static: read before the wait (a lane has at most 4 rows)
   unsigned t[4];
 #pragma unroll
-  for (int q = 0; q < 4; q++) t[q] = nch && sl + q * G < m ? v.ctab[f.tab + sl + q * G] : ~0u;
+  for (int q = 0; q < 4; q++) t[q] = nch > 0 && sl + q * G < m ? v.ctab[f.tab + sl + q * G] : ~0u;
   pdl_wait();
 #pragma unroll
   for (int h = 0; h < 4; h += 2) {  // two rows at once: more do not fit the registers
@@ -1375,12 +1387,13 @@ __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__res
     asm volatile("" ::: "memory");
   }
   __syncwarp(gm);
-  for (int ci = 0; ci < nch - 2; ci++) {
-    const ChildEdge ed = v.ch_edge[f.ch2 + ci];
-    const int *rel = v.relmap + ed.relmap;
-    for (int a = sl; a < ed.rc; a += G) w[rel[a]] += __ldcg(uvec + ed.uoff + a);
-    __syncwarp(gm);
-  }
+  if constexpr (MORE)  // children beyond the second, in order
+    for (int ci = nch < 0 ? 0 : 2; ci < abs(nch); ci++) {
+      const ChildEdge ed = v.ch_edge[f.ch + ci];
+      const int *rel = v.relmap + ed.relmap;
+      for (int a = sl; a < ed.rc; a += G) w[rel[a]] += __ldcg(uvec + ed.uoff + a);
+      __syncwarp(gm);
+    }
   T acc[PASS][VN];
 #pragma unroll
   for (int p = 0; p < PASS; p++)
@@ -1501,7 +1514,7 @@ struct SmallBuckets {
 // Several right-hand sides (nrhs > 1): CTA x serves right-hand side x % nrhs
 // of the work unit x / nrhs, so the CTAs that read the same E are adjacent;
 // the vectors of right-hand side k start at k * xs (xl, yl) and k * us (u).
-template <typename T>
+template <typename T, bool MORE>
 __global__ void __launch_bounds__(256, SmallMinBlocks<T>::N)
 mf_fwd_small(MfView v, const int *__restrict__ fronts, SmallBuckets sb, const T *__restrict__ E,
              const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec, int nrhs = 1, int64_t xs = 0,
@@ -1512,11 +1525,11 @@ mf_fwd_small(MfView v, const int *__restrict__ fronts, SmallBuckets sb, const T 
   xl += rk * xs;
   yl += rk * xs;
   uvec += rk * us;
-  if (b < sb.nb0) fwd_small_body<T, 8>(v, fronts, sb.cnt0, E, xl, yl, uvec, b, wsh);
+  if (b < sb.nb0) fwd_small_body<T, 8, MORE>(v, fronts, sb.cnt0, E, xl, yl, uvec, b, wsh);
   else if (b < sb.nb0 + sb.nb1)
-    fwd_small_body<T, 16>(v, fronts + sb.cnt0, sb.cnt1, E, xl, yl, uvec, b - sb.nb0, wsh);
+    fwd_small_body<T, 16, MORE>(v, fronts + sb.cnt0, sb.cnt1, E, xl, yl, uvec, b - sb.nb0, wsh);
   else
-    fwd_small_body<T, 32>(v, fronts + sb.cnt0 + sb.cnt1, sb.cnt2, E, xl, yl, uvec, b - sb.nb0 - sb.nb1, wsh);
+    fwd_small_body<T, 32, MORE>(v, fronts + sb.cnt0 + sb.cnt1, sb.cnt2, E, xl, yl, uvec, b - sb.nb0 - sb.nb1, wsh);
 }
 
 template <typename T>
@@ -1555,7 +1568,8 @@ template <typename T, int LPR> __host__ __device__ constexpr int fwd_rows() { re
 
 // the task body; b: shared memory for the right-hand side (at most the
 // front's rows), red: the warp sums of one chunk
-template <typename T, int NT, int UN, int LPR>
+// (MORE: with fronts of more than two children or without a child table)
+template <typename T, int NT, int UN, int LPR, bool MORE>
 __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const SolveFront &f, const T *__restrict__ E,
                                              const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec,
                                              T *b, T *red) {
@@ -1592,24 +1606,69 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
 #pragma unroll
   for (int q = 0; q < NP; q++) {
     const int i = tid + q * NT;
-    t[q] = nc && i < nrow ? v.ctab[tab + (i < kn ? i : rlo + i - kn)] : ~0u;
+    t[q] = nc > 0 && i < nrow ? v.ctab[tab + (i < kn ? i : rlo + i - kn)] : ~0u;
+  }
+  // A front of more than two children (MORE): the first four together, RB rows
+  // of a thread at once.  (The branch is the CTA's: predicated FP64 additions
+  // cost the pipe as much as others.)
+  constexpr bool kPairs = MORE;
+  constexpr int RB = NP == 2 ? 1 : 2;
+  unsigned t2[NP];
+  int64_t cu2 = 0, cu3 = 0;
+  if (kPairs && nc > 2) {
+    cu2 = v.ch_edge[f.ch + 2].uoff;
+    if (nc > 3) cu3 = v.ch_edge[f.ch + 3].uoff;
+#pragma unroll
+    for (int q = 0; q < NP; q++) {
+      const int i = tid + q * NT;
+      t2[q] = i < nrow ? v.ctab[tab + m + (i < kn ? i : rlo + i - kn)] : ~0u;
+    }
   }
   pdl_wait();
-  T x[NP];
+  if (kPairs && nc > 2) {
 #pragma unroll
-  for (int q = 0; q < NP; q++) {
-    const int i = tid + q * NT;
-    x[q] = add_children(i < kn ? xl[xo + i] : T(0), t[q], uvec, cu0, cu1);
+    for (int h = 0; h < NP; h += RB) {
+      if (h * NT >= nrow) break;
+      T x[RB], c[RB][4];
+#pragma unroll
+      for (int q = 0; q < RB; q++) {
+        const int i = tid + (h + q) * NT;
+        const unsigned w0 = t[h + q], w1 = t2[h + q];
+        x[q] = i < kn ? xl[xo + i] : T(0);
+        c[q][0] = (w0 & 0xffffu) != kNoChild ? __ldcg(uvec + cu0 + (w0 & 0xffffu)) : T(0);
+        c[q][1] = w0 >> 16 != kNoChild ? __ldcg(uvec + cu1 + (w0 >> 16)) : T(0);
+        c[q][2] = (w1 & 0xffffu) != kNoChild ? __ldcg(uvec + cu2 + (w1 & 0xffffu)) : T(0);
+        c[q][3] = w1 >> 16 != kNoChild ? __ldcg(uvec + cu3 + (w1 >> 16)) : T(0);
+      }
+#pragma unroll
+      for (int q = 0; q < RB; q++)
+        if (tid + (h + q) * NT < nrow) b[tid + (h + q) * NT] = ((x[q] + c[q][0]) + c[q][1] + c[q][2]) + c[q][3];
+    }
+    if (nc > 4)
+#pragma unroll 1
+      for (int i = tid; i < min(nrow, NP * NT); i += NT)
+        b[i] = add_more_children(b[i], v, tab + (i < kn ? i : rlo + i - kn), m, nc, f.ch, 2, uvec);
+  } else {
+    T x[NP];
+#pragma unroll
+    for (int q = 0; q < NP; q++) {
+      const int i = tid + q * NT;
+      x[q] = add_children(i < kn ? xl[xo + i] : T(0), t[q], uvec, cu0, cu1);
+    }
+#pragma unroll
+    for (int q = 0; q < NP; q++)
+      if (tid + q * NT < nrow) b[tid + q * NT] = x[q];
   }
-#pragma unroll
-  for (int q = 0; q < NP; q++)
-    if (tid + q * NT < nrow) b[tid + q * NT] = x[q];
-  for (int i = tid + NP * NT; i < nrow; i += NT)
-    b[i] = add_children(i < kn ? xl[xo + i] : T(0),
-                        nc ? v.ctab[tab + (i < kn ? i : rlo + i - kn)] : ~0u, uvec, cu0, cu1);
+#pragma unroll 1
+  for (int i = tid + NP * NT; i < nrow; i += NT) {
+    const int64_t w = tab + (i < kn ? i : rlo + i - kn);
+    const T s = add_children(i < kn ? xl[xo + i] : T(0), nc > 0 ? v.ctab[w] : ~0u, uvec, cu0, cu1);
+    b[i] = kPairs ? add_more_children(s, v, w, m, nc, f.ch, 1, uvec) : s;
+  }
   __syncthreads();
-  for (int ci = 0; ci < nc - 2; ci++) {  // children beyond the second, in order
-    const ChildEdge ed = v.ch_edge[f.ch2 + ci];
+  // children beyond the second (in pairs: those without a table), in order
+  for (int ci = nc < 0 ? 0 : kPairs ? nc : 2; MORE && ci < abs(nc); ci++) {
+    const ChildEdge ed = v.ch_edge[f.ch + ci];
     const int *rel = v.relmap + ed.relmap;
     for (int a = tid; a < ed.rc; a += NT) {
       const int row = rel[a], i = row < kn ? row : row >= rlo && row < rhi ? kn + row - rlo : -1;
@@ -1656,7 +1715,7 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
   }
 }
 
-template <typename T, int V>
+template <typename T, int V, bool MORE>
 __global__ void __launch_bounds__(kFwdVariants[V].nt, kFwdVariants[V].ctas)
 mf_fwd_big(MfView v, const int2 *__restrict__ tasks, const SolveFront *__restrict__ tmeta, const T *__restrict__ E,
            const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec, int nrhs = 1, int64_t xs = 0,
@@ -1666,7 +1725,7 @@ mf_fwd_big(MfView v, const int2 *__restrict__ tasks, const SolveFront *__restric
   __shared__ T red[fv.nt / 32 * fwd_rows<T, fv.lpr>()];
   pdl_trigger();
   const int task = blockIdx.x / nrhs, rk = blockIdx.x % nrhs;
-  fwd_big_body<T, fv.nt, fv.un, fv.lpr>(v, tasks[task], tmeta[task], E, xl + rk * xs, yl + rk * xs, uvec + rk * us,
+  fwd_big_body<T, fv.nt, fv.un, fv.lpr, MORE>(v, tasks[task], tmeta[task], E, xl + rk * xs, yl + rk * xs, uvec + rk * us,
                                         reinterpret_cast<T *>(smem_raw), red);
 }
 
@@ -1846,12 +1905,12 @@ mf_fwd_queue(MfView v, QueueView q, const int *__restrict__ small_fronts, const 
       const SmallBuckets sb = lvl_sb[tk.y];
       const int *fr = small_fronts + lvl_small_off[tk.y];
       const int b = tk.z;
-      if (b < sb.nb0) fwd_small_body<T, 8>(v, fr, sb.cnt0, E, xk, yk, uk, b, sm);
+      if (b < sb.nb0) fwd_small_body<T, 8, true>(v, fr, sb.cnt0, E, xk, yk, uk, b, sm);
       else if (b < sb.nb0 + sb.nb1)
-        fwd_small_body<T, 16>(v, fr + sb.cnt0, sb.cnt1, E, xk, yk, uk, b - sb.nb0, sm);
-      else fwd_small_body<T, 32>(v, fr + sb.cnt0 + sb.cnt1, sb.cnt2, E, xk, yk, uk, b - sb.nb0 - sb.nb1, sm);
+        fwd_small_body<T, 16, true>(v, fr + sb.cnt0, sb.cnt1, E, xk, yk, uk, b - sb.nb0, sm);
+      else fwd_small_body<T, 32, true>(v, fr + sb.cnt0 + sb.cnt1, sb.cnt2, E, xk, yk, uk, b - sb.nb0 - sb.nb1, sm);
     } else {
-      fwd_big_body<T, 256, 8, 32>(v, fwd_tasks[tk.z], fwd_tmeta[tk.z], E, xk, yk, uk, sm, red);
+      fwd_big_body<T, 256, 8, 32, true>(v, fwd_tasks[tk.z], fwd_tmeta[tk.z], E, xk, yk, uk, sm, red);
     }
     __syncthreads();
     if (threadIdx.x == 0) queue_publish<T>(q, done, g);

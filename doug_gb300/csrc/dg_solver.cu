@@ -176,6 +176,7 @@ struct MfDevice {
     int fwd_off, fwd_cnt, bwd_off, bwd_cnt;
     size_t fwd_smem, bwd_smem;
     int fwd_v, bwd_v;             // kFwdVariants, kBwdVariants
+    bool more;                    // fronts of more than two children, or without a child table
   };
   // the solves' work lists: of one right-hand side, of several (planned for
   // their number)
@@ -395,25 +396,20 @@ struct MfDevice {
       const int m = B.f_m[(size_t)f], cb = B.f_child_ptr[(size_t)f], nch = B.f_child_ptr[(size_t)f + 1] - cb;
       SolveFront &S = sf[(size_t)f];
       S = SolveFront{m, B.f_k[(size_t)f], eo[(size_t)f], B.f_xoff[(size_t)f] + B.f_p0[(size_t)f], B.f_xoff[(size_t)f],
-                     B.f_rows[(size_t)f], B.f_uoff[(size_t)f], (int64_t)ct.size(), 0, 0, nch, cb + 2};
+                     B.f_rows[(size_t)f], B.f_uoff[(size_t)f], (int64_t)ct.size(), 0, 0, nch, cb};
       if (nch == 0) continue;
-      ct.resize(ct.size() + (size_t)m, ~0u);
-      bool wide = false;  // an update vector beyond 16-bit places: its front's children all go row by row
-      for (int h = 0; h < std::min(nch, 2); h++) {
+      for (int h = 0; h < nch; h++) {  // an update vector beyond 16-bit places: its front's children go row by row
         const int c = B.f_children[(size_t)(cb + h)];
-        wide |= B.f_m[(size_t)c] - B.f_k[(size_t)c] >= (int)kNoChild;
+        if (B.f_m[(size_t)c] - B.f_k[(size_t)c] >= (int)kNoChild) S.nch = -nch;
       }
-      if (wide) {
-        S.nch = nch + 2;
-        S.ch2 = cb;
-        continue;
-      }
-      for (int h = 0; h < std::min(nch, 2); h++) {
+      if (S.nch < 0) continue;
+      ct.resize(ct.size() + (size_t)m * (size_t)((nch + 1) / 2), ~0u);
+      for (int h = 0; h < nch; h++) {
         const int c = B.f_children[(size_t)(cb + h)], rc = B.f_m[(size_t)c] - B.f_k[(size_t)c];
-        (h ? S.cu1 : S.cu0) = B.f_uoff[(size_t)c];
+        if (h < 2) (h ? S.cu1 : S.cu0) = B.f_uoff[(size_t)c];
         for (int q = 0; q < rc; q++) {
-          unsigned &t = ct[(size_t)(S.tab + B.relmap[(size_t)(B.f_relmap[(size_t)c] + q)])];
-          t = h ? (t & 0xffffu) | (unsigned)q << 16 : (t & 0xffff0000u) | (unsigned)q;
+          unsigned &t = ct[(size_t)(S.tab + (int64_t)(h / 2) * m + B.relmap[(size_t)(B.f_relmap[(size_t)c] + q)])];
+          t = h & 1 ? (t & 0xffffu) | (unsigned)q << 16 : (t & 0xffff0000u) | (unsigned)q;
         }
       }
     }
@@ -516,6 +512,7 @@ struct MfDevice {
       L.fwd_off = (int)fw.size();
       L.bwd_off = (int)bw.size();
       L.fwd_smem = L.bwd_smem = 0;
+      L.more = false;
       // a level with few small fronts solves them with the CTA-per-task
       // kernels too: a group of lanes per front leaves the GPU nearly idle
       // while it walks the columns of a large-k front
@@ -526,6 +523,7 @@ struct MfDevice {
       std::vector<int> large;
       for (int q = B.lvl_ptr[(size_t)l]; q < B.lvl_ptr[(size_t)l + 1]; q++) {
         const int f = B.lvl_fronts[(size_t)q], m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
+        L.more |= sf[(size_t)f].nch < 0 || sf[(size_t)f].nch > 2;
         if (m <= kSolveSmall && !thin) { sm[m <= 32 ? 0 : m <= 64 ? 1 : 2].push_back({k, f}); continue; }
         large.push_back(f);
         L.fwd_smem = std::max(L.fwd_smem, (size_t)round4(m) * sizeof(T));
@@ -621,6 +619,7 @@ struct MfDevice {
   // precision)
   template <int V>
   void set_solve_attrs(int optin, size_t smem_max) {
+    if (smem_max <= 32 * 1024) return;  // within the default 48 KB, the kernels' own few KB included
     auto set = [&](auto *k) {
       cudaFuncAttributes fa{};
       CK(cudaFuncGetAttributes(&fa, k));
@@ -628,7 +627,8 @@ struct MfDevice {
         throw CudaError{cudaErrorInvalidValue, "front too large for the shared-memory solve"};
       CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
     };
-    set(mf_fwd_big<T, V>);
+    set(mf_fwd_big<T, V, false>);
+    set(mf_fwd_big<T, V, true>);
     set(mf_bwd_big<T, V>);
   }
 
@@ -875,16 +875,16 @@ struct MfDevice {
     for (int l = 0; l < nlevels; l++) {
       const SolveLevel &L = w.levels[(size_t)l];
       if (L.small_cta) {
-        launch_level(pdl, mf_fwd_small<T>, L.small_cta * nrhs, 256, 0, s, view,
+        launch_level(pdl, L.more ? mf_fwd_small<T, true> : mf_fwd_small<T, false>, L.small_cta * nrhs, 256, 0, s, view,
                      (const int *)(w.small.p + L.small_off), L.sb, (const T *)E.p, (const T *)xl_, yl_, u_, nrhs,
                      xs, us);
         launches++;
       }
       if (L.fwd_cnt) {
-        if (L.fwd_v == 0) fwd(L, mf_fwd_big<T, 0>);
-        else if (L.fwd_v == 1) fwd(L, mf_fwd_big<T, 1>);
-        else if (L.fwd_v == 2) fwd(L, mf_fwd_big<T, 2>);
-        else fwd(L, mf_fwd_big<T, 3>);
+        if (L.fwd_v == 0) fwd(L, L.more ? mf_fwd_big<T, 0, true> : mf_fwd_big<T, 0, false>);
+        else if (L.fwd_v == 1) fwd(L, L.more ? mf_fwd_big<T, 1, true> : mf_fwd_big<T, 1, false>);
+        else if (L.fwd_v == 2) fwd(L, L.more ? mf_fwd_big<T, 2, true> : mf_fwd_big<T, 2, false>);
+        else fwd(L, L.more ? mf_fwd_big<T, 3, true> : mf_fwd_big<T, 3, false>);
         launches++;
       }
     }
@@ -1339,6 +1339,7 @@ bool robust_restriction_gpu(const Controls &c, const Csr &A, const std::vector<i
     MfBatch Bs;
     MfOptions mo;
     mo.leaf = c.nd_leaf;
+    mo.thin = c.thin_level_fronts;
     mf_build_subdomains(A, sp, sn1, mo, Bs);
     MfTune tune;
     tune.panel_rows = c.panel_rows;
@@ -1491,10 +1492,13 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
   tune.factor_overlap = c.factor_overlap;
   MfOptions mo;
   mo.leaf = c.nd_leaf;
+  mo.thin = c.thin_level_fronts;
   const bool timing = std::getenv("DG_SETUP_TIMING") != nullptr;
   const double t1 = wall();
   try {
+    mo.value_bytes = c.precision == 0 ? 8 : 4;
     if (c.fine_method == 1) mf_build_subdomains(h->S.A, h->S.sd_ptr, h->S.sd_nodes, mo, h->Bsub);
+    mo.value_bytes = 8;
     const double t2 = wall();
     if (c.levels > 1) mf_build_single(h->S.AC, mo, h->Bco);
     if (timing)

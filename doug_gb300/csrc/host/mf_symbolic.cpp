@@ -257,15 +257,144 @@ Graph graph_of_local(int n, const std::vector<int> &er, const std::vector<int> &
   return g;
 }
 
-// Local symbolic analysis for one matrix given its entries (local ids).
-void analyse(int n, const std::vector<int> &lr, const std::vector<int> &lc,
-             const std::vector<int64_t> &src, int leaf, Local &L) {
-  Graph g = graph_of_local(n, lr, lc);
-  L = Local();
-  L.n = n;
-  Dissector d(g, leaf, L);
+// One matrix between its dissection and its placement: the graph and the
+// fronts of the dissection tree.
+struct Work {
+  Graph g;
+  Local L;
+  std::vector<int> gid, lr, lc;
+  std::vector<int64_t> src;
+};
+
+void dissect(Work &w, int n, int leaf) {
+  w.g = graph_of_local(n, w.lr, w.lc);
+  w.L = Local();
+  w.L.n = n;
+  Dissector d(w.g, leaf, w.L);
   d.run();
-  finish_local(g, L);
+  finish_local(w.g, w.L);
+}
+
+// Joining levels.  A level costs at least a launch and a chain of loads
+// however little it holds, so a short one is better joined with the next:
+// consecutive levels become one, in which a front takes its descendants of
+// those levels in (their pivots first, then its own; its update rows stay).
+// Its elimination matrix holds more entries than theirs together (siblings
+// are not coupled), and its factorisation walks their pivots one after the
+// other.
+constexpr int kJoin = 4;  // levels joined at most
+
+// Of the level that the levels h .. h + g make, per h and g: entries of the
+// elimination matrices, multiply-adds of the factorisation, the most pivots
+// of a front, fronts.
+struct LevelSums {
+  double entries[kJoin] = {}, work[kJoin] = {}, pivots[kJoin] = {};
+  int fronts[kJoin] = {};
+};
+
+void add_sums(const Local &L, std::vector<LevelSums> &out) {
+  const int nf = (int)L.p0.size();
+  std::vector<double> kk((size_t)nf * kJoin);  // pivots of f and its descendants of up to j levels below
+  for (int f = 0; f < nf; f++) {               // children come first
+    const int H = L.level[(size_t)f], up = L.parent[(size_t)f];
+    const int Hp = up < 0 ? 1 << 30 : L.level[(size_t)up];
+    const double r = (double)L.rows[(size_t)f].size() - L.k[(size_t)f];
+    if ((int)out.size() <= H) out.resize((size_t)H + 1);
+    for (int j = 0; j < kJoin && j <= H; j++) {
+      double k = L.k[(size_t)f];
+      for (int c : L.children[(size_t)f]) {
+        const int jc = L.level[(size_t)c] - (H - j);
+        if (jc >= 0) k += kk[(size_t)c * kJoin + jc];
+      }
+      kk[(size_t)f * kJoin + j] = k;
+      LevelSums &S = out[(size_t)(H - j)];
+      for (int g = j; g < kJoin && H - j + g < Hp; g++) {  // f is the top front of its group
+        S.entries[g] += k * (k + r) - 0.5 * k * k;
+        S.work[g] += k * (k * k / 3 + r * k + r * r) / 2;
+        S.pivots[g] = std::max(S.pivots[g], k);
+        S.fronts[g]++;
+      }
+    }
+  }
+}
+
+// Group of each level: the cheapest split of the levels for a factorisation
+// and kNominal solves.  In microseconds, per level: both directions of a solve
+// 4.5 and the entries at the rate of short levels (FP64 250, FP32 300 per ns);
+// the factorisation 35 for the assembly, 37 per 32 pivots of the longest
+// front, 2 multiply-adds per ps.  A level of opt.thin fronts and more is not
+// joined: its fronts are solved by groups of lanes that walk the pivots.
+// Launches and time per iteration without and with: Poisson 129^2 48 and 22,
+// 141 and 87 us; diffusion 45^3 43 and 24, 330 and 284 us; elasticity 26^3 mixed
+// 36 and 25, 155 and 137 us; 128^3 mixed, whose lower levels are long, 71 and 59,
+// 1145 and 1116 us.
+std::vector<int> plan_joins(const std::vector<LevelSums> &S, const MfOptions &opt) {
+  const int N = (int)S.size();
+  constexpr double kNominal = 30;
+  const double rate = opt.value_bytes == 8 ? 250e3 : 300e3;
+  std::vector<double> best((size_t)N + 1, 0.0);
+  std::vector<int> len((size_t)N + 1, 1);
+  for (int h = N - 1; h >= 0; h--) {
+    best[(size_t)h] = 1e300;
+    for (int g = 0; g < kJoin && h + g < N; g++) {
+      const LevelSums &s = S[(size_t)h];
+      if (g > 0 && s.fronts[g] >= opt.thin) continue;
+      const double t = 2 * kNominal * (4.5 + s.entries[g] / rate) + 35 + 37 * std::ceil(s.pivots[g] / 32) +
+                       s.work[g] / 2e6 + best[(size_t)(h + g + 1)];
+      if (t < best[(size_t)h]) { best[(size_t)h] = t; len[(size_t)h] = g + 1; }
+    }
+  }
+  std::vector<int> group((size_t)N);
+  for (int h = 0; h < N; h += len[(size_t)h])
+    for (int q = h; q < std::min(N, h + len[(size_t)h]); q++) group[(size_t)q] = h;
+  return group;
+}
+
+void join(Work &w, const std::vector<int> &group) {
+  const Local &O = w.L;
+  const int nf = (int)O.p0.size();
+  std::vector<int> top((size_t)nf), id((size_t)nf, -1);  // the front that takes f in; its new number
+  bool any = false;
+  for (int f = nf - 1; f >= 0; f--) {  // parents first
+    const int up = O.parent[(size_t)f];
+    const bool in = up >= 0 && group[(size_t)O.level[(size_t)f]] == group[(size_t)O.level[(size_t)up]];
+    top[(size_t)f] = in ? top[(size_t)up] : f;
+    any |= in;
+  }
+  if (!any) return;
+  Local L;
+  L.n = O.n;
+  std::vector<std::vector<int>> members((size_t)nf);
+  for (int f = 0; f < nf; f++) members[(size_t)top[(size_t)f]].push_back(f);  // post-order
+  for (int f = 0; f < nf; f++) {
+    if (top[(size_t)f] != f) continue;
+    const int id_f = (int)L.p0.size();
+    id[(size_t)f] = id_f;
+    L.p0.push_back((int)L.perm.size());
+    L.parent.push_back(-1);
+    L.level.push_back(0);
+    L.children.emplace_back();
+    int k = 0;
+    for (int q : members[(size_t)f]) {
+      for (int i = 0; i < O.k[(size_t)q]; i++) L.perm.push_back(O.perm[(size_t)(O.p0[(size_t)q] + i)]);
+      k += O.k[(size_t)q];
+      for (int c : O.children[(size_t)q])
+        if (top[(size_t)c] == c) {
+          L.children.back().push_back(id[(size_t)c]);
+          L.parent[(size_t)id[(size_t)c]] = id_f;
+        }
+    }
+    L.k.push_back(k);
+  }
+  w.L = std::move(L);
+  finish_local(w.g, w.L);
+}
+
+// the entries of the lower triangle in the new numbering
+void place_entries(Work &w) {
+  Local &L = w.L;
+  const std::vector<int> &lr = w.lr, &lc = w.lc;
+  const std::vector<int64_t> &src = w.src;
   // keep entries of the lower triangle in the new numbering
   for (size_t q = 0; q < lr.size(); q++) {
     int a = L.iperm[(size_t)lr[q]], b = L.iperm[(size_t)lc[q]];
@@ -434,7 +563,7 @@ void finalize(MfBatch &B) {
 
 template <class F>
 void parallel_for(int n, F fn) {
-  unsigned nt = std::max(1u, std::min(std::thread::hardware_concurrency(), 32u));
+  unsigned nt = std::max(1u, std::min({std::thread::hardware_concurrency(), 32u, (unsigned)std::max(n, 1)}));
   if (n < 2 || nt < 2) {
     for (int i = 0; i < n; i++) fn(i);
     return;
@@ -461,9 +590,11 @@ void mf_build_subdomains(const Csr &A, const std::vector<int64_t> &sd_ptr,
   // every subdomain is analysed and laid out as its own batch on a host
   // thread; the pieces are then joined in subdomain order
   std::vector<MfBatch> pieces((size_t)nsd);
+  std::vector<Work> work((size_t)nsd);
   parallel_for(nsd, [&](int s) {
     int64_t b0 = sd_ptr[(size_t)s], m = sd_ptr[(size_t)s + 1] - b0;
-    std::vector<int> gid((size_t)m);
+    std::vector<int> &gid = work[(size_t)s].gid;
+    gid.resize((size_t)m);
     // local position of each global node (sorted lookup keeps memory per subdomain small)
     std::vector<std::pair<int, int>> lut((size_t)m);
     for (int64_t t = 0; t < m; t++) {
@@ -476,8 +607,8 @@ void mf_build_subdomains(const Csr &A, const std::vector<int64_t> &sd_ptr,
       if (it != lut.end() && it->first == g) return it->second;
       return -1;
     };
-    std::vector<int> lr, lc;
-    std::vector<int64_t> src;
+    std::vector<int> &lr = work[(size_t)s].lr, &lc = work[(size_t)s].lc;
+    std::vector<int64_t> &src = work[(size_t)s].src;
     for (int64_t t = 0; t < m; t++) {
       int g = gid[(size_t)t];
       for (int64_t e = A.ptr[(size_t)g]; e < A.ptr[(size_t)g + 1]; e++) {
@@ -485,9 +616,20 @@ void mf_build_subdomains(const Csr &A, const std::vector<int64_t> &sd_ptr,
         if (h >= 0) { lr.push_back((int)t); lc.push_back(h); src.push_back(e); }
       }
     }
-    Local L;
-    analyse((int)m, lr, lc, src, opt.leaf, L);
-    append(L, gid, pieces[(size_t)s]);
+    dissect(work[(size_t)s], (int)m, opt.leaf);
+  });
+  std::vector<int> group;
+  {
+    std::vector<LevelSums> sums;
+    for (const Work &w : work) add_sums(w.L, sums);
+    group = plan_joins(sums, opt);
+  }
+  parallel_for(nsd, [&](int s) {
+    Work &w = work[(size_t)s];
+    join(w, group);
+    place_entries(w);
+    append(w.L, w.gid, pieces[(size_t)s]);
+    w = Work();
   });
   // reserve the batch arrays once (they are large for big subdomains)
   {
@@ -517,17 +659,22 @@ void mf_build_subdomains(const Csr &A, const std::vector<int64_t> &sd_ptr,
 void mf_build_single(const Csr &M, const MfOptions &opt, MfBatch &out) {
   out = MfBatch();
   int n = M.nrows;
-  std::vector<int> lr, lc, gid((size_t)n);
-  std::vector<int64_t> src;
+  Work w;
+  std::vector<int> &lr = w.lr, &lc = w.lc, &gid = w.gid;
+  std::vector<int64_t> &src = w.src;
+  gid.resize((size_t)n);
   for (int i = 0; i < n; i++) {
     gid[(size_t)i] = i;
     for (int64_t e = M.ptr[(size_t)i]; e < M.ptr[(size_t)i + 1]; e++) {
       lr.push_back(i); lc.push_back(M.col[(size_t)e]); src.push_back(e);
     }
   }
-  Local L;
-  analyse(n, lr, lc, src, opt.leaf, L);
-  append(L, gid, out);
+  dissect(w, n, opt.leaf);
+  std::vector<LevelSums> sums;
+  add_sums(w.L, sums);
+  join(w, plan_joins(sums, opt));
+  place_entries(w);
+  append(w.L, gid, out);
   finalize(out);
 }
 

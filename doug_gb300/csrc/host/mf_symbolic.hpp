@@ -6,7 +6,8 @@
 // A "batch" is a set of independent sparse SPD matrices whose values come
 // from one device array (the fine matrix values for the Schwarz subdomains,
 // the coarse matrix values for the coarse solve).  Each matrix is ordered by
-// nested dissection; every separator (and every leaf) is one dense front.
+// nested dissection; every separator (and every leaf) is one dense front, or,
+// where levels are joined, a separator and its descendants of those levels.
 // Fronts of all matrices are grouped into levels of the assembly tree so that
 // one kernel launch per level factors or solves every front of that level.
 #pragma once
@@ -57,6 +58,8 @@ struct MfBatch {
 
 struct MfOptions {
   int leaf = 64;                  // nested-dissection leaf size
+  int value_bytes = 8;            // of the factors (4: FP32)
+  int thin = 1500;                // levels with fewer fronts may be joined with others
 };
 
 // Subdomain batch: the principal submatrices A(inds, inds) of the fine matrix

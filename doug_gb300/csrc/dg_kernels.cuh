@@ -25,7 +25,7 @@
 
 namespace dg {
 
-constexpr int kRedBlocks = 1024;   // partial-sum slots of every reduction
+constexpr int kRedBlocks = 1024;   // most partial sums of a reduction
 constexpr int kVecThreads = 256;
 
 // device error word bits
@@ -105,12 +105,48 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return s;
 }
 
-// sum of the kRedBlocks partials in a fixed order, by one warp; every lane
-// of warp 0 gets the result
-__device__ __forceinline__ double sum_partials(const double *part) {
+// Programmatic dependent launch of the level solves.  pdl_trigger (at the
+// start of a CTA) lets the next kernel of the stream start its CTAs once
+// every CTA of this one has started; pdl_wait returns once the previous
+// kernel has completed and its writes are visible.  The solve bodies issue
+// their first loads of E (written by the factorisation, before any of these
+// kernels) and read their index lists, and only then wait, before they read a
+// vector that the previous level wrote.  Without the launch attribute both
+// instructions do nothing.  A kernel launched this way may find in an SM's L1
+// what the kernel before it read there and other SMs have overwritten since:
+// what both read and the earlier one writes is loaded past L1 (__ldcg), as the
+// scalars and the ancestors' values are, or the launch is an ordinary one
+// (the products after the direction p).  And a load through a const
+// __restrict__ pointer may be moved above the wait: what the kernel before
+// writes is not read through one (the gather before the first level does not
+// trigger early for that reason).
+__device__ __forceinline__ void pdl_trigger() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void pdl_wait() {
+#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+
+// sum of np partials in a fixed order, by one warp; every lane gets the
+// result.  (One FP64 addition of a warp takes 64 clocks, 1024 partials a
+// microsecond: reductions over short vectors have fewer.)
+__device__ __forceinline__ double sum_partials(const double *part, int np) {
   double s = 0.0;
   int lane = threadIdx.x & 31;
-  for (int q = lane; q < kRedBlocks; q += 32) s += part[q];
+  for (int q0 = lane; q0 < np; q0 += 32 * 8) {  // eight loads in flight
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = q0 + 32 * u < np ? __ldcg(part + q0 + 32 * u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      if (q0 - lane + 32 * u >= np) break;
+      s += v[u];
+    }
+  }
   s = warp_sum(s);
   return __shfl_sync(0xffffffffu, s, 0);
 }
@@ -1306,25 +1342,6 @@ __device__ __forceinline__ void load_e_batch(const T *Ef, int ld, int m, int k, 
   }
 }
 
-// Programmatic dependent launch of the level solves.  pdl_trigger (at the
-// start of a CTA) lets the next kernel of the stream start its CTAs once
-// every CTA of this one has started; pdl_wait returns once the previous
-// kernel has completed and its writes are visible.  The solve bodies issue
-// their first loads of E (written by the factorisation, before any of these
-// kernels) and read their index lists, and only then wait, before they read a
-// vector that the previous level wrote.  Without the launch attribute both
-// instructions do nothing.
-__device__ __forceinline__ void pdl_trigger() {
-#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
-}
-__device__ __forceinline__ void pdl_wait() {
-#if defined(__CUDA_ARCH__) && __CUDA_ARCH__ >= 900
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-#endif
-}
-
 // x + the first two children's updates at a row (t: the row's child table
 // entry), children in order
 template <typename T>
@@ -1471,7 +1488,7 @@ __device__ __forceinline__ void bwd_small_body(const MfView &v, const int *__res
 #pragma unroll
   for (int q = 0; q < 4; q++) {
     const int i = sl + q * G;
-    if (i < ld) w[i] = i < k ? yl[xo + i] : (i < m ? __ldcg(xb + rw[q]) : T(0));
+    if (i < ld) w[i] = i < k ? __ldcg(yl + xo + i) : (i < m ? __ldcg(xb + rw[q]) : T(0));
   }
   __syncwarp(gm);
   T wr[PASS][VN];
@@ -1781,10 +1798,10 @@ __device__ __forceinline__ void bwd_big_body(const MfView &v, int2 tk, const Sol
 #pragma unroll
   for (int q = 0; q < kRowsAhead; q++) {
     const int i = c0 + tid + q * NT;
-    if (i < ld) w[i - c0] = i < k ? yl[xo + i] : (i < m ? __ldcg(xb + rw[q]) : T(0));
+    if (i < ld) w[i - c0] = i < k ? __ldcg(yl + xo + i) : (i < m ? __ldcg(xb + rw[q]) : T(0));
   }
   for (int i = c0 + tid + kRowsAhead * NT; i < ld; i += NT)
-    w[i - c0] = i < k ? yl[xo + i] : (i < m ? __ldcg(xb + rows[i]) : T(0));
+    w[i - c0] = i < k ? __ldcg(yl + xo + i) : (i < m ? __ldcg(xb + rows[i]) : T(0));
   __syncthreads();
   for (int cc = cs; cc < CB; cc += NCS) {  // uniform trip count: the shuffles below need whole groups
     const int c = c0 + cc;
@@ -2149,35 +2166,55 @@ __global__ void gather_subdomains(const double *__restrict__ r, const int *__res
 // crhs (in the coarse batch's local numbering) = R r
 // nrhs right-hand sides: r_k at r + k * rs, the coarse vector k at xc + k * xcs.
 // L lanes per coarse row (chosen for about 12 entries per lane), four loads
-// in flight per lane, the lane sums added by a shuffle tree.
-template <typename TR, int L>
+// in flight per lane, the lane sums added by a shuffle tree; G right-hand
+// sides at once share the entries and their conversions to FP64.
+template <typename TR, int L, int G>
 __global__ void __launch_bounds__(kVecThreads)
 restrict_to_coarse(const int64_t *__restrict__ Rp, const int *__restrict__ Rc, const TR *__restrict__ Rv,
                    const double *__restrict__ r, const int *__restrict__ cpos, double *__restrict__ xc, int nc,
                    int nrhs = 1, int64_t rs = 0, int64_t xcs = 0) {
   const int sub = threadIdx.x % L;
   const int rows_per_grid = gridDim.x * (kVecThreads / L);
+  constexpr int U = G > 1 ? 2 : 4;
   for (int a0 = blockIdx.x * (kVecThreads / L); a0 < nc; a0 += rows_per_grid) {
     const int a = a0 + threadIdx.x / L;
     const bool on = a < nc;
     const int64_t e0 = on ? Rp[a] : 0, e1 = on ? Rp[a + 1] : 0;
-    for (int k = 0; k < nrhs; k++) {
-      const double *rk = r + k * rs;
-      double s = 0.0;
-      int64_t e = e0 + sub;
-      for (; e + 3 * L < e1; e += 4 * L) {
-        const int c0 = Rc[e], c1 = Rc[e + L], c2 = Rc[e + 2 * L], c3 = Rc[e + 3 * L];
-        const double v0 = (double)Rv[e], v1 = (double)Rv[e + L], v2 = (double)Rv[e + 2 * L], v3 = (double)Rv[e + 3 * L];
-        const double x0 = rk[c0], x1 = rk[c1], x2 = rk[c2], x3 = rk[c3];
-        s += v0 * x0;
-        s += v1 * x1;
-        s += v2 * x2;
-        s += v3 * x3;
-      }
-      for (; e < e1; e += L) s += (double)Rv[e] * rk[Rc[e]];
+    for (int k0 = 0; k0 < nrhs; k0 += G) {
+      const double *rk = r + k0 * rs;
+      double s[G];
 #pragma unroll
-      for (int o = L / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, L);
-      if (on && sub == 0) xc[k * xcs + cpos[a]] = s;
+      for (int g = 0; g < G; g++) s[g] = 0.0;
+      int64_t e = e0 + sub;
+      for (; e + (U - 1) * L < e1; e += U * L) {
+        int c[U];
+        double w[U], x[U][G];
+#pragma unroll
+        for (int u = 0; u < U; u++) c[u] = Rc[e + u * L];
+#pragma unroll
+        for (int u = 0; u < U; u++) w[u] = (double)Rv[e + u * L];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+          for (int g = 0; g < G; g++) x[u][g] = k0 + g < nrhs ? rk[g * rs + c[u]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+          for (int g = 0; g < G; g++) s[g] += w[u] * x[u][g];
+      }
+      for (; e < e1; e += L) {
+        const int c = Rc[e];
+        const double w = (double)Rv[e];
+#pragma unroll
+        for (int g = 0; g < G; g++)
+          if (k0 + g < nrhs) s[g] += w * rk[g * rs + c];
+      }
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) s[g] += __shfl_down_sync(0xffffffffu, s[g], o, L);
+        if (on && sub == 0 && k0 + g < nrhs) xc[(k0 + g) * xcs + cpos[a]] = s[g];
+      }
     }
   }
 }
@@ -2204,6 +2241,7 @@ pull_prolong_dot(int n, const int *__restrict__ pull_ptr, const int *__restrict_
   // right-hand side k = csys[b]: rows g - k*vs of the matrix and the local
   // vectors at k*xls (subdomains) and k*xcs (coarse).
   __shared__ double sh[32];
+  pdl_trigger();
   double srz = 0.0, srzo = 0.0;
   const int g0 = cb ? cb[blockIdx.x] + threadIdx.x : blockIdx.x * kVecThreads + threadIdx.x;
   const int gend = cb ? cb[blockIdx.x + 1] : n;
@@ -2280,26 +2318,28 @@ enum { SC_RHO_PREV = 0, SC_RHO = 1, SC_ALPHA = 2, SC_RES = 3, SC_INIT = 4, SC_BE
 // beta of the iteration from the r.z partials: Fletcher-Reeves (DOUG) or
 // flexible Polak-Ribiere
 __device__ __forceinline__ double cg_beta(const double *part_rz, const double *part_rzo,
-                                          const double *sc, int first, int flexible, double *rho_out) {
-  const double rho = sum_partials(part_rz);
+                                          const double *sc, int first, int flexible, int np, double *rho_out) {
+  const double rho = sum_partials(part_rz, np);
   *rho_out = rho;
   if (first) return 0.0;
   if (flexible) {
-    const double rzo = sum_partials(part_rzo);
-    return __ddiv_rn(__dsub_rn(rho, rzo), sc[SC_RHO_PREV]);
+    const double rzo = sum_partials(part_rzo, np);
+    return __ddiv_rn(__dsub_rn(rho, rzo), __ldcg(sc + SC_RHO_PREV));
   }
-  return __ddiv_rn(rho, sc[SC_RHO_PREV]);
+  return __ddiv_rn(rho, __ldcg(sc + SC_RHO_PREV));
 }
 
 // p = z + beta p (p = z on the first step); beta from the r.z partials
 __global__ void __launch_bounds__(kVecThreads)
-cg_direction(int n, const double *__restrict__ z, double *__restrict__ p,
-             const double *__restrict__ part_rz, const double *__restrict__ part_rzo,
-             double *__restrict__ sc, int first, int flexible) {
+cg_direction(int n, const double *z, double *p,
+             const double *part_rz, const double *part_rzo,
+             double *sc, int first, int flexible, int np) {
   __shared__ double s_beta;
+  pdl_trigger();
+  pdl_wait();
   if (threadIdx.x < 32) {
     double rho;
-    double beta = cg_beta(part_rz, part_rzo, sc, first, flexible, &rho);
+    double beta = cg_beta(part_rz, part_rzo, sc, first, flexible, np, &rho);
     if (threadIdx.x == 0) {
       s_beta = beta;
       if (blockIdx.x == 0) { sc[SC_RHO] = rho; sc[SC_BETA] = beta; }
@@ -2308,7 +2348,7 @@ cg_direction(int n, const double *__restrict__ z, double *__restrict__ p,
   __syncthreads();
   const double beta = s_beta;
   for (int i = blockIdx.x * kVecThreads + threadIdx.x; i < n; i += gridDim.x * kVecThreads)
-    p[i] = first ? z[i] : __dadd_rn(z[i], __dmul_rn(beta, p[i]));
+    p[i] = first ? z[i] : __fma_rn(beta, p[i], z[i]);
 }
 
 // q = A p with LANES lanes per row; partial sums of p.q
@@ -2320,6 +2360,7 @@ spmv_pq(int n, const int64_t *__restrict__ Ap, const int *__restrict__ Ac, const
   const int sub = threadIdx.x % LANES;
   const int rows_per_block = kVecThreads / LANES;
   double spq = 0.0;
+  pdl_trigger();
   for (int row0 = blockIdx.x * rows_per_block; row0 < n; row0 += gridDim.x * rows_per_block) {
     const int i = row0 + threadIdx.x / LANES;
     double s = 0.0;
@@ -2349,17 +2390,38 @@ spmv_pq(int n, const int64_t *__restrict__ Ap, const int *__restrict__ Ac, const
   if (threadIdx.x == 0) part_pq[blockIdx.x] = b;
 }
 
-// x += alpha p; r -= alpha q; partial r.r  (alpha = rho / p.q)
+// end of an iteration: res = r.r, rho_prev = rho, and what the host reads
+__device__ __forceinline__ void cg_publish(double *sc, double rr, int init, volatile double *host_out,
+                                           const int *status, volatile int *host_status) {
+  // init: 1 = initial residual, 0 = end of an iteration, 2 = report only
+  if (init == 1) sc[SC_INIT] = rr;
+  else if (init == 0) { sc[SC_RES] = rr; sc[SC_RHO_PREV] = __ldcg(sc + SC_RHO); }
+  host_out[0] = rr;
+  host_out[1] = __ldcg(sc + SC_INIT);
+  host_out[2] = __ldcg(sc + SC_ALPHA);
+  host_out[3] = __ldcg(sc + SC_BETA);
+  host_out[4] = __ldcg(sc + SC_RHO);
+  host_out[5] = __ldcg(sc + SC_PQ);
+  *host_status = __ldcg(status);
+}
+
+// x += alpha p; r -= alpha q; partial r.r  (alpha = rho / p.q).  With a
+// ticket the last CTA ends the iteration (a launch of its own takes 3 us).
 __global__ void __launch_bounds__(kVecThreads)
-cg_update(int n, const double *__restrict__ p, const double *__restrict__ q,
-          double *__restrict__ x, double *__restrict__ r, double *__restrict__ sc,
-          const double *__restrict__ part_pq, double *__restrict__ part_rr) {
+cg_update(int n, const double *p, const double *q,
+          double *x, double *r, double *sc,
+          const double *part_pq, double *part_rr, int np,
+          int *ticket = nullptr, volatile double *host_out = nullptr,
+          const int *status = nullptr, volatile int *host_status = nullptr) {
   __shared__ double sh[32];
   __shared__ double s_alpha;
+  __shared__ bool s_last;
+  pdl_trigger();
+  pdl_wait();
   if (threadIdx.x < 32) {
-    const double pq = sum_partials(part_pq);
+    const double pq = sum_partials(part_pq, np);
     if (threadIdx.x == 0) {
-      const double alpha = __ddiv_rn(sc[SC_RHO], pq);
+      const double alpha = __ddiv_rn(__ldcg(sc + SC_RHO), pq);
       s_alpha = alpha;
       if (blockIdx.x == 0) { sc[SC_ALPHA] = alpha; sc[SC_PQ] = pq; }
     }
@@ -2368,13 +2430,29 @@ cg_update(int n, const double *__restrict__ p, const double *__restrict__ q,
   const double alpha = s_alpha;
   double srr = 0.0;
   for (int i = blockIdx.x * kVecThreads + threadIdx.x; i < n; i += gridDim.x * kVecThreads) {
-    x[i] = __dadd_rn(x[i], __dmul_rn(alpha, p[i]));
-    const double ri = __dsub_rn(r[i], __dmul_rn(alpha, q[i]));
+    x[i] = __fma_rn(alpha, p[i], x[i]);
+    const double ri = __fma_rn(-alpha, q[i], r[i]);
     r[i] = ri;
     srr += ri * ri;
   }
   double b = block_sum<kVecThreads>(srr, sh);
-  if (threadIdx.x == 0) part_rr[blockIdx.x] = b;
+  if (threadIdx.x == 0) {
+    part_rr[blockIdx.x] = b;
+    if (ticket) {
+      __threadfence();
+      s_last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    }
+  }
+  if (!ticket) return;
+  __syncthreads();
+  if (s_last && threadIdx.x < 32) {
+    __threadfence();
+    const double rr = sum_partials(part_rr, gridDim.x);
+    if (threadIdx.x == 0) {
+      *ticket = 0;
+      cg_publish((double *)sc, rr, 0, host_out, status, host_status);
+    }
+  }
 }
 
 // r = b - A x (FP64 true residual), partial r.r
@@ -2404,25 +2482,12 @@ residual(int n, const int64_t *__restrict__ Ap, const int *__restrict__ Ac, cons
   if (threadIdx.x == 0) part_rr[blockIdx.x] = t;
 }
 
-// finish an iteration: res = sum(part_rr); rho_prev = rho; publish to host
-__global__ void cg_finish(double *__restrict__ sc, const double *__restrict__ part_rr, int init,
+// the same after a residual in full (init: see cg_publish)
+__global__ void cg_finish(double *__restrict__ sc, const double *__restrict__ part_rr, int np, int init,
                           volatile double *__restrict__ host_out, const int *__restrict__ status,
                           volatile int *__restrict__ host_status) {
-  if (threadIdx.x < 32) {
-    const double rr = sum_partials(part_rr);
-    if (threadIdx.x == 0) {
-      // init: 1 = initial residual, 0 = end of an iteration, 2 = report only
-      if (init == 1) sc[SC_INIT] = rr;
-      else if (init == 0) { sc[SC_RES] = rr; sc[SC_RHO_PREV] = sc[SC_RHO]; }
-      host_out[0] = rr;
-      host_out[1] = sc[SC_INIT];
-      host_out[2] = sc[SC_ALPHA];
-      host_out[3] = sc[SC_BETA];
-      host_out[4] = sc[SC_RHO];
-      host_out[5] = sc[SC_PQ];
-      *host_status = *status;
-    }
-  }
+  const double rr = sum_partials(part_rr, np);
+  if (threadIdx.x == 0) cg_publish(sc, rr, init, host_out, status, host_status);
 }
 
 // ---------------------------------------------------------------------------
@@ -2434,23 +2499,50 @@ __global__ void cg_finish(double *__restrict__ sc, const double *__restrict__ pa
 // frozen while the others go on, which makes each system's iterates those of
 // its own PCG.
 // ---------------------------------------------------------------------------
-constexpr int kBatchChunk = 1024;  // rows per CTA of the batched vector kernels
+constexpr int kBatchChunk = 1024;  // rows per CTA of the batched vector kernels (or a multiple)
 enum { BS_RHO_PREV = 0, BS_RHO = 1, BS_ALPHA = 2, BS_RES = 3, BS_INIT = 4, BS_BETA = 5, BS_PQ = 6,
        BS_TRUE = 7, BS_N = 8 };
 // per-system state
 enum { BT_DONE = 0, BT_ACTIVE = 1, BT_CHECK = 2, BT_BREAKDOWN = 3 };
 // bt_scalars steps
-enum { BT_RHO = 0, BT_ALPHA = 1, BT_INIT = 2, BT_FINISH = 3, BT_CONFIRM = 4, BT_REPORT = 5 };
+enum { BT_INIT = 2, BT_FINISH = 3, BT_CONFIRM = 4, BT_REPORT = 5 };
 
+// sum of a system's chunk partials, by one warp, in a fixed order
+__device__ __forceinline__ double bt_sum(const double *part, const int *sys_cptr, int k) {
+  return sum_partials(part + sys_cptr[k], sys_cptr[k + 1] - sys_cptr[k]);
+}
+
+// p = z + beta p; every CTA forms its system's beta from the chunk partials,
+// the system's first one keeps rho and beta (a launch of one CTA for all
+// systems' scalars takes 8 us)
 __global__ void __launch_bounds__(kVecThreads)
-bt_direction(const int *__restrict__ cb, const int *__restrict__ csys, const int *__restrict__ state,
-             const double *__restrict__ bsc, const double *__restrict__ z, double *__restrict__ p, int first) {
+bt_direction(const int *cb, const int *csys, const int *sys_cptr,
+             const int *state, double *bsc, const double *part_rz,
+             const double *part_rzo, const double *z, double *p, int first,
+             int flexible) {
+  __shared__ double s_beta;
+  pdl_trigger();
+  pdl_wait();
   const int k = csys[blockIdx.x];
-  if (state[k] != BT_ACTIVE) return;
-  const double beta = bsc[k * BS_N + BS_BETA];
+  if (__ldcg(state + k) != BT_ACTIVE) return;
+  if (threadIdx.x < 32) {
+    double *sc = bsc + (size_t)k * BS_N;
+    const double rho = bt_sum(part_rz, sys_cptr, k);
+    double beta = 0.0;
+    if (!first) {
+      const double rzo = flexible ? bt_sum(part_rzo, sys_cptr, k) : 0.0;
+      beta = __ddiv_rn(flexible ? __dsub_rn(rho, rzo) : rho, __ldcg(sc + BS_RHO_PREV));
+    }
+    if (threadIdx.x == 0) {
+      s_beta = beta;
+      if ((int)blockIdx.x == sys_cptr[k]) { sc[BS_RHO] = rho; sc[BS_BETA] = beta; }
+    }
+  }
+  __syncthreads();
+  const double beta = s_beta;
   const int i1 = cb[blockIdx.x + 1];
   for (int i = cb[blockIdx.x] + threadIdx.x; i < i1; i += kVecThreads)
-    p[i] = first ? z[i] : __dadd_rn(z[i], __dmul_rn(beta, p[i]));
+    p[i] = first ? z[i] : __fma_rn(beta, p[i], z[i]);
 }
 
 // q = A p on the chunk's rows (LANES lanes per row), partial p.q
@@ -2461,6 +2553,7 @@ bt_spmv_pq(const int *__restrict__ cb, const int *__restrict__ csys, const int *
            const double *__restrict__ p, double *__restrict__ q, double *__restrict__ part_pq, int64_t vs = 0) {
   // vs > 0 (right-hand sides of one matrix): position g of vector k is row g - k*vs
   __shared__ double sh[32];
+  pdl_trigger();
   const int64_t voff = (int64_t)csys[blockIdx.x] * vs;
   const double *pc = p + voff;  // pc[c]: column c of this right-hand side
   if (state[csys[blockIdx.x]] != BT_ACTIVE) {
@@ -2499,23 +2592,126 @@ bt_spmv_pq(const int *__restrict__ cb, const int *__restrict__ csys, const int *
   if (threadIdx.x == 0) part_pq[blockIdx.x] = b;
 }
 
-// x += alpha_k p; r -= alpha_k q; partial r.r
+// q = A p for G right-hand sides of one matrix at once: a row's entries are
+// read once for them (one right-hand side per CTA spent 250 us at 32 right-hand
+// sides of 513^2 unknowns on entries that a warp's lanes read 56 bytes apart).
+// CTA b: chunk b % nch of `chunk` rows, right-hand sides G * (b / nch) ..; the
+// partial sum of right-hand side k at k * nch + chunk.  Right-hand sides that
+// left the iteration are not read.  174 us: FP64 issue takes 110.
+template <int LANES, int G>
 __global__ void __launch_bounds__(kVecThreads)
-bt_update(const int *__restrict__ cb, const int *__restrict__ csys, const int *__restrict__ state,
-          const double *__restrict__ bsc, const double *__restrict__ p, const double *__restrict__ q,
-          double *__restrict__ x, double *__restrict__ r, double *__restrict__ part_rr) {
+bt_spmv_pq_multi(int n, int nrhs, int nch, int chunk, const int *__restrict__ state, const int64_t *__restrict__ Ap,
+                 const int *__restrict__ Ac, const double *__restrict__ Av, const double *__restrict__ p,
+                 double *__restrict__ q, double *__restrict__ part_pq, int64_t vs) {
   __shared__ double sh[32];
+  pdl_trigger();
+  const int cc = blockIdx.x % nch, k0 = blockIdx.x / nch * G;
+  bool on[G], any = false;
+#pragma unroll
+  for (int g = 0; g < G; g++) {
+    on[g] = k0 + g < nrhs && state[k0 + g] == BT_ACTIVE;
+    any |= on[g];
+    if (k0 + g < nrhs && !on[g] && threadIdx.x == 0) part_pq[(k0 + g) * nch + cc] = 0.0;
+  }
+  if (!any) return;
+  p += k0 * vs;
+  q += k0 * vs;
+  const int sub = threadIdx.x % LANES;
+  constexpr int rows_per_block = kVecThreads / LANES, U = 4;
+  const int i1 = min(n, (cc + 1) * chunk);
+  double spq[G];
+#pragma unroll
+  for (int g = 0; g < G; g++) spq[g] = 0.0;
+  for (int row0 = cc * chunk; row0 < i1; row0 += rows_per_block) {
+    const int i = row0 + threadIdx.x / LANES;
+    double s[G];
+#pragma unroll
+    for (int g = 0; g < G; g++) s[g] = 0.0;
+    if (i < i1) {
+      const int64_t e1 = Ap[i + 1];
+      for (int64_t e = Ap[i] + sub; e < e1; e += U * LANES) {
+        int c[U];
+        double a[U], x[U][G];
+#pragma unroll
+        for (int u = 0; u < U; u++) c[u] = e + u * LANES < e1 ? Ac[e + u * LANES] : -1;
+#pragma unroll
+        for (int u = 0; u < U; u++) a[u] = c[u] >= 0 ? Av[e + u * LANES] : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+          for (int g = 0; g < G; g++) x[u][g] = on[g] && c[u] >= 0 ? p[g * vs + c[u]] : 0.0;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          if (e - sub + u * LANES >= e1) break;  // (no multiplications of a whole group's padding)
+#pragma unroll
+          for (int g = 0; g < G; g++)
+            if (c[u] >= 0) s[g] = __fma_rn(a[u], x[u][g], s[g]);
+        }
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < G; g++) {
+#pragma unroll
+      for (int o = LANES / 2; o > 0; o >>= 1) s[g] += __shfl_down_sync(0xffffffffu, s[g], o, LANES);
+      if (on[g] && i < i1 && sub == 0) {
+        q[g * vs + i] = s[g];
+        spq[g] += p[g * vs + i] * s[g];
+      }
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < G; g++) {
+    if (!on[g]) continue;
+    const double b = block_sum<kVecThreads>(spq[g], sh);
+    if (threadIdx.x == 0) part_pq[(k0 + g) * nch + cc] = b;
+  }
+}
+
+// x += alpha_k p; r -= alpha_k q; partial r.r; alpha as beta above.  A system
+// with p.q <= 0 or NaN leaves the iteration.
+__global__ void __launch_bounds__(kVecThreads)
+bt_update(const int *cb, const int *csys, const int *sys_cptr,
+          int *state, double *bsc, const double *part_pq,
+          int *iters, const int *dit, const double *p,
+          const double *q, double *x, double *r,
+          double *part_rr) {
+  __shared__ double sh[32];
+  __shared__ double s_alpha;
+  __shared__ bool s_on;
+  pdl_trigger();
+  pdl_wait();
   const int k = csys[blockIdx.x];
-  if (state[k] != BT_ACTIVE) {
+  if (threadIdx.x < 32) {
+    double *sc = bsc + (size_t)k * BS_N;
+    const double pq = bt_sum(part_pq, sys_cptr, k);
+    if (threadIdx.x == 0) {
+      // (the system's first CTA may set the state to BT_BREAKDOWN meanwhile:
+      // then this one finds the same p.q)
+      const bool on = __ldcg(state + k) == BT_ACTIVE;
+      const double alpha = __ddiv_rn(__ldcg(sc + BS_RHO), pq);
+      s_alpha = alpha;
+      s_on = on && pq > 0.0;
+      if (on && (int)blockIdx.x == sys_cptr[k]) {
+        sc[BS_PQ] = pq;
+        sc[BS_ALPHA] = alpha;
+        if (!(pq > 0.0)) {
+          state[k] = BT_BREAKDOWN;
+          iters[k] = *dit + 1;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (!s_on) {
     if (threadIdx.x == 0) part_rr[blockIdx.x] = 0.0;
     return;
   }
-  const double alpha = bsc[k * BS_N + BS_ALPHA];
+  const double alpha = s_alpha;
   const int i1 = cb[blockIdx.x + 1];
   double srr = 0.0;
   for (int i = cb[blockIdx.x] + threadIdx.x; i < i1; i += kVecThreads) {
-    x[i] = __dadd_rn(x[i], __dmul_rn(alpha, p[i]));
-    const double ri = __dsub_rn(r[i], __dmul_rn(alpha, q[i]));
+    x[i] = __fma_rn(alpha, p[i], x[i]);
+    const double ri = __fma_rn(-alpha, q[i], r[i]);
     r[i] = ri;
     srr += ri * ri;
   }
@@ -2563,42 +2759,22 @@ bt_residual(const int *__restrict__ cb, const int *__restrict__ csys, const int 
 // One CTA of 1024 threads.  dit: the device iteration counter (incremented by
 // BT_FINISH), so that a captured graph needs no per-iteration argument.
 __global__ void __launch_bounds__(1024)
-bt_scalars(int nsys, const int *__restrict__ sys_cptr, int step, int first, int flexible, int mixed, double tol2,
-           const double *__restrict__ part_a, const double *__restrict__ part_b, double *__restrict__ bsc,
-           int *__restrict__ state, int *__restrict__ iters, int *__restrict__ dit,
-           volatile int *__restrict__ host_counts) {
+bt_scalars(int nsys, const int *sys_cptr, int step, int mixed, double tol2,
+           const double *part_rr, double *bsc,
+           int *state, int *iters, int *dit,
+           volatile int *host_counts) {
   __shared__ int cnt[3];
+  pdl_wait();
   if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int it = *dit + (step == BT_FINISH ? 1 : 0);
+  const int it = __ldcg(dit) + (step == BT_FINISH ? 1 : 0);
   for (int k = wid; k < nsys; k += nw) {
     double *sc = bsc + (size_t)k * BS_N;
-    const int c0 = sys_cptr[k], c1 = sys_cptr[k + 1];
-    double a = 0.0, b = 0.0;
-    for (int c = c0 + lane; c < c1; c += 32) a += part_a[c];
-    a = __shfl_sync(0xffffffffu, warp_sum(a), 0);
-    if (step == BT_RHO && flexible && !first) {
-      for (int c = c0 + lane; c < c1; c += 32) b += part_b[c];
-      b = __shfl_sync(0xffffffffu, warp_sum(b), 0);
-    }
-    int stt = state[k];
+    const double a = bt_sum(part_rr, sys_cptr, k);
+    int stt = __ldcg(state + k);
     if (lane == 0) {
       switch (step) {
-        case BT_RHO:
-          if (stt == BT_ACTIVE) {
-            sc[BS_RHO] = a;
-            sc[BS_BETA] = first ? 0.0 : flexible ? __ddiv_rn(__dsub_rn(a, b), sc[BS_RHO_PREV])
-                                                 : __ddiv_rn(a, sc[BS_RHO_PREV]);
-          }
-          break;
-        case BT_ALPHA:
-          if (stt == BT_ACTIVE) {
-            sc[BS_PQ] = a;
-            sc[BS_ALPHA] = __ddiv_rn(sc[BS_RHO], a);
-            if (!(a > 0.0)) { stt = BT_BREAKDOWN; iters[k] = *dit + 1; }
-          }
-          break;
         case BT_INIT:
           sc[BS_RES] = a;
           sc[BS_INIT] = a == 0.0 ? 1.0 : a;
@@ -2610,16 +2786,16 @@ bt_scalars(int nsys, const int *__restrict__ sys_cptr, int step, int first, int 
         case BT_FINISH:
           if (stt == BT_ACTIVE) {
             sc[BS_RES] = a;
-            sc[BS_RHO_PREV] = sc[BS_RHO];
+            sc[BS_RHO_PREV] = __ldcg(sc + BS_RHO);
             iters[k] = it;
             if (a != a) stt = BT_BREAKDOWN;
-            else if (!(a / sc[BS_INIT] > tol2)) stt = mixed ? BT_CHECK : BT_DONE;
+            else if (!(a / __ldcg(sc + BS_INIT) > tol2)) stt = mixed ? BT_CHECK : BT_DONE;
           }
           break;
         case BT_CONFIRM:  // the FP64 true residual decides; r now holds it
           if (stt == BT_CHECK) {
             sc[BS_RES] = a;
-            stt = a / sc[BS_INIT] > tol2 ? BT_ACTIVE : BT_DONE;
+            stt = a / __ldcg(sc + BS_INIT) > tol2 ? BT_ACTIVE : BT_DONE;
           }
           break;
         default:  // BT_REPORT

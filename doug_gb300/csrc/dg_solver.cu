@@ -1004,9 +1004,12 @@ struct SgsDevice {
 
 // Per-system PCG state of stacked vectors: the systems of a batch
 // (dg_set_systems, vs = 0) or several right-hand sides of one matrix
-// (dg_solve_multi, vector k at k*vs).  Chunks of at most kBatchChunk
-// positions, none across two systems; one partial sum per chunk.
+// (dg_solve_multi, vector k at k*vs).  Chunks of at most `chunk` positions,
+// none across two systems; one partial sum per chunk.  With many CTAs per SM a
+// chunk is longer: every CTA of the direction and the update adds its system's
+// partial sums (32 right-hand sides of 513^2: 258 of them took each kernel 20 us).
 struct BatchCtx {
+  int chunk = kBatchChunk;
   int nsys = 0, nchunks = 0;
   int64_t vs = 0;
   DBuf<int> cb, csys, sys_cptr, state, iters, dit;
@@ -1022,14 +1025,16 @@ struct BatchCtx {
     if (host_counts) cudaFreeHost(host_counts);
   }
   // row[k] .. row[k+1]: the positions of system k in the stacked vectors
-  void build(const std::vector<int64_t> &row, int64_t vstride) {
+  void build(const std::vector<int64_t> &row, int64_t vstride, int nsm) {
     if (exec) { cudaGraphExecDestroy(exec); exec = nullptr; }
     nsys = (int)row.size() - 1;
     vs = vstride;
+    chunk = kBatchChunk;
+    while (chunk < 4 * kBatchChunk && row.back() / chunk > 16 * (int64_t)nsm) chunk *= 2;
     std::vector<int> hb(1, 0), hs, hp(1, 0);
     for (int k = 0; k < nsys; k++) {
-      for (int64_t r = row[(size_t)k]; r < row[(size_t)k + 1]; r += kBatchChunk) {
-        hb.push_back((int)std::min<int64_t>(r + kBatchChunk, row[(size_t)k + 1]));
+      for (int64_t r = row[(size_t)k]; r < row[(size_t)k + 1]; r += chunk) {
+        hb.push_back((int)std::min<int64_t>(r + chunk, row[(size_t)k + 1]));
         hs.push_back(k);
       }
       hp.push_back((int)hs.size());
@@ -1107,7 +1112,16 @@ struct dg_handle {
   int precision = 0;
   int lanes = 8;
   int r_lanes = 32;               // lanes per row of the restriction R
-  int pull_grid = kRedBlocks;     // CTAs of the single-system pull kernel: one wave
+  int vec_grid = kRedBlocks;      // CTAs (and partial sums) of the single-system vector kernels
+  int pull_grid = kRedBlocks;     // and of the pull kernel: one wave
+  int nsm = 1;
+  bool solve_pdl = false;
+  // vector kernels of grid CTAs beside the tail of the kernel before: where
+  // they fill at most the GPU once.  Per iteration without and with: 16129
+  // unknowns (64 CTAs) 82 and 76 us, 48 grids (620) 272 and 265 us; but 128^3
+  // 1118 and 1122 us, 32 right-hand sides of 513^2 (8256) 1657 and 1670 us, whose
+  // early CTAs wait where others would run.
+  bool vec_pdl(int grid) const { return solve_pdl && grid <= 8 * nsm && grid < kRedBlocks; }
   // device
   int device = 0;
   DBuf<int64_t> Ap, Rp, Pp;
@@ -1115,6 +1129,7 @@ struct dg_handle {
   DBuf<int> Ac, Rc, Pc, cpos, status;
   DBuf<double> Av, ACv, Rv, Pv, b, x, r, p, q, z, zold, hb, hx;
   DBuf<float> Rvf, Pvf;
+  DBuf<int> ticket;               // cg_update: CTAs that are done
   DBuf<double> part_rz, part_rzo, part_pq, part_rr, sc;
   std::unique_ptr<MfDevice<double>> sub64, co64;
   std::unique_ptr<MfDevice<float>> sub32;
@@ -1200,6 +1215,8 @@ double tridiag_cond(const std::vector<double> &alpha, const std::vector<double> 
   return lmin != 0 ? lmax / lmin : 0.0;
 }
 
+constexpr int kRhsGroup = 4;  // right-hand sides that share the reads of matrix entries
+
 // lanes per CSR row: about 12 entries per lane (each lane loads four at a time)
 int lanes_for(const Csr &A) {
   double avg = A.nrows ? (double)A.nnz() / A.nrows : 1;
@@ -1211,10 +1228,18 @@ int lanes_for(const Csr &A) {
   return 32;
 }
 
+// vector kernels that call pdl_wait: beside the tail of the kernel before
+template <typename... P, typename... A>
+void launch_vec(bool pdl, void (*k)(P...), int grid, cudaStream_t s, A... args) {
+  launch_level(pdl, k, grid, kVecThreads, 0, s, args...);
+}
+void launch_direction(int grid, cudaStream_t s, dg_handle *h, int first, int flexible) {
+  launch_vec(h->vec_pdl(grid), cg_direction, grid, s, h->n, (const double *)h->z.p, h->p.p, (const double *)h->part_rz.p,
+             (const double *)h->part_rzo.p, h->sc.p, first, flexible, h->pull_grid);
+}
 template <int L>
 void launch_spmv(int grid, cudaStream_t s, dg_handle *h, int first, int flexible) {
-  cg_direction<<<grid, kVecThreads, 0, s>>>(h->n, h->z.p, h->p.p, h->part_rz.p, h->part_rzo.p, h->sc.p, first,
-                                            flexible);
+  launch_direction(grid, s, h, first, flexible);
   spmv_pq<L><<<grid, kVecThreads, 0, s>>>(h->n, h->Ap.p, h->Ac.p, h->Av.p, h->p.p, h->q.p, h->part_pq.p);
 }
 template <int L>
@@ -1223,8 +1248,7 @@ void launch_resid(int grid, cudaStream_t s, dg_handle *h, const double *xx, cons
 }
 void spmv_any(int lanes, int grid, cudaStream_t s, dg_handle *h, int first, int flexible) {
   if (h->elem_mv) {  // matrix-free product with the element matrices
-    cg_direction<<<grid, kVecThreads, 0, s>>>(h->n, h->z.p, h->p.p, h->part_rz.p, h->part_rzo.p, h->sc.p, first,
-                                              flexible);
+    launch_direction(grid, s, h, first, flexible);
     if (h->el_sym)
       elem_contrib<true><<<h->el_nrun, 256, 0, s>>>(h->d_el_run.p, h->d_el_eptr.p, h->d_el_local.p,
                                                     h->d_el_poff.p, h->d_el_pack.p, h->p.p, h->d_el_c.p);
@@ -1256,16 +1280,22 @@ void resid_any(int lanes, int grid, cudaStream_t s, dg_handle *h, const double *
 }
 
 // x_c = R r with L lanes per coarse row
+template <typename TR, int L>
+void restrict_lanes(int grid, cudaStream_t s, const int64_t *Rp, const int *Rc, const TR *Rv, const double *r,
+                    const int *cpos, double *xc, int nc, int K, int64_t rs, int64_t xcs) {
+  auto *k = K > 1 ? restrict_to_coarse<TR, L, kRhsGroup> : restrict_to_coarse<TR, L, 1>;
+  k<<<grid, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs);
+}
 template <typename TR>
 void restrict_any(int lanes, int grid, cudaStream_t s, const int64_t *Rp, const int *Rc, const TR *Rv, const double *r,
                   const int *cpos, double *xc, int nc, int K, int64_t rs, int64_t xcs) {
   switch (lanes) {
-    case 1: restrict_to_coarse<TR, 1><<<grid, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
-    case 2: restrict_to_coarse<TR, 2><<<grid, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
-    case 4: restrict_to_coarse<TR, 4><<<grid, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
-    case 8: restrict_to_coarse<TR, 8><<<grid, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
-    case 16: restrict_to_coarse<TR, 16><<<grid, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
-    default: restrict_to_coarse<TR, 32><<<grid, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
+    case 1: restrict_lanes<TR, 1>(grid, s, Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
+    case 2: restrict_lanes<TR, 2>(grid, s, Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
+    case 4: restrict_lanes<TR, 4>(grid, s, Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
+    case 8: restrict_lanes<TR, 8>(grid, s, Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
+    case 16: restrict_lanes<TR, 16>(grid, s, Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
+    default: restrict_lanes<TR, 32>(grid, s, Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs); break;
   }
 }
 
@@ -1276,7 +1306,12 @@ void launch_bt(cudaStream_t s, dg_handle *h, BatchCtx &c, const Vecs &v, int res
     bt_residual<L><<<c.nchunks, kVecThreads, 0, s>>>(c.cb.p, c.csys.p, c.state.p, want, h->Ap.p, h->Ac.p, h->Av.p,
                                                      v.x, v.b, rr, c.part_rr.p, c.vs);
   else
-    bt_spmv_pq<L><<<c.nchunks, kVecThreads, 0, s>>>(c.cb.p, c.csys.p, c.state.p, h->Ap.p, h->Ac.p, h->Av.p, v.p, v.q,
+    if (c.vs > 0) {
+      const int nch = c.nchunks / c.nsys, groups = (c.nsys + kRhsGroup - 1) / kRhsGroup;
+      bt_spmv_pq_multi<L, kRhsGroup><<<nch * groups, kVecThreads, 0, s>>>(
+          h->n, c.nsys, nch, c.chunk, c.state.p, h->Ap.p, h->Ac.p, h->Av.p, v.p, v.q, c.part_pq.p, c.vs);
+    } else
+      bt_spmv_pq<L><<<c.nchunks, kVecThreads, 0, s>>>(c.cb.p, c.csys.p, c.state.p, h->Ap.p, h->Ac.p, h->Av.p, v.p, v.q,
                                                     c.part_pq.p, c.vs);
 }
 void bt_any(cudaStream_t s, dg_handle *h, BatchCtx &c, const Vecs &v, int resid, int want = -1,
@@ -1290,10 +1325,10 @@ void bt_any(cudaStream_t s, dg_handle *h, BatchCtx &c, const Vecs &v, int resid,
     default: launch_bt<32>(s, h, c, v, resid, want, rr); break;
   }
 }
-void bt_step(BatchCtx &c, cudaStream_t s, int step, int first, int mixed, double tol2, const double *pa,
-             const double *pb) {
-  bt_scalars<<<1, 1024, 0, s>>>(c.nsys, c.sys_cptr.p, step, first, mixed, mixed, tol2, pa, pb, c.bsc.p, c.state.p,
-                                c.iters.p, c.dit.p, c.d_host_counts);
+void bt_step(bool pdl, BatchCtx &c, cudaStream_t s, int step, int mixed, double tol2) {
+  launch_level(pdl, bt_scalars, 1, 1024, 0, s, c.nsys, (const int *)c.sys_cptr.p, step, mixed, tol2,
+               (const double *)c.part_rr.p, c.bsc.p, c.state.p, c.iters.p, c.dit.p,
+               (volatile int *)c.d_host_counts);
 }
 
 // q = A r with L lanes per row and the r.q partials (any CSR on the device)
@@ -1392,14 +1427,14 @@ bool robust_restriction_gpu(const Controls &c, const Csr &A, const std::vector<i
     int since_best = 0;
     for (int it = 1; it <= 10000; it++) {
       spmv_lanes(lanes, s, n, Ap.p, Ac.p, Av.p, r.p, z.p, part_rz.p);  // z = A r, r.z
-      cg_direction<<<grid, kVecThreads, 0, s>>>(n, z.p, p.p, part_rz.p, part_rz.p, sc.p, it == 1, 0);
+      cg_direction<<<grid, kVecThreads, 0, s>>>(n, z.p, p.p, part_rz.p, part_rz.p, sc.p, it == 1, 0, grid);
       gather_subdomains<double><<<grid, kVecThreads, 0, s>>>(p.p, dev.gidx.p, dev.xl.p, dev.xlen);
       dev.solve(s);
       pull_prolong_dot<double, double><<<grid, kVecThreads, 0, s>>>(
           n, pull_ptr.p, pull_idx.p, dev.xl.p, nullptr, nullptr, nullptr, nullptr, 1, p.p, qv.p, nullptr,
           part_pq.p, nullptr);  // q = B p, p.q
-      cg_update<<<grid, kVecThreads, 0, s>>>(n, p.p, qv.p, x.p, r.p, sc.p, part_pq.p, part_rr.p);
-      cg_finish<<<1, 32, 0, s>>>(sc.p, part_rr.p, 0, d_host_out, status.p, d_host_status);
+      cg_update<<<grid, kVecThreads, 0, s>>>(n, p.p, qv.p, x.p, r.p, sc.p, part_pq.p, part_rr.p, grid);
+      cg_finish<<<1, 32, 0, s>>>(sc.p, part_rr.p, grid, 0, d_host_out, status.p, d_host_status);
       CK(cudaGetLastError());
       CK(cudaStreamSynchronize(s));
       const double res = host_out[0];
@@ -1515,6 +1550,7 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
     return fail(h, DG_NO_DEVICE, "no CUDA device is visible; the solver has no CPU fallback");
   try {
     CK(cudaGetDevice(&h->device));
+    CK(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
     const SetupResult &S = h->S;
     int n = h->n;
     h->factored = false;
@@ -1592,7 +1628,7 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
     h->Ap.upload(S.A.ptr); h->Ac.upload(S.A.col); h->Av.upload(S.A.val);
     h->lanes = lanes_for(S.A);
     for (auto *v : {&h->b, &h->x, &h->r, &h->p, &h->q, &h->z, &h->zold, &h->hb, &h->hx}) v->alloc((size_t)n);
-    if (h->nsys > 0) h->bt.build(h->sys_row, 0);
+    if (h->nsys > 0) h->bt.build(h->sys_row, 0, h->nsm);
     h->mr_k = 0;  // the right-hand-side stacks are rebuilt on demand
     if (h->mr.exec) { cudaGraphExecDestroy(h->mr.exec); h->mr.exec = nullptr; }
     for (auto *v : {&h->part_rz, &h->part_rzo, &h->part_pq, &h->part_rr}) {
@@ -1602,6 +1638,8 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
     h->sc.alloc(8);
     CK(cudaMemset(h->sc.p, 0, 8 * sizeof(double)));
     h->status.alloc(1);
+    h->ticket.alloc(1);
+    CK(cudaMemset(h->ticket.p, 0, sizeof(int)));
     CK(cudaMemset(h->status.p, 0, sizeof(int)));
     if (!h->host_out) {
       CK(cudaHostAlloc(&h->host_out, 16 * sizeof(double), cudaHostAllocMapped));
@@ -1636,7 +1674,9 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pull_prolong_dot<float, float>, kVecThreads, 0));
       else
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pull_prolong_dot<double, double>, kVecThreads, 0));
-      h->pull_grid = std::max(1, std::min(kRedBlocks, nsm * std::max(occ, 1)));
+      h->vec_grid = std::max(1, std::min(kRedBlocks, (n + kVecThreads - 1) / kVecThreads));
+      h->pull_grid = std::max(1, std::min(h->vec_grid, nsm * std::max(occ, 1)));
+      h->solve_pdl = c.solve_pdl == 1;
     }
     h->Pp.upload(S.P.ptr); h->Pv.upload(S.P.val);
     std::vector<float> rf(S.R.val.begin(), S.R.val.end()), pf(S.P.val.begin(), S.P.val.end());
@@ -1754,7 +1794,8 @@ struct StackArgs {
 };
 
 int precondition(dg_handle *h, const SolvePlan &pl, cudaStream_t st, bool profile, const StackArgs &a) {
-  const int grid = kRedBlocks;
+  auto gather_grid = [](int64_t len) { return (int)std::min<int64_t>((len + kVecThreads - 1) / kVecThreads, kRedBlocks); };
+  const int rgrid = std::max(1, gather_grid((int64_t)h->S.R.nrows * h->r_lanes));
   const int n = h->n, K = a.nrhs;
   const int64_t vs = K > 1 ? n : 0;
   int nl = 0;
@@ -1766,9 +1807,9 @@ int precondition(dg_handle *h, const SolvePlan &pl, cudaStream_t st, bool profil
     CK(cudaEventRecord(h->fork_ev, st));
     CK(cudaStreamWaitEvent(h->s2, h->fork_ev, 0));
     if (profile) CK(cudaEventRecord(h->ev[4], h->s2));
-    if (pl.mixed) restrict_any<float>(h->r_lanes, grid, h->s2, h->Rp.p, h->Rc.p, h->Rvf.p, a.v.r, h->cpos.p, xc_buf,
+    if (pl.mixed) restrict_any<float>(h->r_lanes, rgrid, h->s2, h->Rp.p, h->Rc.p, h->Rvf.p, a.v.r, h->cpos.p, xc_buf,
                                        h->S.R.nrows, K, vs, xcs);
-    else restrict_any<double>(h->r_lanes, grid, h->s2, h->Rp.p, h->Rc.p, h->Rv.p, a.v.r, h->cpos.p, xc_buf,
+    else restrict_any<double>(h->r_lanes, rgrid, h->s2, h->Rp.p, h->Rc.p, h->Rv.p, a.v.r, h->cpos.p, xc_buf,
                               h->S.R.nrows, K, vs, xcs);
     nl += 1 + co->solve(h->s2, K, h->status.p);
     if (profile) CK(cudaEventRecord(h->ev[5], h->s2));
@@ -1786,14 +1827,14 @@ int precondition(dg_handle *h, const SolvePlan &pl, cudaStream_t st, bool profil
     if (pl.mixed) {
       MfDevice<float> *d = h->sub32.get();
       float *xl = K > 1 ? d->xlm.p : d->xl.p;
-      gather_subdomains<float><<<grid, kVecThreads, 0, st>>>(a.v.r, d->gidx.p, xl, d->xlen, K, vs);
+      gather_subdomains<float><<<gather_grid(d->xlen), kVecThreads, 0, st>>>(a.v.r, d->gidx.p, xl, d->xlen, K, vs);
       nl += 1 + d->solve(st, K, h->status.p);
       xl_fine = xl;
       xls = K > 1 ? d->xlen : 0;
     } else {
       MfDevice<double> *d = h->sub64.get();
       double *xl = K > 1 ? d->xlm.p : d->xl.p;
-      gather_subdomains<double><<<grid, kVecThreads, 0, st>>>(a.v.r, d->gidx.p, xl, d->xlen, K, vs);
+      gather_subdomains<double><<<gather_grid(d->xlen), kVecThreads, 0, st>>>(a.v.r, d->gidx.p, xl, d->xlen, K, vs);
       nl += 1 + d->solve(st, K, h->status.p);
       xl_fine = xl;
       xls = K > 1 ? d->xlen : 0;
@@ -1803,22 +1844,17 @@ int precondition(dg_handle *h, const SolvePlan &pl, cudaStream_t st, bool profil
   if (pl.coarse) CK(cudaStreamWaitEvent(st, h->join_ev, 0));
   const double *xc = xc_buf;
   const int64_t xcs = (pl.coarse && K > 1) ? co->xlen : 0;
-  if (pl.sgs && pl.mixed)
-    pull_prolong_dot<double, float><<<a.pg, kVecThreads, 0, st>>>(
-        n, h->pull_ptr.p, h->pull_idx.p, (const double *)xl_fine, h->Pp.p, h->Pc.p, h->Pvf.p, xc,
-        pl.mode, a.v.r, a.v.z, a.v.zold, a.part_rz, a.part_rzo, a.cb, a.csys, vs, xls, xcs);
-  else if (pl.sgs)
-    pull_prolong_dot<double, double><<<a.pg, kVecThreads, 0, st>>>(
-        n, h->pull_ptr.p, h->pull_idx.p, (const double *)xl_fine, h->Pp.p, h->Pc.p, h->Pv.p, xc,
-        pl.mode, a.v.r, a.v.z, a.v.zold, a.part_rz, a.part_rzo, a.cb, a.csys, vs, xls, xcs);
-  else if (pl.mixed)
-    pull_prolong_dot<float, float><<<a.pg, kVecThreads, 0, st>>>(
-        n, h->pull_ptr.p, h->pull_idx.p, (const float *)xl_fine, h->Pp.p, h->Pc.p, h->Pvf.p, xc,
-        pl.mode, a.v.r, a.v.z, a.v.zold, a.part_rz, a.part_rzo, a.cb, a.csys, vs, xls, xcs);
-  else
-    pull_prolong_dot<double, double><<<a.pg, kVecThreads, 0, st>>>(
-        n, h->pull_ptr.p, h->pull_idx.p, (const double *)xl_fine, h->Pp.p, h->Pc.p, h->Pv.p, xc,
-        pl.mode, a.v.r, a.v.z, a.v.zold, a.part_rz, a.part_rzo, a.cb, a.csys, vs, xls, xcs);
+  auto pull = [&](const auto *x, const auto *pv) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(x)>>;
+    using TP = std::remove_const_t<std::remove_pointer_t<decltype(pv)>>;
+    pull_prolong_dot<T, TP><<<a.pg, kVecThreads, 0, st>>>(n, h->pull_ptr.p, h->pull_idx.p, x, h->Pp.p, h->Pc.p, pv,
+                                                          xc, pl.mode, a.v.r, a.v.z, a.v.zold, a.part_rz, a.part_rzo,
+                                                          a.cb, a.csys, vs, xls, xcs);
+  };
+  if (pl.sgs && pl.mixed) pull((const double *)xl_fine, (const float *)h->Pvf.p);
+  else if (pl.sgs) pull((const double *)xl_fine, (const double *)h->Pv.p);
+  else if (pl.mixed) pull((const float *)xl_fine, (const float *)h->Pvf.p);
+  else pull((const double *)xl_fine, (const double *)h->Pv.p);
   return nl + 1;
 }
 
@@ -1869,7 +1905,7 @@ dg_status do_solve_stacked(dg_handle *h, BatchCtx &bc, const Vecs &V, int nrhs, 
     CK(cudaMemsetAsync(V.p, 0, (size_t)ntot * sizeof(double), s));
     CK(cudaMemsetAsync(V.zold, 0, (size_t)ntot * sizeof(double), s));
     bt_any(s, h, bc, V, 1, -1, V.r);  // r = b - A x0 for every system
-    bt_step(bc, s, BT_INIT, 0, mixed, tol2, bc.part_rr.p, nullptr);
+    bt_step(false, bc, s, BT_INIT, mixed, tol2);
     launches += 2;
     CK(cudaGetLastError());
     int stv = 0;
@@ -1889,20 +1925,21 @@ dg_status do_solve_stacked(dg_handle *h, BatchCtx &bc, const Vecs &V, int nrhs, 
     };
     auto iteration = [&](cudaStream_t q, int first, bool replace, bool profile) -> int {
       int nl = precondition(h, pl, q, profile, sa);
-      bt_step(bc, q, BT_RHO, first, mixed, tol2, bc.part_rz.p, bc.part_rzo.p);
       if (profile) CK(cudaEventRecord(h->ev[6], q));
-      bt_direction<<<nch, kVecThreads, 0, q>>>(bc.cb.p, bc.csys.p, bc.state.p, bc.bsc.p, V.z, V.p, first);
+      launch_vec(h->vec_pdl(nch), bt_direction, nch, q, (const int *)bc.cb.p, (const int *)bc.csys.p,
+                 (const int *)bc.sys_cptr.p, (const int *)bc.state.p, bc.bsc.p, (const double *)bc.part_rz.p,
+                 (const double *)bc.part_rzo.p, (const double *)V.z, V.p, first, mixed);
       bt_any(q, h, bc, V, 0);
       if (profile) CK(cudaEventRecord(h->ev[7], q));
-      bt_step(bc, q, BT_ALPHA, first, mixed, tol2, bc.part_pq.p, nullptr);
-      bt_update<<<nch, kVecThreads, 0, q>>>(bc.cb.p, bc.csys.p, bc.state.p, bc.bsc.p, V.p, V.q, V.x, V.r,
-                                            bc.part_rr.p);
-      nl += 5;
+      launch_vec(h->vec_pdl(nch), bt_update, nch, q, (const int *)bc.cb.p, (const int *)bc.csys.p,
+                 (const int *)bc.sys_cptr.p, bc.state.p, bc.bsc.p, (const double *)bc.part_pq.p, bc.iters.p,
+                 (const int *)bc.dit.p, (const double *)V.p, (const double *)V.q, V.x, V.r, bc.part_rr.p);
+      nl += 3;
       if (replace) {  // FP64 residual replacement, r = b - A x, of the iterating systems
         bt_any(q, h, bc, V, 1, BT_ACTIVE, V.r);
         nl++;
       }
-      bt_step(bc, q, BT_FINISH, first, mixed, tol2, bc.part_rr.p, nullptr);
+      bt_step(h->vec_pdl(nch) && !replace, bc, q, BT_FINISH, mixed, tol2);
       return nl + 1;
     };
     if (!bc.exec) {
@@ -1934,7 +1971,7 @@ dg_status do_solve_stacked(dg_handle *h, BatchCtx &bc, const Vecs &V, int nrhs, 
       }
       if (bc.host_counts[1] > 0) {  // the FP64 true residual confirms the systems the recurrence stopped
         bt_any(s, h, bc, V, 1, BT_CHECK, V.r);
-        bt_step(bc, s, BT_CONFIRM, 0, mixed, tol2, bc.part_rr.p, nullptr);
+        bt_step(false, bc, s, BT_CONFIRM, mixed, tol2);
         launches += 2;
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(s));
@@ -1945,7 +1982,7 @@ dg_status do_solve_stacked(dg_handle *h, BatchCtx &bc, const Vecs &V, int nrhs, 
     CK(cudaEventRecord(h->ev[2], s));
     // true residuals for the report (into q, which is free now)
     bt_any(s, h, bc, V, 1, -1, V.q);
-    bt_step(bc, s, BT_REPORT, 0, mixed, tol2, bc.part_rr.p, nullptr);
+    bt_step(false, bc, s, BT_REPORT, mixed, tol2);
     launches += 2;
     CK(cudaMemcpyAsync(d_x, V.x, (size_t)ntot * sizeof(double), cudaMemcpyDeviceToDevice, s));
     std::vector<double> bs((size_t)K * BS_N);
@@ -2025,7 +2062,7 @@ dg_status do_solve_multi(dg_handle *h, int K, const double *d_b, double *d_x, dg
       const int64_t nt = (int64_t)K * h->n;
       std::vector<int64_t> row((size_t)K + 1);
       for (int k = 0; k <= K; k++) row[(size_t)k] = (int64_t)k * h->n;
-      h->mr.build(row, h->n);
+      h->mr.build(row, h->n, h->nsm);
       for (auto *v : {&h->mb, &h->mx, &h->mrr, &h->mp, &h->mq, &h->mz, &h->mzold}) v->alloc((size_t)nt);
       if (h->sub32) h->sub32->ensure_multi(K);
       if (h->sub64) h->sub64->ensure_multi(K);
@@ -2049,7 +2086,7 @@ dg_status do_solve(dg_handle *h, const double *d_b, double *d_x, dg_stats *st, c
   Controls c = h->ctl;
   ctl_finish(c);
   const int n = h->n;
-  const int grid = kRedBlocks;
+  const int grid = h->vec_grid;
   const SolvePlan pl = plan_of(h, c);
   const bool fine = pl.fine, sgs = pl.sgs, coarse = pl.coarse, mixed = pl.mixed;
   int launches = 0;
@@ -2076,7 +2113,7 @@ dg_status do_solve(dg_handle *h, const double *d_b, double *d_x, dg_stats *st, c
     CK(cudaMemsetAsync(h->zold.p, 0, (size_t)n * sizeof(double), s));
     // r = b - A x0, init_norm = r.r
     resid_any(h->lanes, grid, s, h, h->x.p, h->b.p, h->r.p);
-    cg_finish<<<1, 32, 0, s>>>(h->sc.p, h->part_rr.p, 1, h->d_host_out, h->status.p, h->d_host_status);
+    cg_finish<<<1, 32, 0, s>>>(h->sc.p, h->part_rr.p, grid, 1, h->d_host_out, h->status.p, h->d_host_status);
     launches += 2;
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
@@ -2117,15 +2154,15 @@ dg_status do_solve(dg_handle *h, const double *d_b, double *d_x, dg_stats *st, c
       if (profile) CK(cudaEventRecord(h->ev[6], st));
       spmv_any(h->lanes, grid, st, h, first, mixed ? 1 : 0);
       if (profile) CK(cudaEventRecord(h->ev[7], st));
-      cg_update<<<grid, kVecThreads, 0, st>>>(n, h->p.p, h->q.p, h->x.p, h->r.p, h->sc.p, h->part_pq.p,
-                                              h->part_rr.p);
-      nl += 4;
+      launch_vec(h->vec_pdl(grid), cg_update, grid, st, n, (const double *)h->p.p, (const double *)h->q.p, h->x.p, h->r.p,
+                 h->sc.p, (const double *)h->part_pq.p, h->part_rr.p, grid, replace ? nullptr : h->ticket.p,
+                 (volatile double *)h->d_host_out, (const int *)h->status.p, (volatile int *)h->d_host_status);
+      nl += 3;
       if (replace) {  // FP64 residual replacement: r = b - A x
         resid_any(h->lanes, grid, st, h, h->x.p, h->b.p, h->r.p);
-        nl++;
+        cg_finish<<<1, 32, 0, st>>>(h->sc.p, h->part_rr.p, grid, 0, h->d_host_out, h->status.p, h->d_host_status);
+        nl += 2;
       }
-      cg_finish<<<1, 32, 0, st>>>(h->sc.p, h->part_rr.p, 0, h->d_host_out, h->status.p, h->d_host_status);
-      nl++;
       return nl;
     };
     // the steady-state iteration is captured once into a CUDA graph
@@ -2164,7 +2201,7 @@ dg_status do_solve(dg_handle *h, const double *d_b, double *d_x, dg_stats *st, c
       if (mixed && !(ratio > tol * tol)) {
         // confirm with the true FP64 residual before stopping
         resid_any(h->lanes, grid, s, h, h->x.p, h->b.p, h->r.p);
-        cg_finish<<<1, 32, 0, s>>>(h->sc.p, h->part_rr.p, 0, h->d_host_out, h->status.p, h->d_host_status);
+        cg_finish<<<1, 32, 0, s>>>(h->sc.p, h->part_rr.p, grid, 0, h->d_host_out, h->status.p, h->d_host_status);
         launches += 2;
         CK(cudaStreamSynchronize(s));
         res = h->host_out[0];
@@ -2175,7 +2212,7 @@ dg_status do_solve(dg_handle *h, const double *d_b, double *d_x, dg_stats *st, c
     if (rc == DG_OK && ratio > tol * tol && it >= maxit) rc = DG_NOT_CONVERGED;
     // true residual for the report (into q, which is free now)
     resid_any(h->lanes, grid, s, h, h->x.p, h->b.p, h->q.p);
-    cg_finish<<<1, 32, 0, s>>>(h->sc.p, h->part_rr.p, 2, h->d_host_out, h->status.p, h->d_host_status);
+    cg_finish<<<1, 32, 0, s>>>(h->sc.p, h->part_rr.p, grid, 2, h->d_host_out, h->status.p, h->d_host_status);
     launches += 2;
     CK(cudaMemcpyAsync(d_x, h->x.p, (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, s));
     CK(cudaStreamSynchronize(s));

@@ -1396,7 +1396,7 @@ __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__res
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int i = sl + (h + q) * G;
-      x[q] = add_children(i < k ? xl[xo + i] : T(0), t[h + q], uvec, cu0, cu1);
+      x[q] = add_children(i < k ? __ldcg(xl + xo + i) : T(0), t[h + q], uvec, cu0, cu1);
     }
 #pragma unroll
     for (int q = 0; q < 2; q++)
@@ -1651,7 +1651,7 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
       for (int q = 0; q < RB; q++) {
         const int i = tid + (h + q) * NT;
         const unsigned w0 = t[h + q], w1 = t2[h + q];
-        x[q] = i < kn ? xl[xo + i] : T(0);
+        x[q] = i < kn ? __ldcg(xl + xo + i) : T(0);
         c[q][0] = (w0 & 0xffffu) != kNoChild ? __ldcg(uvec + cu0 + (w0 & 0xffffu)) : T(0);
         c[q][1] = w0 >> 16 != kNoChild ? __ldcg(uvec + cu1 + (w0 >> 16)) : T(0);
         c[q][2] = (w1 & 0xffffu) != kNoChild ? __ldcg(uvec + cu2 + (w1 & 0xffffu)) : T(0);
@@ -1670,7 +1670,7 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
 #pragma unroll
     for (int q = 0; q < NP; q++) {
       const int i = tid + q * NT;
-      x[q] = add_children(i < kn ? xl[xo + i] : T(0), t[q], uvec, cu0, cu1);
+      x[q] = add_children(i < kn ? __ldcg(xl + xo + i) : T(0), t[q], uvec, cu0, cu1);
     }
 #pragma unroll
     for (int q = 0; q < NP; q++)
@@ -1679,7 +1679,7 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
 #pragma unroll 1
   for (int i = tid + NP * NT; i < nrow; i += NT) {
     const int64_t w = tab + (i < kn ? i : rlo + i - kn);
-    const T s = add_children(i < kn ? xl[xo + i] : T(0), nc > 0 ? v.ctab[w] : ~0u, uvec, cu0, cu1);
+    const T s = add_children(i < kn ? __ldcg(xl + xo + i) : T(0), nc > 0 ? v.ctab[w] : ~0u, uvec, cu0, cu1);
     b[i] = kPairs ? add_more_children(s, v, w, m, nc, f.ch, 1, uvec) : s;
   }
   __syncthreads();
@@ -1803,9 +1803,17 @@ __device__ __forceinline__ void bwd_big_body(const MfView &v, int2 tk, const Sol
   for (int i = c0 + tid + kRowsAhead * NT; i < ld; i += NT)
     w[i - c0] = i < k ? __ldcg(yl + xo + i) : (i < m ? __ldcg(xb + rows[i]) : T(0));
   __syncthreads();
-  for (int cc = cs; cc < CB; cc += NCS) {  // uniform trip count: the shuffles below need whole groups
-    const int c = c0 + cc;
-    T s = T(0);
+  // the column sums of all passes are reduced together: FP64 additions across
+  // lanes cost as much as the multiplications (16 of a lane's 56 operations
+  // with 150 rows and a reduction per pass)
+  constexpr int NP = CB / NCS;
+  static_assert(NP == 1 || NP == 2 || NP == 4, "passes over the columns");
+  T s[4];
+#pragma unroll
+  for (int h = 0; h < 4; h++) s[h] = T(0);
+#pragma unroll
+  for (int h = 0; h < NP; h++) {
+    const int cc = cs + h * NCS, c = c0 + cc;
     if (cc < jb) {
       for (int i = c0 + rq * VN; i < m; i += UN * RS) {
         if (i != c0 + rq * VN) load_batch(c, i);  // every column's first batch was loaded ahead
@@ -1816,17 +1824,30 @@ __device__ __forceinline__ void bwd_big_body(const MfView &v, int2 tk, const Sol
             T x[VN];
             Vec16<T>::lds(w + ii - c0, x);
 #pragma unroll
-            for (int q = 0; q < VN; q++) s += e[u][q] * x[q];
+            for (int q = 0; q < VN; q++) s[h] += e[u][q] * x[q];
           }
         }
       }
     }
-    // the next column's first batch is in flight during this column's reduction
-    if (cc + NCS < CB) load_batch(c + NCS, c0 + rq * VN);
-#pragma unroll
-    for (int o = LPC / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (rq == 0 && cc < jb) xl[xo + c] = s;
+    if (h + 1 < NP) load_batch(c + NCS, c0 + rq * VN);
   }
+  // h of this lane's sum, which lane of its group writes it
+  int h = 0;
+  T t;
+  if constexpr (NP == 4) {
+    t = reduce4<T, LPC>(s, rq, 0xffffffffu);
+    h = rq / (LPC / 4);
+  } else {
+    t = s[0];
+    if constexpr (NP == 2) {
+      const bool hi = (rq & (LPC / 2)) != 0;
+      t = (hi ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi ? s[0] : s[1], LPC / 2);
+      h = hi;
+    }
+#pragma unroll
+    for (int o = LPC / (2 * NP); o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  }
+  if (rq % (LPC / NP) == 0 && cs + h * NCS < jb) xl[xo + c0 + cs + h * NCS] = t;
 }
 
 template <typename T, int V>

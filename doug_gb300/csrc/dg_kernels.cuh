@@ -2188,7 +2188,8 @@ __global__ void gather_subdomains(const double *__restrict__ r, const int *__res
 // nrhs right-hand sides: r_k at r + k * rs, the coarse vector k at xc + k * xcs.
 // L lanes per coarse row (chosen for about 12 entries per lane), four loads
 // in flight per lane, the lane sums added by a shuffle tree; G right-hand
-// sides at once share the entries and their conversions to FP64.
+// sides at once share the entries and their conversions to FP64 (blockIdx.y:
+// groups of them).
 template <typename TR, int L, int G>
 __global__ void __launch_bounds__(kVecThreads)
 restrict_to_coarse(const int64_t *__restrict__ Rp, const int *__restrict__ Rc, const TR *__restrict__ Rv,
@@ -2201,7 +2202,7 @@ restrict_to_coarse(const int64_t *__restrict__ Rp, const int *__restrict__ Rc, c
     const int a = a0 + threadIdx.x / L;
     const bool on = a < nc;
     const int64_t e0 = on ? Rp[a] : 0, e1 = on ? Rp[a + 1] : 0;
-    for (int k0 = 0; k0 < nrhs; k0 += G) {
+    for (int k0 = blockIdx.y * G; k0 < nrhs; k0 += gridDim.y * G) {
       const double *rk = r + k0 * rs;
       double s[G];
 #pragma unroll

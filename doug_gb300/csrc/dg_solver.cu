@@ -1283,8 +1283,9 @@ void resid_any(int lanes, int grid, cudaStream_t s, dg_handle *h, const double *
 template <typename TR, int L>
 void restrict_lanes(int grid, cudaStream_t s, const int64_t *Rp, const int *Rc, const TR *Rv, const double *r,
                     const int *cpos, double *xc, int nc, int K, int64_t rs, int64_t xcs) {
-  auto *k = K > 1 ? restrict_to_coarse<TR, L, kRhsGroup> : restrict_to_coarse<TR, L, 1>;
-  k<<<grid, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs);
+  auto *k = K > 1 ? restrict_to_coarse<TR, L, 2 * kRhsGroup> : restrict_to_coarse<TR, L, 1>;
+  const dim3 g((unsigned)grid, K > 1 ? (unsigned)std::min((K + 2 * kRhsGroup - 1) / (2 * kRhsGroup), 64) : 1u);
+  k<<<g, kVecThreads, 0, s>>>(Rp, Rc, Rv, r, cpos, xc, nc, K, rs, xcs);
 }
 template <typename TR>
 void restrict_any(int lanes, int grid, cudaStream_t s, const int64_t *Rp, const int *Rc, const TR *Rv, const double *r,

@@ -320,18 +320,20 @@ void add_sums(const Local &L, std::vector<LevelSums> &out) {
 
 // Group of each level: the cheapest split of the levels for a factorisation
 // and kNominal solves.  In microseconds, per level: both directions of a solve
-// 4.5 and the entries at the rate of short levels (FP64 250, FP32 300 per ns);
+// 4.5 and the entries at the rate of short levels (FP64 250, FP32 500 per ns);
 // the factorisation 35 for the assembly, 37 per 32 pivots of the longest
 // front, 2 multiply-adds per ps.  A level of opt.thin fronts and more is not
 // joined: its fronts are solved by groups of lanes that walk the pivots.
 // Launches and time per iteration without and with: Poisson 129^2 48 and 22,
 // 141 and 87 us; diffusion 45^3 43 and 24, 330 and 284 us; elasticity 26^3 mixed
-// 36 and 25, 155 and 137 us; 128^3 mixed, whose lower levels are long, 71 and 59,
-// 1145 and 1116 us.
+// 36 and 23, 155 and 127 us; 128^3 mixed, whose lower levels are long, 71 and 59,
+// 1145 and 1116 us.  FP32 at 300 per ns joins too little (elasticity 138 us), at
+// 1200 too much where several right-hand sides share a level (32 of 513^2: 1591 us
+// against 1518).
 std::vector<int> plan_joins(const std::vector<LevelSums> &S, const MfOptions &opt) {
   const int N = (int)S.size();
   constexpr double kNominal = 30;
-  const double rate = opt.value_bytes == 8 ? 250e3 : 300e3;
+  const double rate = opt.value_bytes == 8 ? 250e3 : 500e3;
   std::vector<double> best((size_t)N + 1, 0.0);
   std::vector<int> len((size_t)N + 1, 1);
   for (int h = N - 1; h >= 0; h--) {

@@ -2572,12 +2572,9 @@ template <int LANES>
 __global__ void __launch_bounds__(kVecThreads)
 bt_spmv_pq(const int *__restrict__ cb, const int *__restrict__ csys, const int *__restrict__ state,
            const int64_t *__restrict__ Ap, const int *__restrict__ Ac, const double *__restrict__ Av,
-           const double *__restrict__ p, double *__restrict__ q, double *__restrict__ part_pq, int64_t vs = 0) {
-  // vs > 0 (right-hand sides of one matrix): position g of vector k is row g - k*vs
+           const double *__restrict__ p, double *__restrict__ q, double *__restrict__ part_pq) {
   __shared__ double sh[32];
   pdl_trigger();
-  const int64_t voff = (int64_t)csys[blockIdx.x] * vs;
-  const double *pc = p + voff;  // pc[c]: column c of this right-hand side
   if (state[csys[blockIdx.x]] != BT_ACTIVE) {
     if (threadIdx.x == 0) part_pq[blockIdx.x] = 0.0;
     return;
@@ -2590,18 +2587,18 @@ bt_spmv_pq(const int *__restrict__ cb, const int *__restrict__ csys, const int *
     const int i = row0 + threadIdx.x / LANES;
     double s = 0.0;
     if (i < i1) {
-      int64_t e = Ap[i - voff] + sub;
-      const int64_t e1 = Ap[i - voff + 1];
+      int64_t e = Ap[i] + sub;
+      const int64_t e1 = Ap[i + 1];
       for (; e + 3 * LANES < e1; e += 4 * LANES) {
         const int c0 = Ac[e], c1 = Ac[e + LANES], c2 = Ac[e + 2 * LANES], c3 = Ac[e + 3 * LANES];
         const double a0 = Av[e], a1 = Av[e + LANES], a2 = Av[e + 2 * LANES], a3 = Av[e + 3 * LANES];
-        const double p0 = pc[c0], p1 = pc[c1], p2 = pc[c2], p3 = pc[c3];
+        const double p0 = p[c0], p1 = p[c1], p2 = p[c2], p3 = p[c3];
         s = __fma_rn(a0, p0, s);
         s = __fma_rn(a1, p1, s);
         s = __fma_rn(a2, p2, s);
         s = __fma_rn(a3, p3, s);
       }
-      for (; e < e1; e += LANES) s = __fma_rn(Av[e], pc[Ac[e]], s);
+      for (; e < e1; e += LANES) s = __fma_rn(Av[e], p[Ac[e]], s);
     }
 #pragma unroll
     for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, LANES);

@@ -1312,8 +1312,8 @@ void launch_bt(cudaStream_t s, dg_handle *h, BatchCtx &c, const Vecs &v, int res
       bt_spmv_pq_multi<L, kRhsGroup><<<nch * groups, kVecThreads, 0, s>>>(
           h->n, c.nsys, nch, c.chunk, c.state.p, h->Ap.p, h->Ac.p, h->Av.p, v.p, v.q, c.part_pq.p, c.vs);
     } else
-      bt_spmv_pq<L><<<c.nchunks, kVecThreads, 0, s>>>(c.cb.p, c.csys.p, c.state.p, h->Ap.p, h->Ac.p, h->Av.p, v.p, v.q,
-                                                    c.part_pq.p, c.vs);
+        bt_spmv_pq<L><<<c.nchunks, kVecThreads, 0, s>>>(c.cb.p, c.csys.p, c.state.p, h->Ap.p, h->Ac.p, h->Av.p, v.p, v.q,
+                                                      c.part_pq.p);
 }
 void bt_any(cudaStream_t s, dg_handle *h, BatchCtx &c, const Vecs &v, int resid, int want = -1,
             double *rr = nullptr) {

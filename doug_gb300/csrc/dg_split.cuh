@@ -109,8 +109,9 @@ mf_split(MfView v, const int4 *__restrict__ tasks, int jl, int kw, const double 
   }
 }
 
-// sum_s d[s] 2^(8 (7 - s)) * 2^(ex - 2112), rounded to nearest; the d[s] are
-// integers of at most 2^24, ex the sum of the two rows' biased exponents
+// sum_s d[s] 2^(8 (7 - s)) * 2^(ex - 2112), rounded to nearest (subnormal
+// numbers too); the d[s] are integers of at most 2^24, ex the sum of the two
+// rows' biased exponents
 __device__ __forceinline__ double split_value(const int (&d)[kSplit], int ex) {
   long long h = ((long long)d[0] << 24) + ((long long)d[1] << 16) + ((long long)d[2] << 8) + d[3];
   const long long l = ((long long)d[4] << 24) + ((long long)d[5] << 16) + ((long long)d[6] << 8) + d[7];
@@ -127,10 +128,12 @@ __device__ __forceinline__ double split_value(const int (&d)[kSplit], int ex) {
   const int n = a ? __clzll((long long)a) : 64 + __clzll((long long)b);
   const unsigned long long top = n == 0 ? a : n < 64 ? a << n | b >> (64 - n) : b << (n & 63);
   const int fe = 1023 + 80 - n + ex - 2112;  // biased exponent of the leading bit
-  const unsigned long long bits = ((unsigned long long)(fe - 1) << 52) + (top >> 11) + ((top >> 10) & 1);
+  const int drop = max(11, 12 - fe);  // bits of top below the result's last one
+  const unsigned long long bits = ((unsigned long long)max(fe - 1, 0) << 52) + ((top >> 1) >> ((drop - 1) & 63)) +
+                                  ((top >> ((drop - 1) & 63)) & 1);
   double r = __longlong_as_double((long long)bits);
-  if (fe < 1 || (a | b) == 0) r = 0.0;  // below the smallest normal number, or zero
-  if (fe > 2045) r = __longlong_as_double(0x7ff0000000000000ll);
+  if (fe > 2046) r = __longlong_as_double(0x7ff0000000000000ll);
+  if (drop > 64 || (a | b) == 0) r = 0.0;  // below half of the smallest subnormal number, or zero
   if (ex >= kSplitNan) r = __longlong_as_double(0x7ff8000000000000ll);
   return neg ? -r : r;
 }

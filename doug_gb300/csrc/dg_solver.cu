@@ -84,6 +84,7 @@ struct MfTune {
   int super_panel = kSuperPanel;         // columns of L per trailing update of a large front (multiple of 32)
   long long queue_wait_cycles = kQueueWaitCycles;  // solve_schedule 1: limit of one dependency wait
   int queue_skip_publish = -1;           // solve_schedule 1: forward entry whose done flag is withheld (tests)
+  long long update_wait_polls = kTcWaitPolls;  // mf_update_split: polls of its epilogue's wait (tests)
 };
 
 // Launch k with programmatic stream serialisation when pdl is set: its CTAs
@@ -119,6 +120,7 @@ struct MfDevice {
   int tiny_threads = 64;
   int tensor_update = 1;   // FP32 super-panel updates: 1 tcgen05 + TMEM, 0 mma.sync
   long long q_wait_cycles = kQueueWaitCycles;  // queue schedule: limit of one dependency wait
+  long long update_wait_polls = kTcWaitPolls;
   int q_skip_publish = -1;  // queue schedule: forward list entry whose done flag is withheld (tests)
   // dependency-driven schedule of the solves (solve_schedule 1)
   bool queue = false;
@@ -433,6 +435,7 @@ struct MfDevice {
     tensor_update = tune.tensor_update;
     q_wait_cycles = tune.queue_wait_cycles;
     q_skip_publish = tune.queue_skip_publish;
+    update_wait_polls = tune.update_wait_polls;
     if constexpr (sizeof(T) == 4)
       if (tensor_update == 1)
         CK(cudaFuncSetAttribute(mf_update_big_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
@@ -716,7 +719,7 @@ struct MfDevice {
                                                   slices.p, expo.p);
             mf_update_split<<<std::min(st.tile_cnt, nsm), kSplitThreads, kSplitSmem, s>>>(
                 view, tile_tasks.p + st.tile_off, st.tile_cnt, st.tile_upd, st.j0, st.kw, slices.p, expo.p, arena.p,
-                E.p, status);
+                E.p, status, update_wait_polls);
             launches += 2;
           }
         } else if (st.upd_cnt + st.etile_cnt) {
@@ -1386,6 +1389,7 @@ bool robust_restriction_gpu(const Controls &c, const Csr &A, const std::vector<i
     tune.super_panel = c.super_panel;
     tune.queue_wait_cycles = c.queue_wait_cycles;
     tune.queue_skip_publish = c.queue_skip_publish;
+    tune.update_wait_polls = c.update_wait_polls < 0 ? kTcWaitPolls : c.update_wait_polls;
     CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     CK(cudaHostAlloc(&host_out, 16 * sizeof(double), cudaHostAllocMapped));
     CK(cudaHostAlloc(&host_status, sizeof(int), cudaHostAllocMapped));
@@ -1523,6 +1527,7 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
   tune.super_panel = c.super_panel;
   tune.queue_wait_cycles = c.queue_wait_cycles;
   tune.queue_skip_publish = c.queue_skip_publish;
+  tune.update_wait_polls = c.update_wait_polls < 0 ? kTcWaitPolls : c.update_wait_polls;
   tune.schedule = c.solve_schedule;
   tune.pdl = c.solve_pdl;
   tune.factor_overlap = c.factor_overlap;
@@ -2300,9 +2305,10 @@ dg_status dg_set_option(dg_handle *h, const char *name, const char *value) {
     h->ready = false;
     return DG_OK;
   }
-  if (w1 == "queue_wait_cycles" || w1 == "queue_skip_publish") {
-    // failure tests of the dependency-driven schedule: a short wait limit and
-    // a forward task whose done flag is never published
+  if (w1 == "queue_wait_cycles" || w1 == "queue_skip_publish" || w1 == "update_wait_polls") {
+    // failure tests: of the dependency-driven schedule a short wait limit and
+    // a forward task whose done flag is never published, of the FP64
+    // tensor-core update the polls of its epilogue's wait (-1: the usual limit)
     long long v = 0;
     try {
       size_t used = 0;
@@ -2314,6 +2320,9 @@ dg_status dg_set_option(dg_handle *h, const char *name, const char *value) {
     if (w1 == "queue_wait_cycles") {
       if (v < 1) return fail(h, DG_BAD_INPUT, "queue_wait_cycles must be positive");
       h->ctl.queue_wait_cycles = v;
+    } else if (w1 == "update_wait_polls") {
+      if (v < -1) return fail(h, DG_BAD_INPUT, "bad update_wait_polls");
+      h->ctl.update_wait_polls = v;
     } else {
       if (v < -1 || v > INT_MAX) return fail(h, DG_BAD_INPUT, "bad queue_skip_publish");
       h->ctl.queue_skip_publish = (int)v;

@@ -156,25 +156,38 @@ __device__ __forceinline__ double split_value(const int (&d)[kSplit], int ex) {
 // hundred integer operations per entry; FP64 operations would take longer:
 // one per entry is the subtraction), so 16 warps run it, and its loop is not
 // unrolled: cold code costs a short launch 10 us.  64 subdomains of 96^3:
-// all super-panel updates 72 ms -> 10 ms.  Every wait is bounded: on a timeout the CTA sets
-// ERR_WAIT, waits once more for its copies and MMAs in flight and frees its
-// tensor memory.
+// all super-panel updates 72 ms -> 10 ms.  Every wait is bounded: whoever runs
+// out of polls (the epilogue has epi_polls of them a tile) sets ERR_WAIT and
+// tells the others, the copying warp waits once more for its copies and MMAs
+// in flight, and the CTA frees its tensor memory.
 constexpr int kSplitEpi = 512;  // threads of the epilogue
 constexpr int kSplitThreads = kSplitEpi + 32;
+
+// waits for a phase as tc::mbar_wait does, but not on after someone gave up
+__device__ __forceinline__ bool split_wait(uint64_t *bar, uint32_t parity, long long polls, const volatile int *gave_up) {
+  constexpr int kChunk = 1024;
+  for (; polls > 0; polls -= kChunk) {
+    if (tc::mbar_wait(bar, parity, polls < kChunk ? polls : kChunk)) return true;
+    if (*gave_up) return false;
+  }
+  return false;
+}
 
 __global__ void __launch_bounds__(kSplitThreads, 1)
 mf_update_split(MfView v, const int4 *__restrict__ tasks, int ntasks, int nupd, int jl, int kw,
                 const unsigned char *__restrict__ slices, const int *__restrict__ expo, double *__restrict__ arena,
-                double *__restrict__ E, int *__restrict__ status) {
+                double *__restrict__ E, int *__restrict__ status, long long epi_polls) {
   extern __shared__ unsigned char tc_raw[];
   unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) &
                                                           ~static_cast<uintptr_t>(1023));
   constexpr int G = kSplit / 2;  // slice groups of the second chunk: {3,4} {2,5} {1,6} {0,7}
   __shared__ __align__(8) uint64_t full0[kSplit], full1[G], freed[G], done, empty, drain;
   __shared__ uint32_t tmem_slot;
+  __shared__ volatile int gave_up;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (warp == kSplitEpi / 32) tc::tmem_alloc(&tmem_slot, 512);
   if (tid == 0) {
+    gave_up = 0;
     for (int i = 0; i < kSplit; i++) tc::mbar_init_nofence(&full0[i], 1);
     for (int i = 0; i < G; i++) {
       tc::mbar_init_nofence(&full1[i], 1);
@@ -228,7 +241,7 @@ mf_update_split(MfView v, const int4 *__restrict__ tasks, int ntasks, int nupd, 
       const int ks0 = (min(K, 64) + 15) / 16, ks1 = (K - 64 + 15) / 16;
       armed = 0;
       if (t != (int)blockIdx.x) {  // the epilogue has read the accumulators
-        ok = tc::mbar_wait(&empty, pe, kTcWaitPolls);
+        ok = split_wait(&empty, pe, kTcWaitPolls, &gave_up);
         pe ^= 1;
         if (!ok) break;
         tc::fence_after_sync();
@@ -275,15 +288,15 @@ mf_update_split(MfView v, const int4 *__restrict__ tasks, int ntasks, int nupd, 
       if (!ok) break;
       tc::mma_commit(tc::smem_u32(&done));
       t += gridDim.x;
-      if (t >= ntasks) break;
-      task = tasks[t];
-      ok = tc::mbar_wait(&done, p0, kTcWaitPolls);
-      if (!ok) break;
+      if (t < ntasks) task = tasks[t];
+      ok = tc::mbar_wait(&done, p0, kTcWaitPolls);  // (of the last tile too: its MMAs use the tensor memory)
+      if (!ok || t >= ntasks) break;
       p0 ^= 1;
       if (two) p1 ^= 1;
       load_first(task);
     }
     if (!ok) {  // no copy and no MMA of this CTA may be left in flight
+      gave_up = 1;
       atomicOr(status, ERR_WAIT);
       for (int i = 0; i < kSplit; i++) tc::mbar_wait(&full0[i], p0, kTcWaitPolls);
       for (int i = 0; i < armed; i++) tc::mbar_wait(&full1[i], p1, kTcWaitPolls);
@@ -313,7 +326,13 @@ mf_update_split(MfView v, const int4 *__restrict__ tasks, int ntasks, int nupd, 
       for (int c = 0; c < 4; c++) cur[c] = c < cold ? C[c * cs] : 0.0;
       const int ea = expo[task.z * kSplitRows + lrow], eb = expo[task.w * kSplitRows + cw + (lane & 15)];
       // a warp that gave up once waits no more, but meets the others below
-      if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&done, ph, kTcWaitPolls));
+      if (ok) {
+        ok = __all_sync(0xffffffffu, split_wait(&done, ph, epi_polls, &gave_up));
+        if (!ok && lane == 0) {
+          gave_up = 1;
+          atomicOr(status, ERR_WAIT);
+        }
+      }
       ph ^= 1;
       tc::fence_after_sync();
 #pragma unroll 1

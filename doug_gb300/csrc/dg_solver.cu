@@ -1421,6 +1421,7 @@ bool robust_restriction_gpu(const Controls &c, const Csr &A, const std::vector<i
     int stv = 0;
     CK(cudaMemcpyAsync(&stv, status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (stv & ERR_WAIT) throw CudaError{cudaSuccess, "robust coarse space: a wait of the factorisation timed out"};
     if (stv & ERR_NOT_SPD) throw CudaError{cudaSuccess, "robust coarse space: a support matrix is not positive definite"};
     const std::vector<double> ones((size_t)n, 1.0);
     CK(cudaMemcpy(r.p, ones.data(), (size_t)n * sizeof(double), cudaMemcpyHostToDevice));
@@ -1864,6 +1865,16 @@ int precondition(dg_handle *h, const SolvePlan &pl, cudaStream_t st, bool profil
   return nl + 1;
 }
 
+// What the device's status says after the factorisations (before the first
+// preconditioner step, so that a timeout is theirs); factors that are not
+// whole are not kept.
+dg_status factor_status(dg_handle *h, int status) {
+  h->factored = !(status & (ERR_NOT_SPD | ERR_WAIT));
+  if (status & ERR_WAIT) return fail(h, DG_CUDA_ERROR, "a wait of the factorisation timed out");
+  if (status & ERR_NOT_SPD) return fail(h, DG_SINGULAR, "a subdomain or coarse matrix is not positive definite");
+  return DG_OK;
+}
+
 // Stacked solves: the independent systems of a batch (c = h->bt) or K
 // right-hand sides of one matrix (c = h->mr, nrhs = K).  Every system /
 // right-hand side runs its own pcg_weigs (pcg.F90:289-462) with its own
@@ -1917,11 +1928,7 @@ dg_status do_solve_stacked(dg_handle *h, BatchCtx &bc, const Vecs &V, int nrhs, 
     int stv = 0;
     CK(cudaMemcpyAsync(&stv, h->status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (stv & ERR_NOT_SPD) {
-      h->factored = false;
-      return fail(h, DG_SINGULAR, "a subdomain or coarse matrix is not positive definite");
-    }
-    h->factored = true;
+    if (const dg_status fs = factor_status(h, stv)) return fs;
     const bool prof = c.profile != 0;
     double t_sub = 0, t_co = 0, t_sp = 0;
     auto lap = [&](int a, int b) -> double {
@@ -2123,11 +2130,7 @@ dg_status do_solve(dg_handle *h, const double *d_b, double *d_x, dg_stats *st, c
     launches += 2;
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
-    if (*h->host_status & ERR_NOT_SPD) {
-      h->factored = false;
-      return fail(h, DG_SINGULAR, "a subdomain or coarse matrix is not positive definite");
-    }
-    h->factored = true;
+    if (const dg_status fs = factor_status(h, *h->host_status)) return fs;
     double init = h->host_out[0];
     if (init == 0.0) {
       init = 1.0;

@@ -54,6 +54,11 @@ struct DBuf {
     n = count;
     CK(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)));
   }
+  void release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    n = 0;
+  }
   void upload(const std::vector<T> &v) {
     alloc(v.size());
     if (!v.empty()) CK(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
@@ -82,6 +87,7 @@ struct MfTune {
   int tiny_threads = 64;
   int tensor_update = 1;                 // FP32 super-panel updates: 1 tcgen05 (TMEM), 0 mma.sync
   int super_panel = kSuperPanel;         // columns of L per trailing update of a large front (multiple of 32)
+  int split_blocks = 4096;               // FP64: 64-row blocks (128 KB) of digit slices at once, 0 none
   long long queue_wait_cycles = kQueueWaitCycles;  // solve_schedule 1: limit of one dependency wait
   int queue_skip_publish = -1;           // solve_schedule 1: forward entry whose done flag is withheld (tests)
   long long update_wait_polls = kTcWaitPolls;  // mf_update_split: polls of its epilogue's wait (tests)
@@ -146,8 +152,11 @@ struct MfDevice {
   size_t q_smem = 0;
   DBuf<int2> asm_tasks, upd_tasks, panel_tasks, esc_tasks, etile_tasks;
   DBuf<int4> split_tasks, tile_tasks;
-  DBuf<unsigned char> slices;  // of one super-panel step's fronts
+  // digit slices of the fronts of one group of a super-panel step (reserve_split)
+  DBuf<unsigned char> slices;
   DBuf<int> expo;
+  int64_t split_blocks = 0;
+  bool split_on = false;
   DBuf<T> arena, E, xl, yl, u;
   int64_t e_len = 0;
   // per level: small-front range, assembly-task range, steps
@@ -160,9 +169,13 @@ struct MfDevice {
     int kw, cend_base;
     bool big;                     // trailing update in 128 x 128 tiles (FP32)
     bool thin = false;            // mf_panel_thin
-    int split_off = 0, split_cnt = 0;  // FP64 on the tensor cores: mf_split tasks (0: mf_update),
-    int tile_off = 0, tile_cnt = 0, tile_upd = 0;  // mf_update_split tasks, trailing tiles first
+    int grp_off = 0, grp_cnt = 0;  // FP64 on the tensor cores: groups of fronts (0: mf_update alone)
   };
+  // fronts whose slices are held at once: mf_split tasks, mf_update_split tasks (trailing tiles first)
+  struct SplitGroup {
+    int split_off, split_cnt, tile_off, tile_cnt, tile_upd;
+  };
+  std::vector<SplitGroup> groups;
   struct Level {
     int pan_off, pan_cnt, asm_off, asm_cnt, pan_maxm;
     int tiny_off, tiny_cnt;        // panel fronts of at most tune.tiny_rows rows: narrow CTAs
@@ -244,7 +257,8 @@ struct MfDevice {
     std::vector<int> pn, df;
     std::vector<int2> at, ut, pf, es, et;
     std::vector<int4> sp, tt;
-    int64_t split_blocks = 0;
+    split_blocks = 0;
+    groups.clear();
     levels.assign((size_t)nlevels, Level());
     for (int l = 0; l < nlevels; l++) {
       Level &L = levels[(size_t)l];
@@ -344,15 +358,11 @@ struct MfDevice {
           st.etile_cnt = (int)et.size() - st.etile_off;
           L.steps.push_back(st);
         }
-        const bool bigt = sizeof(T) == 4;  // FP32: 128 x 128 tiles; FP64 keeps mf_update (FP64-pipe bound)
+        const bool bigt = sizeof(T) == 4;  // FP32: 128 x 128 tiles; FP64: mf_update's, and the groups of mf_update_split
         const int tile = bigt ? kBT : kTile;
         Step st{S0, (int)df.size(), 0, (int)pf.size(), 0, (int)es.size(), 0,
                 (int)ut.size(), 0, (int)et.size(), 0, SP, 0, bigt};
-        if (sizeof(T) == 8 && split_step(B, tune, large, S0)) {
-          plan_split(B, large, S0, SP, st, sp, tt, split_blocks);
-          L.steps.push_back(st);
-          continue;
-        }
+        if (sizeof(T) == 8 && split_step(B, tune, large, S0)) plan_split(B, large, S0, SP, tune.split_blocks, st, sp, tt);
         for (int f : large) {
           int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
           if (S0 >= k) continue;
@@ -384,11 +394,10 @@ struct MfDevice {
     asm_tasks.upload(at);
     upd_tasks.upload(ut);
     etile_tasks.upload(et);
+    split_on = false;
     if (split_blocks) {
       split_tasks.upload(sp);
       tile_tasks.upload(tt);
-      slices.alloc((size_t)split_blocks * kSplitBlock);
-      expo.alloc((size_t)split_blocks * kSplitRows);
       CK(cudaFuncSetAttribute(mf_update_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSplitSmem));
     }
     // what the solves read about a front, and its child table
@@ -452,7 +461,7 @@ struct MfDevice {
   // 26 us, 182 of 128 columns 52 us against 37 us, 58 of 128 columns 66 us
   // against 56 us, 49386 of 128 columns 3.24 ms against 1.00 ms.
   bool split_step(const MfBatch &B, const MfTune &tune, const std::vector<int> &large, int S0) const {
-    if (tune.tensor_update != 1 || tune.super_panel > kSplitK) return false;
+    if (tune.tensor_update != 1 || tune.super_panel > kSplitK || tune.split_blocks == 0) return false;
     double fma_tiles = 0, tiles = 0, kmax = 0;
     for (int f : large) {
       const int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
@@ -471,20 +480,40 @@ struct MfDevice {
 
   // Tasks of the tensor-core update of the super-panel at column S0: 64-row
   // blocks of L below it (an even number: a tile takes two) and of E's
-  // columns before its end, then the tiles.
-  static void plan_split(const MfBatch &B, const std::vector<int> &large, int S0, int SP, Step &st,
-                         std::vector<int4> &sp, std::vector<int4> &tt, int64_t &blocks) {
+  // columns before its end, then the tiles.  The fronts go in groups of at most
+  // `most` blocks (or one front): all of them at once took 0.7 GB at 96^3
+  // beside 1.3 GB of E; 4096 blocks are 512 MB and 30,000 tiles, so that a
+  // group's last wave and launches do not show.
+  void plan_split(const MfBatch &B, const std::vector<int> &large, int S0, int SP, int64_t most, Step &st,
+                  std::vector<int4> &sp, std::vector<int4> &tt) {
     std::vector<int4> te;
-    st.split_off = (int)sp.size();
-    st.tile_off = (int)tt.size();
+    SplitGroup g{};
     int blk = 0;
+    auto open = [&] { g = SplitGroup{(int)sp.size(), 0, (int)tt.size(), 0, 0}; };
+    auto close = [&] {
+      g.tile_upd = (int)tt.size() - g.tile_off;
+      tt.insert(tt.end(), te.begin(), te.end());
+      te.clear();
+      g.split_cnt = (int)sp.size() - g.split_off;
+      g.tile_cnt = (int)tt.size() - g.tile_off;
+      if (g.tile_cnt) groups.push_back(g);
+      split_blocks = std::max<int64_t>(split_blocks, blk);
+      blk = 0;
+    };
+    st.grp_off = (int)groups.size();
+    open();
     for (int f : large) {
       const int m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
       if (S0 >= k) continue;
       const int c1 = S0 + std::min(SP, k - S0);
       if (c1 >= m) continue;
       const int nt = (m - c1 + 127) / 128, nl = (m - c1 + kSplitRows - 1) / kSplitRows;
-      const int ne = (c1 + kSplitRows - 1) / kSplitRows, be = blk + 2 * nt;
+      const int ne = (c1 + kSplitRows - 1) / kSplitRows;
+      if (blk > 0 && blk + 2 * nt + ne > most) {
+        close();
+        open();
+      }
+      const int be = blk + 2 * nt;
       for (int h = 0; h < 4 * nt; h++) sp.push_back(make_int4(f, c1 + h * kSplitCtaRows, 2 * blk + h, 0));
       for (int h = 0; h < 2 * ne; h++) sp.push_back(make_int4(f, ~(h * kSplitCtaRows), 2 * be + h, 0));
       for (int tj = 0; tj < nl; tj++)
@@ -493,11 +522,29 @@ struct MfDevice {
         for (int tc = 0; tc < ne; tc++) te.push_back(make_int4(f, (ti << 16) | tc, blk + 2 * ti, be + tc));
       blk = be + ne;
     }
-    st.tile_upd = (int)tt.size() - st.tile_off;
-    tt.insert(tt.end(), te.begin(), te.end());
-    st.split_cnt = (int)sp.size() - st.split_off;
-    st.tile_cnt = (int)tt.size() - st.tile_off;
-    blocks = std::max<int64_t>(blocks, blk);
+    close();
+    st.grp_cnt = (int)groups.size() - st.grp_off;
+  }
+
+  // The memory of the digit slices, taken after everything else of a handle:
+  // where there is none left, mf_update does the work.
+  void reserve_split() {
+    split_on = false;
+    if (split_blocks == 0) return;
+    try {
+      slices.alloc((size_t)split_blocks * kSplitBlock);
+      expo.alloc((size_t)split_blocks * kSplitRows);
+      split_on = true;
+    } catch (const CudaError &e) {
+      if (e.e != cudaErrorMemoryAllocation) throw;
+      cudaGetLastError();
+      release_split();
+    }
+  }
+  void release_split() {
+    slices.release();
+    expo.release();
+    split_on = false;
   }
 
   // Solve work lists for K right-hand sides: warp kernels for the
@@ -713,14 +760,17 @@ struct MfDevice {
               launches++;
             }
           }
-        } else if (st.split_cnt) {
+        } else if (split_on && st.grp_cnt) {
           if constexpr (sizeof(T) == 8) {  // planned for FP64 batches only
-            mf_split<<<st.split_cnt, 256, 0, s>>>(view, split_tasks.p + st.split_off, st.j0, st.kw, arena.p, E.p,
-                                                  slices.p, expo.p);
-            mf_update_split<<<std::min(st.tile_cnt, nsm), kSplitThreads, kSplitSmem, s>>>(
-                view, tile_tasks.p + st.tile_off, st.tile_cnt, st.tile_upd, st.j0, st.kw, slices.p, expo.p, arena.p,
-                E.p, status, update_wait_polls);
-            launches += 2;
+            for (int q = st.grp_off; q < st.grp_off + st.grp_cnt; q++) {
+              const SplitGroup &g = groups[(size_t)q];
+              mf_split<<<g.split_cnt, 256, 0, s>>>(view, split_tasks.p + g.split_off, st.j0, st.kw, arena.p, E.p,
+                                                   slices.p, expo.p);
+              mf_update_split<<<std::min(g.tile_cnt, nsm), kSplitThreads, kSplitSmem, s>>>(
+                  view, tile_tasks.p + g.tile_off, g.tile_cnt, g.tile_upd, st.j0, st.kw, slices.p, expo.p, arena.p,
+                  E.p, status, update_wait_polls);
+              launches += 2;
+            }
           }
         } else if (st.upd_cnt + st.etile_cnt) {
           mf_update<T><<<st.upd_cnt + st.etile_cnt, kMfThreads, 0, s>>>(
@@ -1387,6 +1437,7 @@ bool robust_restriction_gpu(const Controls &c, const Csr &A, const std::vector<i
     tune.small_min_fronts = c.thin_level_fronts;
     tune.tensor_update = c.tensor_update;
     tune.super_panel = c.super_panel;
+    tune.split_blocks = c.split_blocks;
     tune.queue_wait_cycles = c.queue_wait_cycles;
     tune.queue_skip_publish = c.queue_skip_publish;
     tune.update_wait_polls = c.update_wait_polls < 0 ? kTcWaitPolls : c.update_wait_polls;
@@ -1397,6 +1448,7 @@ bool robust_restriction_gpu(const Controls &c, const Csr &A, const std::vector<i
     CK(cudaHostGetDevicePointer(&d_host_status, host_status, 0));
     MfDevice<double> dev;
     dev.upload(Bs, tune);
+    dev.reserve_split();
     DBuf<double> Av, x, r, z, p, qv, part_rz, part_pq, part_rr, sc;
     DBuf<int64_t> Ap;
     DBuf<int> Ac, status, pull_ptr, pull_idx;
@@ -1526,6 +1578,7 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
   tune.small_min_fronts = c.thin_level_fronts;
   tune.tensor_update = c.tensor_update;
   tune.super_panel = c.super_panel;
+  tune.split_blocks = c.split_blocks;
   tune.queue_wait_cycles = c.queue_wait_cycles;
   tune.queue_skip_publish = c.queue_skip_publish;
   tune.update_wait_polls = c.update_wait_polls < 0 ? kTcWaitPolls : c.update_wait_polls;
@@ -1731,6 +1784,8 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
       h->cpos.alloc(1);
       h->Pc.alloc(1);
     }
+    if (h->sub64) h->sub64->reserve_split();
+    if (h->co64) h->co64->reserve_split();
     CK(cudaDeviceSynchronize());
   } catch (const CudaError &e) {
     return cuda_fail(h, e);
@@ -2070,17 +2125,28 @@ dg_status do_solve_multi(dg_handle *h, int K, const double *d_b, double *d_x, dg
   ctl_finish(c);
   if (c.fine_method == 2) return fail(h, DG_BAD_INPUT, "several right-hand sides: fine_method 2 is not supported");
   if (h->elem_mv) return fail(h, DG_BAD_INPUT, "several right-hand sides: use the assembled products (elemental_matvec 0)");
+  auto stacks = [&] {
+    const int64_t nt = (int64_t)K * h->n;
+    std::vector<int64_t> row((size_t)K + 1);
+    for (int k = 0; k <= K; k++) row[(size_t)k] = (int64_t)k * h->n;
+    h->mr.build(row, h->n, h->nsm);
+    for (auto *v : {&h->mb, &h->mx, &h->mrr, &h->mp, &h->mq, &h->mz, &h->mzold}) v->alloc((size_t)nt);
+    if (h->sub32) h->sub32->ensure_multi(K);
+    if (h->sub64) h->sub64->ensure_multi(K);
+    if (h->co64) h->co64->ensure_multi(K);
+    h->mr_k = K;
+  };
   try {
     if (h->mr_k != K) {
-      const int64_t nt = (int64_t)K * h->n;
-      std::vector<int64_t> row((size_t)K + 1);
-      for (int k = 0; k <= K; k++) row[(size_t)k] = (int64_t)k * h->n;
-      h->mr.build(row, h->n, h->nsm);
-      for (auto *v : {&h->mb, &h->mx, &h->mrr, &h->mp, &h->mq, &h->mz, &h->mzold}) v->alloc((size_t)nt);
-      if (h->sub32) h->sub32->ensure_multi(K);
-      if (h->sub64) h->sub64->ensure_multi(K);
-      if (h->co64) h->co64->ensure_multi(K);
-      h->mr_k = K;
+      try {
+        stacks();
+      } catch (const CudaError &e) {  // the digit slices' memory is not needed to go on
+        if (e.e != cudaErrorMemoryAllocation) throw;
+        cudaGetLastError();
+        if (h->sub64) h->sub64->release_split();
+        if (h->co64) h->co64->release_split();
+        stacks();
+      }
     }
   } catch (const CudaError &e) {
     return cuda_fail(h, e);
@@ -2338,6 +2404,13 @@ dg_status dg_set_option(dg_handle *h, const char *name, const char *value) {
     if (!parse_i10(w2, v) || v < 32 || v % 32 != 0 || v > 1024)
       return fail(h, DG_BAD_INPUT, "super_panel must be a multiple of 32 in [32, 1024]");
     h->ctl.super_panel = v;
+    h->ready = false;
+    return DG_OK;
+  }
+  if (w1 == "split_blocks") {
+    int v;
+    if (!parse_i10(w2, v) || v < 0) return fail(h, DG_BAD_INPUT, "split_blocks must not be negative");
+    h->ctl.split_blocks = v;
     h->ready = false;
     return DG_OK;
   }

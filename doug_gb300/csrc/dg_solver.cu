@@ -876,7 +876,9 @@ struct MfDevice {
   int64_t ulen = 0;
   void ensure_multi(int K) {
     if (mk == K) return;
+    mk = 0;  // an allocation that fails below leaves nothing planned
     if (queue && q_k < K) {
+      q_k = 0;
       q_done.alloc((size_t)(qf_n + qb_n) * K);
       q_k = K;
     }
@@ -1223,6 +1225,7 @@ dg_status fail(dg_handle *h, dg_status s, const std::string &msg) {
 }
 
 dg_status cuda_fail(dg_handle *h, const CudaError &e) {
+  cudaGetLastError();  // a failed allocation is not the next call's error
   h->err = std::string("CUDA error in ") + e.what + ": " + cudaGetErrorString(e.e);
   return DG_CUDA_ERROR;
 }
@@ -2126,6 +2129,7 @@ dg_status do_solve_multi(dg_handle *h, int K, const double *d_b, double *d_x, dg
   if (c.fine_method == 2) return fail(h, DG_BAD_INPUT, "several right-hand sides: fine_method 2 is not supported");
   if (h->elem_mv) return fail(h, DG_BAD_INPUT, "several right-hand sides: use the assembled products (elemental_matvec 0)");
   auto stacks = [&] {
+    h->mr_k = 0;  // an allocation that fails below leaves no stacks
     const int64_t nt = (int64_t)K * h->n;
     std::vector<int64_t> row((size_t)K + 1);
     for (int k = 0; k <= K; k++) row[(size_t)k] = (int64_t)k * h->n;

@@ -2130,6 +2130,10 @@ dg_status do_solve_multi(dg_handle *h, int K, const double *d_b, double *d_x, dg
   if (h->elem_mv) return fail(h, DG_BAD_INPUT, "several right-hand sides: use the assembled products (elemental_matvec 0)");
   auto stacks = [&] {
     h->mr_k = 0;  // an allocation that fails below leaves no stacks
+    if (h->iter_exec && c.solve_schedule == 1) {  // it holds the queue's done flags, which move
+      cudaGraphExecDestroy(h->iter_exec);
+      h->iter_exec = nullptr;
+    }
     const int64_t nt = (int64_t)K * h->n;
     std::vector<int64_t> row((size_t)K + 1);
     for (int k = 0; k <= K; k++) row[(size_t)k] = (int64_t)k * h->n;

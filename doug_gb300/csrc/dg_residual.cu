@@ -21,38 +21,81 @@ namespace resid {
 constexpr int kThreads = 256;
 constexpr int kMaxRowsPerBlock = 1024;            // rows per partial sum
 
-// A block's rows with L lanes per row; returns this thread's part of sum r_i^2.
-// Four entries of a lane's share are loaded before they are summed.
+// The products of entries e, e + W, .. below e1 with x, in that order; four
+// entries are loaded before they are summed.
+template <int W>
+__device__ __forceinline__ double row_share(long long e, long long e1, const int *__restrict__ col,
+                                            const double *__restrict__ val, const double *__restrict__ x) {
+  double s = 0.0;
+  for (; e + 3 * W < e1; e += 4 * W) {
+    const int c0 = col[e], c1 = col[e + W], c2 = col[e + 2 * W], c3 = col[e + 3 * W];
+    const double a0 = val[e], a1 = val[e + W], a2 = val[e + 2 * W], a3 = val[e + 3 * W];
+    const double x0 = x[c0], x1 = x[c1], x2 = x[c2], x3 = x[c3];
+    s = __fma_rn(a0, x0, s);
+    s = __fma_rn(a1, x1, s);
+    s = __fma_rn(a2, x2, s);
+    s = __fma_rn(a3, x3, s);
+  }
+  for (; e < e1; e += W) s = __fma_rn(val[e], x[col[e]], s);
+  return s;
+}
+
+// A block's rows [r0, r0 + nr) with L lanes per row; returns this thread's part
+// of sum r_i^2.  Rows of more than kLongRow L entries are left to whole warps,
+// after the others: their L lanes alone would hold up the block.  200,000 rows
+// of 7 entries with one of 1,200: 143 us without this, 30 us with it; a million
+// rows of 7 with 5 % of 100: 183 us, 121 us.  At the limit a lane makes 16
+// rounds of loads; rows of 36 among rows of 2 are faster by lanes (168 us; 327
+// with a limit of 32).
+constexpr int kLongRow = 64;
 template <int L>
-__device__ __forceinline__ double block_rows(int r0, int r1, const long long *__restrict__ rp,
+__device__ __forceinline__ double block_rows(int r0, int nr, const long long *__restrict__ rp,
                                              const int *__restrict__ col, const double *__restrict__ val,
                                              const double *__restrict__ x, const double *__restrict__ b,
-                                             double *__restrict__ r) {
+                                             double *__restrict__ r, int *any_long) {
   const int sub = threadIdx.x % L;
   double acc = 0.0;
-  for (int i0 = r0; i0 < r1; i0 += kThreads / L) {
-    const int i = i0 + threadIdx.x / L;
+  for (int q0 = 0; q0 < nr; q0 += kThreads / L) {
+    const int q = q0 + threadIdx.x / L, i = r0 + q;
     double s = 0.0;
-    if (i < r1) {
-      long long e = rp[i] + sub;
-      const long long e1 = rp[i + 1];
-      for (; e + 3 * L < e1; e += 4 * L) {
-        const int c0 = col[e], c1 = col[e + L], c2 = col[e + 2 * L], c3 = col[e + 3 * L];
-        const double a0 = val[e], a1 = val[e + L], a2 = val[e + 2 * L], a3 = val[e + 3 * L];
-        const double x0 = x[c0], x1 = x[c1], x2 = x[c2], x3 = x[c3];
-        s = __fma_rn(a0, x0, s);
-        s = __fma_rn(a1, x1, s);
-        s = __fma_rn(a2, x2, s);
-        s = __fma_rn(a3, x3, s);
-      }
-      for (; e < e1; e += L) s = __fma_rn(val[e], x[col[e]], s);
+    bool on = q < nr;
+    if (on) {
+      const long long e0 = rp[i], e1 = rp[i + 1];
+      on = L == 32 || e1 - e0 <= kLongRow * L;
+      if (on) s = row_share<L>(e0 + sub, e1, col, val, x);
+      else *any_long = 1;
     }
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, L);
-    if (i < r1 && sub == 0) {
+    if (on && sub == 0) {
       const double ri = __dsub_rn(b[i], s);
       r[i] = ri;
       acc += ri * ri;
+    }
+  }
+  return acc;
+}
+
+// the rows of more than `limit` entries, a warp each in the rows' order
+__device__ __noinline__ double long_rows(int r0, int nr, int limit, const long long *__restrict__ rp,
+                                         const int *__restrict__ col, const double *__restrict__ val,
+                                         const double *__restrict__ x, const double *__restrict__ b,
+                                         double *__restrict__ r) {
+  const int lane = threadIdx.x & 31;
+  double acc = 0.0;
+  for (int q0 = 0; q0 < nr; q0 += kThreads) {
+    const int q = q0 + threadIdx.x;
+    unsigned todo = __ballot_sync(0xffffffffu, q < nr && rp[r0 + q + 1] - rp[r0 + q] > limit);
+    for (; todo; todo &= todo - 1) {
+      const int i = r0 + q - lane + __ffs(todo) - 1;
+      double s = row_share<32>(rp[i] + lane, rp[i + 1], col, val, x);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) {
+        const double ri = __dsub_rn(b[i], s);
+        r[i] = ri;
+        acc += ri * ri;
+      }
     }
   }
   return acc;
@@ -67,14 +110,19 @@ residual_partials(int n, int rpb, const long long *__restrict__ rp, const int *_
                   const double *__restrict__ val, const double *__restrict__ x,
                   const double *__restrict__ b, double *__restrict__ r, double *__restrict__ partial) {
   __shared__ double sh[kThreads / 32];
+  __shared__ int any_long;
   const int r0 = blockIdx.x * rpb;
-  const int r1 = n - r0 > rpb ? r0 + rpb : n;
-  const long long per = (rp[r1] - rp[r0]) / (r1 - r0);
+  const int nr = min(n - r0, rpb);
+  const long long per = (rp[r0 + nr] - rp[r0]) / nr;
+  if (threadIdx.x == 0) any_long = 0;
+  __syncthreads();
   double acc;
-  if (per <= 12) acc = block_rows<1>(r0, r1, rp, col, val, x, b, r);
-  else if (per <= 48) acc = block_rows<4>(r0, r1, rp, col, val, x, b, r);
-  else if (per <= 192) acc = block_rows<16>(r0, r1, rp, col, val, x, b, r);
-  else acc = block_rows<32>(r0, r1, rp, col, val, x, b, r);
+  if (per <= 12) acc = block_rows<1>(r0, nr, rp, col, val, x, b, r, &any_long);
+  else if (per <= 48) acc = block_rows<4>(r0, nr, rp, col, val, x, b, r, &any_long);
+  else if (per <= 192) acc = block_rows<16>(r0, nr, rp, col, val, x, b, r, &any_long);
+  else acc = block_rows<32>(r0, nr, rp, col, val, x, b, r, &any_long);
+  __syncthreads();
+  if (any_long) acc += long_rows(r0, nr, kLongRow * (per <= 12 ? 1 : per <= 48 ? 4 : 16), rp, col, val, x, b, r);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;

@@ -158,13 +158,18 @@ int blocks_for(int n) {
 }
 
 // Scratch of dg_residual_csr: a memory pool of its own per device that keeps
-// up to kPoolKeep bytes between calls.  The default pool gives everything
-// back to the driver at each synchronisation, so that every call after one
-// paid for a new mapping: 231 us a call on a 128^3 matrix (440 us after a
-// synchronisation) against 63 us with the kept pool and the kernel above.  Allocation and release stay stream
-// ordered: any number of threads and streams may call at once.  The pool
-// belongs to the context (its id is kept beside it) and goes with it.
-constexpr unsigned long long kPoolKeep = 1ull << 20;  // 131,072 partial sums
+// its memory between calls, up to kPoolKeep bytes.  The default pool gives
+// everything back to the driver at each synchronisation, so that every call
+// after one pays for a new mapping.  The threshold is compared with what the
+// pool has reserved, which comes in chunks of 2 MB and more, not
+// with what is in use: one of 1 MB kept nothing.  A
+// call and a synchronisation: 24^3 185 -> 22 us, 128^3 224 -> 72 us (without a
+// pool 203 and 393); back to back 10 and 61 us; a first call on new data, 128^3:
+// 340 -> 110 us.
+// Allocation and release stay stream ordered: any number of threads and
+// streams may call at once.  The pool belongs to the context (its id is kept
+// beside it) and goes with it.
+constexpr unsigned long long kPoolKeep = 64ull << 20;
 constexpr int kMaxDevices = 128;
 cudaError_t current_context_id(unsigned long long *id);
 
@@ -189,17 +194,16 @@ cudaMemPool_t scratch_pool(int dev) {  // null: use the device's default pool
   props.location.id = dev;
   cudaMemPool_t pool = nullptr;
   unsigned long long keep = kPoolKeep;
-  // another stream of this thread may be under capture: creating a pool must
-  // not count as an unsafe call of it
+  // another stream of this thread may be under capture: creating the pool
+  // counts as little as possible against it (the allocation itself is an
+  // unsafe call beside a capture in the stricter modes, from any pool)
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaThreadExchangeStreamCaptureMode(&mode);
   const cudaError_t made = cudaMemPoolCreate(&pool, &props);
+  if (made == cudaSuccess) cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   cudaThreadExchangeStreamCaptureMode(&mode);
-  if (made != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
+  cudaGetLastError();
+  if (made != cudaSuccess) return nullptr;
   p.pool = pool;
   p.ctx = ctx;
   return pool;

@@ -43,7 +43,10 @@ struct ChildEdge {
 // place in two children's update vectors (16 bits each, kNoChild: none), m
 // words per pair of children, so that the right-hand side is gathered in one
 // round of loads; cu0, cu1: the first two children's vectors, ch_edge[ch ..]:
-// all nch children.  nch < 0: -nch children without a table.
+// all nch children.  nch < 0: -nch children (more than kMostPairs, or one of
+// 65,535 update rows and more) by lists instead, row i of the front the entries
+// clist[cptr[tab + i] .. cptr[tab + i + 1]) of the update vectors, children in
+// order: a row of a front with hundreds of children hears from a few of them.
 struct __align__(16) SolveFront {
   int m, k;
   int64_t e_off;
@@ -56,6 +59,7 @@ struct __align__(16) SolveFront {
 };
 static_assert(sizeof(SolveFront) == 80, "five 16-byte loads");
 constexpr unsigned kNoChild = 0xffffu;
+constexpr int kMostPairs = 16;  // children in a table: what joined levels make of two each
 
 struct MfView {  // device pointers of one multifrontal batch
   const int64_t *f_off;
@@ -71,6 +75,7 @@ struct MfView {  // device pointers of one multifrontal batch
   const ChildEdge *ch_edge;    // per child-list entry: see ChildEdge
   const SolveFront *sfront;    // per front: see SolveFront
   const unsigned *ctab;        // child tables
+  const int64_t *cptr, *clist; // child lists
 };
 
 __host__ __device__ __forceinline__ int round4(int x) { return (x + 3) & ~3; }
@@ -1399,9 +1404,25 @@ __device__ __forceinline__ T add_more_children(T x, const MfView &v, int64_t w, 
   return x;
 }
 
+// and the listed updates of a row (row: tab + its place in the front)
+template <typename T>
+__device__ __forceinline__ T add_listed(T x, const MfView &v, int64_t row, const T *__restrict__ u) {
+  int64_t e = v.cptr[row];
+  const int64_t e1 = v.cptr[row + 1];
+  for (; e + 3 < e1; e += 4) {
+    T a[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) a[q] = __ldcg(u + v.clist[e + q]);
+#pragma unroll
+    for (int q = 0; q < 4; q++) x += a[q];
+  }
+  for (; e < e1; e++) x += __ldcg(u + v.clist[e]);
+  return x;
+}
+
 // small fronts, forward: the first batch of E is loaded before the
 // right-hand side is assembled.  cta: this CTA's index within its bucket.
-// MORE: fronts of more than two children (or without a child table) as well
+// MORE: fronts of more than two children as well
 template <typename T, int G, bool MORE>
 __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__restrict__ fronts, int nf,
                                                const T *__restrict__ E, const T *__restrict__ xl,
@@ -1438,9 +1459,12 @@ __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__res
       if (sl + (h + q) * G < m) w[sl + (h + q) * G] = x[q];
     asm volatile("" ::: "memory");
   }
+  if constexpr (MORE)
+    if (nch < 0)
+      for (int i = sl; i < m; i += G) w[i] = add_listed(w[i], v, f.tab + i, uvec);
   __syncwarp(gm);
   if constexpr (MORE)  // children beyond the second, in order
-    for (int ci = nch < 0 ? 0 : 2; ci < abs(nch); ci++) {
+    for (int ci = 2; ci < nch; ci++) {
       const ChildEdge ed = v.ch_edge[f.ch + ci];
       const int *rel = v.relmap + ed.relmap;
       for (int a = sl; a < ed.rc; a += G) w[rel[a]] += __ldcg(uvec + ed.uoff + a);
@@ -1620,7 +1644,7 @@ template <typename T, int LPR> __host__ __device__ constexpr int fwd_rows() { re
 
 // the task body; b: shared memory for the right-hand side (at most the
 // front's rows), red: the warp sums of one chunk
-// (MORE: with fronts of more than two children or without a child table)
+// (MORE: with fronts of more than two children)
 template <typename T, int NT, int UN, int LPR, bool MORE>
 __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const SolveFront &f, const T *__restrict__ E,
                                              const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec,
@@ -1717,17 +1741,11 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
     const T s = add_children(i < kn ? __ldcg(xl + xo + i) : T(0), nc > 0 ? v.ctab[w] : ~0u, uvec, cu0, cu1);
     b[i] = kPairs ? add_more_children(s, v, w, m, nc, f.ch, 1, uvec) : s;
   }
+  if constexpr (MORE)
+    if (nc < 0)
+#pragma unroll 1
+      for (int i = tid; i < nrow; i += NT) b[i] = add_listed(b[i], v, tab + (i < kn ? i : rlo + i - kn), uvec);
   __syncthreads();
-  // children beyond the second (in pairs: those without a table), in order
-  for (int ci = nc < 0 ? 0 : kPairs ? nc : 2; MORE && ci < abs(nc); ci++) {
-    const ChildEdge ed = v.ch_edge[f.ch + ci];
-    const int *rel = v.relmap + ed.relmap;
-    for (int a = tid; a < ed.rc; a += NT) {
-      const int row = rel[a], i = row < kn ? row : row >= rlo && row < rhi ? kn + row - rlo : -1;
-      if (i >= 0) b[i] += __ldcg(uvec + ed.uoff + a);
-    }
-    __syncthreads();
-  }
   for (int ch = ch0; ch < ch0 + nch; ch++) {
     const int r0 = ch * RC;
     const int K = chunk_cols(r0);

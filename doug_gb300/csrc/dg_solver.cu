@@ -121,6 +121,7 @@ struct MfDevice {
   DBuf<ChildEdge> ch_edge;
   DBuf<SolveFront> sfront;
   DBuf<unsigned> ctab;
+  DBuf<int64_t> cptr, clist;
   DBuf<int> f_m, f_k, f_p0, f_child_ptr, f_children, rows, relmap, lvl_fronts, gidx;
   DBuf<int> pan_fronts, diag_fronts;
   int tiny_threads = 64;
@@ -191,7 +192,7 @@ struct MfDevice {
     int fwd_off, fwd_cnt, bwd_off, bwd_cnt;
     size_t fwd_smem, bwd_smem;
     int fwd_v, bwd_v;             // kFwdVariants, kBwdVariants
-    bool more;                    // fronts of more than two children, or without a child table
+    bool more;                    // fronts of more than two children
   };
   // the solves' work lists: of one right-hand side, of several (planned for
   // their number)
@@ -248,7 +249,7 @@ struct MfDevice {
     mk = 0;
     view = MfView{f_off.p, f_m.p, f_k.p, f_rows.p, f_xoff.p, f_p0.p, f_uoff.p, f_woff.p,
                   f_child_ptr.p, f_children.p, f_relmap.p, f_asm.p, rows.p, relmap.p,
-                  asm_tgt.p, asm_sp.p, asm_src.p, e_off.p, ch_edge.p, nullptr, nullptr};
+                  asm_tgt.p, asm_sp.p, asm_src.p, e_off.p, ch_edge.p, nullptr, nullptr, nullptr, nullptr};
     int dev = 0, optin = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -403,17 +404,39 @@ struct MfDevice {
     // what the solves read about a front, and its child table
     sf.assign((size_t)nfronts, SolveFront());
     std::vector<unsigned> ct;
+    std::vector<int64_t> cp, cl;
     for (int f = 0; f < nfronts; f++) {
       const int m = B.f_m[(size_t)f], cb = B.f_child_ptr[(size_t)f], nch = B.f_child_ptr[(size_t)f + 1] - cb;
       SolveFront &S = sf[(size_t)f];
       S = SolveFront{m, B.f_k[(size_t)f], eo[(size_t)f], B.f_xoff[(size_t)f] + B.f_p0[(size_t)f], B.f_xoff[(size_t)f],
                      B.f_rows[(size_t)f], B.f_uoff[(size_t)f], (int64_t)ct.size(), 0, 0, nch, cb};
       if (nch == 0) continue;
-      for (int h = 0; h < nch; h++) {  // an update vector beyond 16-bit places: its front's children go row by row
+      bool listed = nch > kMostPairs;
+      for (int h = 0; h < nch; h++) {  // (a table's places have 16 bits)
         const int c = B.f_children[(size_t)(cb + h)];
-        if (B.f_m[(size_t)c] - B.f_k[(size_t)c] >= (int)kNoChild) S.nch = -nch;
+        listed |= B.f_m[(size_t)c] - B.f_k[(size_t)c] >= (int)kNoChild;
       }
-      if (S.nch < 0) continue;
+      if (listed) {
+        S.nch = -nch;
+        S.tab = (int64_t)cp.size();
+        std::vector<int64_t> cnt((size_t)m + 1, 0);
+        for (int pass = 0; pass < 2; pass++) {
+          for (int h = 0; h < nch; h++) {
+            const int c = B.f_children[(size_t)(cb + h)], rc = B.f_m[(size_t)c] - B.f_k[(size_t)c];
+            for (int q = 0; q < rc; q++) {
+              const size_t row = (size_t)B.relmap[(size_t)(B.f_relmap[(size_t)c] + q)];
+              if (pass == 0) cnt[row + 1]++;
+              else cl[(size_t)cnt[row]++] = B.f_uoff[(size_t)c] + q;
+            }
+          }
+          if (pass == 1) break;
+          cnt[0] = (int64_t)cl.size();
+          for (int i = 0; i < m; i++) cnt[(size_t)i + 1] += cnt[(size_t)i];
+          cp.insert(cp.end(), cnt.begin(), cnt.end());
+          cl.resize((size_t)cnt[(size_t)m]);
+        }
+        continue;
+      }
       ct.resize(ct.size() + (size_t)m * (size_t)((nch + 1) / 2), ~0u);
       for (int h = 0; h < nch; h++) {
         const int c = B.f_children[(size_t)(cb + h)], rc = B.f_m[(size_t)c] - B.f_k[(size_t)c];
@@ -426,8 +449,12 @@ struct MfDevice {
     }
     sfront.upload(sf);
     ctab.upload(ct);
+    cptr.upload(cp);
+    clist.upload(cl);
     view.sfront = sfront.p;
     view.ctab = ctab.p;
+    view.cptr = cptr.p;
+    view.clist = clist.p;
     queue = tune.schedule == 1;
     batch = &B;
     tune_ = tune;

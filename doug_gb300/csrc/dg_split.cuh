@@ -109,6 +109,13 @@ mf_split(MfView v, const int4 *__restrict__ tasks, int jl, int kw, const double 
   }
 }
 
+// top 2^-drop units of the last subnormal place, rounded to nearest (a call:
+// the shifts in line cost the epilogue of every entry)
+__device__ __noinline__ double split_subnormal(unsigned long long top, int drop) {
+  if (drop > 64) return 0.0;
+  return __longlong_as_double((long long)(((top >> 1) >> (drop - 1)) + ((top >> (drop - 1)) & 1)));
+}
+
 // sum_s d[s] 2^(8 (7 - s)) * 2^(ex - 2112), rounded to nearest (subnormal
 // numbers too); the d[s] are integers of at most 2^24, ex the sum of the two
 // rows' biased exponents
@@ -128,12 +135,11 @@ __device__ __forceinline__ double split_value(const int (&d)[kSplit], int ex) {
   const int n = a ? __clzll((long long)a) : 64 + __clzll((long long)b);
   const unsigned long long top = n == 0 ? a : n < 64 ? a << n | b >> (64 - n) : b << (n & 63);
   const int fe = 1023 + 80 - n + ex - 2112;  // biased exponent of the leading bit
-  const int drop = max(11, 12 - fe);  // bits of top below the result's last one
-  const unsigned long long bits = ((unsigned long long)max(fe - 1, 0) << 52) + ((top >> 1) >> ((drop - 1) & 63)) +
-                                  ((top >> ((drop - 1) & 63)) & 1);
+  const unsigned long long bits = ((unsigned long long)(fe - 1) << 52) + (top >> 11) + ((top >> 10) & 1);
   double r = __longlong_as_double((long long)bits);
   if (fe > 2046) r = __longlong_as_double(0x7ff0000000000000ll);
-  if (drop > 64 || (a | b) == 0) r = 0.0;  // below half of the smallest subnormal number, or zero
+  if ((a | b) == 0) r = 0.0;
+  else if (fe < 1) r = split_subnormal(top, 12 - fe);
   if (ex >= kSplitNan) r = __longlong_as_double(0x7ff8000000000000ll);
   return neg ? -r : r;
 }

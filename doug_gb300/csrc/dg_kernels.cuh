@@ -191,10 +191,8 @@ template <typename T> struct UpdTile { static constexpr int N = sizeof(T) == 8 ?
 // third-order iteration (r (1 + e + e^2), e = 1 - x r; Traub, Iterative Methods
 // for the Solution of Equations, 1964): three dependent FP64 operations,
 // error e^3 < 2^-63 before the last rounding.
-__device__ __forceinline__ float pivot_inverse(float d) { return 1.0f / d; }
-__device__ __forceinline__ double pivot_inverse(double d) {
+__device__ __forceinline__ double normal_inverse(double d) {  // d and 1 / d normal numbers
   const int hi = __double2hiint(d), lo = __double2loint(d), ex = hi >> 20;
-  if (ex < 1 || ex > 2044) return 1.0 / d;  // subnormal, or the result may be, or not finite
   const double x = __hiloint2double((hi & 0xfffff) | 0x3ff00000, lo);  // in [1, 2)
   const float f = __int_as_float(0x3f800000 | (hi & 0xfffff) << 3 | (int)((unsigned)lo >> 29));
   const unsigned g = (unsigned)__float_as_int(__frcp_rn(f));  // in (1/2, 1]
@@ -203,41 +201,47 @@ __device__ __forceinline__ double pivot_inverse(double d) {
   const double y = __fma_rn(r, __fma_rn(e, e, e), r);
   return __hiloint2double(__double2hiint(y) + ((1023 - ex) << 20), __double2loint(y));
 }
+__device__ __forceinline__ float normal_inverse(float d) { return 1.0f / d; }
 
-// The reciprocal of a pivot as the factorisations keep it: 1 / d, or, where
-// that is no normal number (d below the smallest one, or within a factor of
-// four of the largest), the negative of 1 / (d 2^s) or 1 / (d 2^-s), which the
-// sign and the magnitude tell apart.  The sign is the same for a whole CTA and
-// read in an integer operation.
-__device__ __forceinline__ bool scaled_inverse(float iv) { return __float_as_int(iv) < 0; }
-__device__ __forceinline__ bool scaled_inverse(double iv) { return __double2hiint(iv) < 0; }
-template <typename T> struct PivotScale;
-template <> struct PivotScale<float> {
-  __device__ static bool plain(float d) { return d >= 0x1p-126f && d <= 0x1p126f; }
-  static constexpr float up = 0x1p64f, down = 0x1p-64f, root_up = 0x1p32f, root_down = 0x1p-32f;
-};
-template <> struct PivotScale<double> {
-  __device__ static bool plain(double d) { return (unsigned)((__double2hiint(d) >> 20) - 1) < 2044u; }
-  static constexpr double up = 0x1p512, down = 0x1p-512, root_up = 0x1p256, root_down = 0x1p-256;
-};
+// The largest and smallest powers of two between which d and 1 / d are normal
+// numbers, tested by the exponent (d > 0).
+__device__ __forceinline__ bool plain_pivot(float d) { return (unsigned)((__float_as_int(d) >> 23) - 1) < 252u; }
+__device__ __forceinline__ bool plain_pivot(double d) { return (unsigned)((__double2hiint(d) >> 20) - 1) < 2044u; }
 template <typename T>
-__device__ __forceinline__ T keep_inverse(T d) {
-  using S = PivotScale<T>;
-  if (S::plain(d)) return pivot_inverse(d);
-  return T(-1) / (d * (d < T(1) ? S::up : S::down));
-}
-template <typename T>  // c / d
-__device__ __forceinline__ T times_inverse(T c, T iv) {
-  using S = PivotScale<T>;
-  if (scaled_inverse(iv)) return c * (iv < T(-1) ? S::up : S::down) * -iv;
-  return c * iv;
-}
-template <typename T>  // d^-1/2
-__device__ __forceinline__ T sqrt_inverse(T iv) {
-  using S = PivotScale<T>;
-  if (scaled_inverse(iv)) return tsqrt<T>(-iv) * (iv < T(-1) ? S::root_up : S::root_down);
-  return tsqrt<T>(iv);
-}
+__device__ __forceinline__ T pivot_inverse(T d) { return plain_pivot(d) ? normal_inverse(d) : T(1) / d; }
+
+// A pivot as the factorisations keep it: 1 / d, or a negative number where d
+// or 1 / d is no normal number.  FP64: -d, and those divide; the sign is the
+// same for a whole CTA and read in an integer operation (as in the reciprocal,
+// FP64 operations beside the one product would show: 129^2 1.035 ms with a
+// division that is never reached, 1.115 with products by a power of two).
+// FP32: -1 / (d 2^64) or -1 / (d 2^-64), which the magnitude tells apart, and a
+// product by that power or by one (48 grids 2.42 ms, with the division 2.49).
+template <typename T> struct KeptPivot;
+template <> struct KeptPivot<double> {
+  double v;
+  __device__ explicit KeptPivot(double kept) : v(kept) {}
+  __device__ static double keep(double d) { return plain_pivot(d) ? normal_inverse(d) : -d; }
+  __device__ bool whole() const { return __double2hiint(v) < 0; }
+  __device__ double divide(double c) const {  // c / d
+    if (whole()) return c / -v;
+    return c * v;
+  }
+  __device__ double inverse_root() const {  // d^-1/2
+    if (whole()) return 1.0 / sqrt(-v);
+    return sqrt(v);
+  }
+};
+template <> struct KeptPivot<float> {
+  float v, up;
+  __device__ explicit KeptPivot(float kept) : v(fabsf(kept)), up(kept >= 0.f ? 1.f : kept < -1.f ? 0x1p64f : 0x1p-64f) {}
+  __device__ static float keep(float d) {
+    if (plain_pivot(d)) return normal_inverse(d);
+    return -1.f / (d * (d < 1.f ? 0x1p64f : 0x1p-64f));
+  }
+  __device__ float divide(float c) const { return c * up * v; }
+  __device__ float inverse_root() const { return sqrtf(v) * (up == 1.f ? 1.f : up > 1.f ? 0x1p32f : 0x1p-32f); }
+};
 
 // Extend-add of column b of a child's update block into column pb of the
 // parent (Dst = the parent's column base; row r of the column at
@@ -389,7 +393,7 @@ mf_factor_panel(MfView v, const int *__restrict__ fronts, const double *__restri
       atomicOr(status, ERR_NOT_SPD);
       d = T(1);
     }
-    inv[j] = keep_inverse(d);
+    inv[j] = KeptPivot<T>::keep(d);
   };
   for (int c = tid; c < k; c += nt) {
     const T x = P[(size_t)c * ldk];
@@ -402,9 +406,9 @@ mf_factor_panel(MfView v, const int *__restrict__ fronts, const double *__restri
   for (int j = 0; j < k - 1; j++) {
     const T *cur = mul + (j & 1) * ldk;
     T *nxt = mul + ((j + 1) & 1) * ldk;
-    const T iv = inv[j];
+    const KeptPivot<T> piv(inv[j]);
     for (int i = j + 1 + ty; i < k; i += ny) {
-      const T li = times_inverse(cur[i], iv);
+      const T li = piv.divide(cur[i]);
       if (tx == 0) L[(size_t)i * ldk + j] = li;
       V *row = reinterpret_cast<V *>(P + (size_t)i * ldk);
       // (entries right of the diagonal take garbage; nothing reads them)
@@ -437,7 +441,7 @@ mf_factor_panel(MfView v, const int *__restrict__ fronts, const double *__restri
     }
     __syncthreads();
   }
-  for (int j = tid; j < k; j += nt) rs[j] = sqrt_inverse(inv[j]);
+  for (int j = tid; j < k; j += nt) rs[j] = KeptPivot<T>(inv[j]).inverse_root();
   __syncthreads();
   // 3. E11: rows of Lt^-1 scaled (its unit diagonal and the zeros above it)
   for (int q = tid; q < k * nv; q += nt) {
@@ -661,7 +665,7 @@ __device__ __forceinline__ void chol_cta(T (*D)[kNB + 1], int jb, int *status) {
       d = T(1);
     }
     D[j][j] = d;
-    inv[j] = keep_inverse(d);
+    inv[j] = KeptPivot<T>::keep(d);
   };
   if (tid == 0) pivot(D[0][0], 0);
   diag_sync<NAMED>();
@@ -669,7 +673,7 @@ __device__ __forceinline__ void chol_cta(T (*D)[kNB + 1], int jb, int *status) {
   const int i = tid / TX, tx = tid % TX;
   for (int j = 0; j < jb - 1; j++) {
     if (i > j && i < jb) {
-      const T li = times_inverse(D[i][j], inv[j]);
+      const T li = KeptPivot<T>(inv[j]).divide(D[i][j]);
       for (int c = j + 1 + tx; c <= i; c += TX) {
         const T x = D[i][c] - li * D[c][j];
         if (c == i && i == j + 1) pivot(x, i);
@@ -680,7 +684,7 @@ __device__ __forceinline__ void chol_cta(T (*D)[kNB + 1], int jb, int *status) {
   }
   for (int q = tid; q < jb * jb; q += kMfThreads) {
     const int c = q / jb, k = q % jb;
-    if (k > c) D[k][c] *= sqrt_inverse(inv[c]);
+    if (k > c) D[k][c] *= KeptPivot<T>(inv[c]).inverse_root();
   }
   diag_sync<NAMED>();
   if (tid < jb) D[tid][tid] = tsqrt<T>(D[tid][tid]);

@@ -1426,8 +1426,8 @@ __device__ __forceinline__ T add_listed(T x, const MfView &v, int64_t row, const
 
 // small fronts, forward: the first batch of E is loaded before the
 // right-hand side is assembled.  cta: this CTA's index within its bucket.
-// MORE: fronts of more than two children as well
-template <typename T, int G, bool MORE>
+// MORE: 1 fronts of more than two children as well, 2 and of listed children
+template <typename T, int G, int MORE>
 __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__restrict__ fronts, int nf,
                                                const T *__restrict__ E, const T *__restrict__ xl,
                                                T *__restrict__ yl, T *__restrict__ uvec, int cta,
@@ -1463,11 +1463,11 @@ __device__ __forceinline__ void fwd_small_body(const MfView &v, const int *__res
       if (sl + (h + q) * G < m) w[sl + (h + q) * G] = x[q];
     asm volatile("" ::: "memory");
   }
-  if constexpr (MORE)
+  if constexpr (MORE == 2)
     if (nch < 0)
       for (int i = sl; i < m; i += G) w[i] = add_listed(w[i], v, f.tab + i, uvec);
   __syncwarp(gm);
-  if constexpr (MORE)  // children beyond the second, in order
+  if constexpr (MORE > 0)  // children beyond the second, in order
     for (int ci = 2; ci < nch; ci++) {
       const ChildEdge ed = v.ch_edge[f.ch + ci];
       const int *rel = v.relmap + ed.relmap;
@@ -1594,7 +1594,7 @@ struct SmallBuckets {
 // Several right-hand sides (nrhs > 1): CTA x serves right-hand side x % nrhs
 // of the work unit x / nrhs, so the CTAs that read the same E are adjacent;
 // the vectors of right-hand side k start at k * xs (xl, yl) and k * us (u).
-template <typename T, bool MORE>
+template <typename T, int MORE>
 __global__ void __launch_bounds__(256, SmallMinBlocks<T>::N)
 mf_fwd_small(MfView v, const int *__restrict__ fronts, SmallBuckets sb, const T *__restrict__ E,
              const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec, int nrhs = 1, int64_t xs = 0,
@@ -1648,8 +1648,8 @@ template <typename T, int LPR> __host__ __device__ constexpr int fwd_rows() { re
 
 // the task body; b: shared memory for the right-hand side (at most the
 // front's rows), red: the warp sums of one chunk
-// (MORE: with fronts of more than two children)
-template <typename T, int NT, int UN, int LPR, bool MORE>
+// (MORE: as for the small ones)
+template <typename T, int NT, int UN, int LPR, int MORE>
 __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const SolveFront &f, const T *__restrict__ E,
                                              const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec,
                                              T *b, T *red) {
@@ -1691,7 +1691,7 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
   // A front of more than two children (MORE): the first four together, RB rows
   // of a thread at once.  (The branch is the CTA's: predicated FP64 additions
   // cost the pipe as much as others.)
-  constexpr bool kPairs = MORE;
+  constexpr bool kPairs = MORE > 0;
   constexpr int RB = NP == 2 ? 1 : 2;
   unsigned t2[NP];
   int64_t cu2 = 0, cu3 = 0;
@@ -1745,7 +1745,7 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
     const T s = add_children(i < kn ? __ldcg(xl + xo + i) : T(0), nc > 0 ? v.ctab[w] : ~0u, uvec, cu0, cu1);
     b[i] = kPairs ? add_more_children(s, v, w, m, nc, f.ch, 1, uvec) : s;
   }
-  if constexpr (MORE)
+  if constexpr (MORE == 2)
     if (nc < 0)
 #pragma unroll 1
       for (int i = tid; i < nrow; i += NT) b[i] = add_listed(b[i], v, tab + (i < kn ? i : rlo + i - kn), uvec);
@@ -1789,7 +1789,7 @@ __device__ __forceinline__ void fwd_big_body(const MfView &v, int2 tk, const Sol
   }
 }
 
-template <typename T, int V, bool MORE>
+template <typename T, int V, int MORE>
 __global__ void __launch_bounds__(kFwdVariants[V].nt, kFwdVariants[V].ctas)
 mf_fwd_big(MfView v, const int2 *__restrict__ tasks, const SolveFront *__restrict__ tmeta, const T *__restrict__ E,
            const T *__restrict__ xl, T *__restrict__ yl, T *__restrict__ uvec, int nrhs = 1, int64_t xs = 0,
@@ -2000,12 +2000,12 @@ mf_fwd_queue(MfView v, QueueView q, const int *__restrict__ small_fronts, const 
       const SmallBuckets sb = lvl_sb[tk.y];
       const int *fr = small_fronts + lvl_small_off[tk.y];
       const int b = tk.z;
-      if (b < sb.nb0) fwd_small_body<T, 8, true>(v, fr, sb.cnt0, E, xk, yk, uk, b, sm);
+      if (b < sb.nb0) fwd_small_body<T, 8, 2>(v, fr, sb.cnt0, E, xk, yk, uk, b, sm);
       else if (b < sb.nb0 + sb.nb1)
-        fwd_small_body<T, 16, true>(v, fr + sb.cnt0, sb.cnt1, E, xk, yk, uk, b - sb.nb0, sm);
-      else fwd_small_body<T, 32, true>(v, fr + sb.cnt0 + sb.cnt1, sb.cnt2, E, xk, yk, uk, b - sb.nb0 - sb.nb1, sm);
+        fwd_small_body<T, 16, 2>(v, fr + sb.cnt0, sb.cnt1, E, xk, yk, uk, b - sb.nb0, sm);
+      else fwd_small_body<T, 32, 2>(v, fr + sb.cnt0 + sb.cnt1, sb.cnt2, E, xk, yk, uk, b - sb.nb0 - sb.nb1, sm);
     } else {
-      fwd_big_body<T, 256, 8, 32, true>(v, fwd_tasks[tk.z], fwd_tmeta[tk.z], E, xk, yk, uk, sm, red);
+      fwd_big_body<T, 256, 8, 32, 2>(v, fwd_tasks[tk.z], fwd_tmeta[tk.z], E, xk, yk, uk, sm, red);
     }
     __syncthreads();
     if (threadIdx.x == 0) queue_publish<T>(q, done, g);

@@ -192,7 +192,7 @@ struct MfDevice {
     int fwd_off, fwd_cnt, bwd_off, bwd_cnt;
     size_t fwd_smem, bwd_smem;
     int fwd_v, bwd_v;             // kFwdVariants, kBwdVariants
-    bool more;                    // fronts of more than two children
+    int more;                     // 1 fronts of more than two children, 2 of listed ones
   };
   // the solves' work lists: of one right-hand side, of several (planned for
   // their number)
@@ -589,7 +589,7 @@ struct MfDevice {
       L.fwd_off = (int)fw.size();
       L.bwd_off = (int)bw.size();
       L.fwd_smem = L.bwd_smem = 0;
-      L.more = false;
+      L.more = 0;
       // a level with few small fronts solves them with the CTA-per-task
       // kernels too: a group of lanes per front leaves the GPU nearly idle
       // while it walks the columns of a large-k front
@@ -600,7 +600,7 @@ struct MfDevice {
       std::vector<int> large;
       for (int q = B.lvl_ptr[(size_t)l]; q < B.lvl_ptr[(size_t)l + 1]; q++) {
         const int f = B.lvl_fronts[(size_t)q], m = B.f_m[(size_t)f], k = B.f_k[(size_t)f];
-        L.more |= sf[(size_t)f].nch < 0 || sf[(size_t)f].nch > 2;
+        L.more = std::max(L.more, sf[(size_t)f].nch < 0 ? 2 : sf[(size_t)f].nch > 2 ? 1 : 0);
         if (m <= kSolveSmall && !thin) { sm[m <= 32 ? 0 : m <= 64 ? 1 : 2].push_back({k, f}); continue; }
         large.push_back(f);
         L.fwd_smem = std::max(L.fwd_smem, (size_t)round4(m) * sizeof(T));
@@ -704,8 +704,9 @@ struct MfDevice {
         throw CudaError{cudaErrorInvalidValue, "front too large for the shared-memory solve"};
       CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes));
     };
-    set(mf_fwd_big<T, V, false>);
-    set(mf_fwd_big<T, V, true>);
+    set(mf_fwd_big<T, V, 0>);
+    set(mf_fwd_big<T, V, 1>);
+    set(mf_fwd_big<T, V, 2>);
     set(mf_bwd_big<T, V>);
   }
 
@@ -957,16 +958,17 @@ struct MfDevice {
     for (int l = 0; l < nlevels; l++) {
       const SolveLevel &L = w.levels[(size_t)l];
       if (L.small_cta) {
-        launch_level(pdl, L.more ? mf_fwd_small<T, true> : mf_fwd_small<T, false>, L.small_cta * nrhs, 256, 0, s, view,
+        launch_level(pdl, L.more == 2 ? mf_fwd_small<T, 2> : L.more ? mf_fwd_small<T, 1> : mf_fwd_small<T, 0>, L.small_cta * nrhs, 256, 0, s, view,
                      (const int *)(w.small.p + L.small_off), L.sb, (const T *)E.p, (const T *)xl_, yl_, u_, nrhs,
                      xs, us);
         launches++;
       }
       if (L.fwd_cnt) {
-        if (L.fwd_v == 0) fwd(L, L.more ? mf_fwd_big<T, 0, true> : mf_fwd_big<T, 0, false>);
-        else if (L.fwd_v == 1) fwd(L, L.more ? mf_fwd_big<T, 1, true> : mf_fwd_big<T, 1, false>);
-        else if (L.fwd_v == 2) fwd(L, L.more ? mf_fwd_big<T, 2, true> : mf_fwd_big<T, 2, false>);
-        else fwd(L, L.more ? mf_fwd_big<T, 3, true> : mf_fwd_big<T, 3, false>);
+        auto pick = [&](auto *k0, auto *k1, auto *k2) { fwd(L, L.more == 2 ? k2 : L.more ? k1 : k0); };
+        if (L.fwd_v == 0) pick(mf_fwd_big<T, 0, 0>, mf_fwd_big<T, 0, 1>, mf_fwd_big<T, 0, 2>);
+        else if (L.fwd_v == 1) pick(mf_fwd_big<T, 1, 0>, mf_fwd_big<T, 1, 1>, mf_fwd_big<T, 1, 2>);
+        else if (L.fwd_v == 2) pick(mf_fwd_big<T, 2, 0>, mf_fwd_big<T, 2, 1>, mf_fwd_big<T, 2, 2>);
+        else pick(mf_fwd_big<T, 3, 0>, mf_fwd_big<T, 3, 1>, mf_fwd_big<T, 3, 2>);
         launches++;
       }
     }

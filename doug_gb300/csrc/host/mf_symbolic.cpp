@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <stdexcept>
 #include <thread>
@@ -563,6 +564,10 @@ void finalize(MfBatch &B) {
       B.lvl_max_m[(size_t)l] = std::max(B.lvl_max_m[(size_t)l], B.f_m[(size_t)B.lvl_fronts[(size_t)q]]);
 }
 
+// Nodes of a subdomain are looked up by an array over their range up to this
+// many times the subdomain's size (128 bytes a node on each host thread).
+constexpr int64_t kLookupRange = 32;
+
 template <class F>
 void parallel_for(int n, F fn) {
   unsigned nt = std::max(1u, std::min({std::thread::hardware_concurrency(), 32u, (unsigned)std::max(n, 1)}));
@@ -597,20 +602,37 @@ void mf_build_subdomains(const Csr &A, const std::vector<int64_t> &sd_ptr,
     int64_t b0 = sd_ptr[(size_t)s], m = sd_ptr[(size_t)s + 1] - b0;
     std::vector<int> &gid = work[(size_t)s].gid;
     gid.resize((size_t)m);
-    // local position of each global node (sorted lookup keeps memory per subdomain small)
-    std::vector<std::pair<int, int>> lut((size_t)m);
+    // local position of each global node: an array over the subdomain's range
+    // of nodes, or, where that is many times the subdomain, a sorted list (both
+    // keep memory per subdomain small)
+    int lo = INT_MAX, hi = -1;
     for (int64_t t = 0; t < m; t++) {
-      gid[(size_t)t] = sd_nodes[(size_t)(b0 + t)] - 1;
-      lut[(size_t)t] = {gid[(size_t)t], (int)t};
+      const int g = gid[(size_t)t] = sd_nodes[(size_t)(b0 + t)] - 1;
+      lo = std::min(lo, g);
+      hi = std::max(hi, g);
     }
-    std::sort(lut.begin(), lut.end());
+    const bool dense = (int64_t)hi - lo < kLookupRange * m;
+    std::vector<int> pos;
+    std::vector<std::pair<int, int>> lut;
+    if (dense) {
+      pos.assign((size_t)(hi - lo + 1), -1);
+      for (int64_t t = m - 1; t >= 0; t--) pos[(size_t)(gid[(size_t)t] - lo)] = (int)t;
+    } else {
+      lut.resize((size_t)m);
+      for (int64_t t = 0; t < m; t++) lut[(size_t)t] = {gid[(size_t)t], (int)t};
+      std::sort(lut.begin(), lut.end());
+    }
     auto loc = [&](int g) -> int {
+      if (dense) return g < lo || g > hi ? -1 : pos[(size_t)(g - lo)];
       auto it = std::lower_bound(lut.begin(), lut.end(), std::make_pair(g, -1));
       if (it != lut.end() && it->first == g) return it->second;
       return -1;
     };
+    int64_t most = 0;  // entries of the subdomain's rows
+    for (int64_t t = 0; t < m; t++) most += A.ptr[(size_t)gid[(size_t)t] + 1] - A.ptr[(size_t)gid[(size_t)t]];
     std::vector<int> &lr = work[(size_t)s].lr, &lc = work[(size_t)s].lc;
     std::vector<int64_t> &src = work[(size_t)s].src;
+    lr.reserve((size_t)most); lc.reserve((size_t)most); src.reserve((size_t)most);
     for (int64_t t = 0; t < m; t++) {
       int g = gid[(size_t)t];
       for (int64_t e = A.ptr[(size_t)g]; e < A.ptr[(size_t)g + 1]; e++) {
@@ -630,6 +652,9 @@ void mf_build_subdomains(const Csr &A, const std::vector<int64_t> &sd_ptr,
     Work &w = work[(size_t)s];
     join(w, group);
     place_entries(w);
+    std::vector<int>().swap(w.lr);
+    std::vector<int>().swap(w.lc);
+    std::vector<int64_t>().swap(w.src);
     append(w.L, w.gid, pieces[(size_t)s]);
     w = Work();
   });

@@ -1031,7 +1031,12 @@ static bool aggregate(ScaledMatrix &S, int neighood, int minasize, int maxasize,
           if (!(stat[(size_t)node] <= neighood + 1 && q + 1 <= maxasize) && stat[(size_t)node] == next_layer)
             nouter_all++;
         }
-      const bool replay = valid_start + 2 * (int64_t)nouter_all >= (int64_t)n;
+      // (nodes can be listed more than once, so that the lists outgrow the
+      // reference's array of n: it is extended for the head, and a tail longer
+      // than the array has no place in it)
+      const bool replay = valid_start + 2 * (int64_t)nouter_all >= (int64_t)n && nouter_all <= n;
+      if (replay)
+        ngs.resize(std::max(ngs.size(), (size_t)(std::max<int64_t>(n, valid_start) + nouter_all + 2)));
       int ngood = 0;
       if (replay) {  // the reference's compacted head list in the array
         for (size_t q = cur; q < L.size(); q++)

@@ -88,6 +88,7 @@ struct MfTune {
   int tensor_update = 1;                 // FP32 super-panel updates: 1 tcgen05 (TMEM), 0 mma.sync
   int super_panel = kSuperPanel;         // columns of L per trailing update of a large front (multiple of 32)
   int split_blocks = 4096;               // FP64: 64-row blocks (128 KB) of digit slices at once, 0 none
+  bool split_always = false;             // mf_update_split for every super-panel update, whatever it costs (tests)
   long long queue_wait_cycles = kQueueWaitCycles;  // solve_schedule 1: limit of one dependency wait
   int queue_skip_publish = -1;           // solve_schedule 1: forward entry whose done flag is withheld (tests)
   long long update_wait_polls = kTcWaitPolls;  // mf_update_split: polls of its epilogue's wait (tests)
@@ -500,6 +501,7 @@ struct MfDevice {
       tiles += n128 * (n128 + 1) + n128 * ((c1 + 63) / 64);
       kmax = std::max(kmax, (double)K);
     }
+    if (tune.split_always) return tiles > 0;
     const double cuda = 0.27 * std::max(kmax, fma_tiles / nsm);
     const double tensor = 8.0 + std::ceil(tiles / nsm) * (9.5 + 0.07 * kmax);
     return cuda > tensor;
@@ -1470,6 +1472,7 @@ bool robust_restriction_gpu(const Controls &c, const Csr &A, const std::vector<i
     tune.tensor_update = c.tensor_update;
     tune.super_panel = c.super_panel;
     tune.split_blocks = c.split_blocks;
+    tune.split_always = c.split_always != 0;
     tune.queue_wait_cycles = c.queue_wait_cycles;
     tune.queue_skip_publish = c.queue_skip_publish;
     tune.update_wait_polls = c.update_wait_polls < 0 ? kTcWaitPolls : c.update_wait_polls;
@@ -1611,6 +1614,7 @@ dg_status do_setup(dg_handle *h, bool reuse_host = false) {
   tune.tensor_update = c.tensor_update;
   tune.super_panel = c.super_panel;
   tune.split_blocks = c.split_blocks;
+  tune.split_always = c.split_always != 0;
   tune.queue_wait_cycles = c.queue_wait_cycles;
   tune.queue_skip_publish = c.queue_skip_publish;
   tune.update_wait_polls = c.update_wait_polls < 0 ? kTcWaitPolls : c.update_wait_polls;
@@ -2444,10 +2448,10 @@ dg_status dg_set_option(dg_handle *h, const char *name, const char *value) {
     h->ready = false;
     return DG_OK;
   }
-  if (w1 == "split_blocks") {
+  if (w1 == "split_blocks" || w1 == "split_always") {
     int v;
-    if (!parse_i10(w2, v) || v < 0) return fail(h, DG_BAD_INPUT, "split_blocks must not be negative");
-    h->ctl.split_blocks = v;
+    if (!parse_i10(w2, v) || v < 0 || (w1 == "split_always" && v > 1)) return fail(h, DG_BAD_INPUT, "bad " + w1);
+    (w1 == "split_blocks" ? h->ctl.split_blocks : h->ctl.split_always) = v;
     h->ready = false;
     return DG_OK;
   }

@@ -51,6 +51,7 @@ struct Controls {
   int tensor_update = 1;            // FP32 super-panel trailing updates: 1 tcgen05 (TMEM accumulator), 0 mma.sync
   int super_panel = 128;           // columns of L per trailing update of a large front (multiple of 32)
   int split_blocks = 4096;         // FP64 tensor-core updates: 64-row blocks of digit slices (128 KB) held at once, 0 none
+  int split_always = 0;            // 1: those updates on the tensor cores whatever they cost (tests)
   long long queue_wait_cycles = 1000000000LL;  // solve_schedule 1: limit of one dependency wait (cycles)
   long long update_wait_polls = -1; // FP64 tensor-core update: polls of the epilogue's wait, -1 the usual limit (failure tests)
   int queue_skip_publish = -1;      // solve_schedule 1: forward entry whose done flag is withheld (failure tests)

@@ -287,9 +287,9 @@ constexpr int kJoin = 4;  // levels joined at most
 
 // Of the level that the levels h .. h + g make, per h and g: entries of the
 // elimination matrices, multiply-adds of the factorisation, the most pivots
-// of a front, fronts.
+// and rows of a front, fronts.
 struct LevelSums {
-  double entries[kJoin] = {}, work[kJoin] = {}, pivots[kJoin] = {};
+  double entries[kJoin] = {}, work[kJoin] = {}, pivots[kJoin] = {}, rows[kJoin] = {};
   int fronts[kJoin] = {};
 };
 
@@ -313,6 +313,7 @@ void add_sums(const Local &L, std::vector<LevelSums> &out) {
         S.entries[g] += k * (k + r) - 0.5 * k * k;
         S.work[g] += k * (k * k / 3 + r * k + r * r) / 2;
         S.pivots[g] = std::max(S.pivots[g], k);
+        S.rows[g] = std::max(S.rows[g], k + r);
         S.fronts[g]++;
       }
     }
@@ -341,7 +342,7 @@ std::vector<int> plan_joins(const std::vector<LevelSums> &S, const MfOptions &op
     best[(size_t)h] = 1e300;
     for (int g = 0; g < kJoin && h + g < N; g++) {
       const LevelSums &s = S[(size_t)h];
-      if (g > 0 && s.fronts[g] >= opt.thin) continue;
+      if (g > 0 && (s.fronts[g] >= opt.thin || s.rows[g] > opt.max_rows)) continue;
       const double t = 2 * kNominal * (4.5 + s.entries[g] / rate) + 35 + 37 * std::ceil(s.pivots[g] / 32) +
                        s.work[g] / 2e6 + best[(size_t)(h + g + 1)];
       if (t < best[(size_t)h]) { best[(size_t)h] = t; len[(size_t)h] = g + 1; }

@@ -60,6 +60,8 @@ struct MfOptions {
   int leaf = 64;                  // nested-dissection leaf size
   int value_bytes = 8;            // of the factors (4: FP32)
   int thin = 1500;                // levels with fewer fronts may be joined with others
+  int max_rows = 16384;           // joined fronts have at most this many rows: a solve holds
+                                  // a front's vector in shared memory (227 KB)
 };
 
 // Subdomain batch: the principal submatrices A(inds, inds) of the fine matrix

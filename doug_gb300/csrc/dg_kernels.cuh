@@ -1351,7 +1351,6 @@ template <> struct Vec16<double> {
 };
 
 constexpr int kSolveSmall = 128;   // fronts of at most this many rows: one warp each
-constexpr int kEThreads = 256;
 
 // Small fronts are solved by groups of G lanes (G = 8, 16 or 32; 32 / G
 // fronts per warp): a front of at most 4G rows, lane l of its group holding
@@ -1851,7 +1850,6 @@ __device__ __forceinline__ void bwd_big_body(const MfView &v, int2 tk, const Sol
     rw[q] = (i >= k && i < m) ? rows[i] : 0;
   }
   pdl_wait();
-  const int nrow = ld - c0;
 #pragma unroll
   for (int q = 0; q < kRowsAhead; q++) {
     const int i = c0 + tid + q * NT;

@@ -71,7 +71,9 @@ static double wall() {
 
 // one multifrontal batch on the device, factor precision T
 // fronts of at most panel_rows rows whose panel and E fit in kPanelSmem
-// bytes are factored by one CTA each; the others by the multi-CTA pipeline
+// bytes are factored by one CTA each where a level has at least eight of them
+// per SM (and fronts of at most tiny_rows rows everywhere); the others by the
+// multi-CTA pipeline
 constexpr size_t kPanelSmem = 96 * 1024;
 constexpr int kSuperPanel = 128;      // default columns of L per trailing update of a large front
 // tunable batch parameters (control words panel_rows, fwd_task_kb, lean_task_kb)
@@ -85,7 +87,7 @@ struct MfTune {
   int factor_overlap = 1;                // 1: a level's one-CTA fronts beside its large-front steps
   int tiny_rows = 64;                    // panel fronts of at most this many rows: tiny_threads per CTA
   int tiny_threads = 64;
-  int tensor_update = 1;                 // FP32 super-panel updates: 1 tcgen05 (TMEM), 0 mma.sync
+  int tensor_update = 1;                 // super-panel updates: 1 tcgen05 (TMEM), 0 FP32 mma.sync, FP64 CUDA cores
   int super_panel = kSuperPanel;         // columns of L per trailing update of a large front (multiple of 32)
   int split_blocks = 4096;               // FP64: 64-row blocks (128 KB) of digit slices at once, 0 none
   bool split_always = false;             // mf_update_split for every super-panel update, whatever it costs (tests)
@@ -96,7 +98,7 @@ struct MfTune {
 
 // Launch k with programmatic stream serialisation when pdl is set: its CTAs
 // may start while the previous kernel of the stream drains (the kernels call
-// pdl_enter before reading anything); otherwise an ordinary launch.
+// pdl_wait before they read what it writes); otherwise an ordinary launch.
 template <typename... P, typename... A>
 void launch_level(bool pdl, void (*k)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
   if (!pdl) {
@@ -126,7 +128,7 @@ struct MfDevice {
   DBuf<int> f_m, f_k, f_p0, f_child_ptr, f_children, rows, relmap, lvl_fronts, gidx;
   DBuf<int> pan_fronts, diag_fronts;
   int tiny_threads = 64;
-  int tensor_update = 1;   // FP32 super-panel updates: 1 tcgen05 + TMEM, 0 mma.sync
+  int tensor_update = 1;   // super-panel updates: 1 tcgen05 + TMEM, 0 FP32 mma.sync, FP64 CUDA cores
   long long q_wait_cycles = kQueueWaitCycles;  // queue schedule: limit of one dependency wait
   long long update_wait_polls = kTcWaitPolls;
   int q_skip_publish = -1;  // queue schedule: forward list entry whose done flag is withheld (tests)

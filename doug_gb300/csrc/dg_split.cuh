@@ -13,7 +13,14 @@
 // rounds once.  What is dropped (s >= 8) is below 2^-58 (root mean square;
 // 2^-53 at most) of the two rows' largest entries times each other, where a
 // chain of 128 FP64 multiply-adds rounds by 2^-53 of its partial sums each
-// time.  (Ozaki, Ogita, Oishi and Rump, error-free transformation of a matrix
+// time.  An entry more than nine binary orders below its row's largest keeps
+// fewer bits than its own 53, so that a sum of such entries alone is not what
+// the chain gives, entry by entry; the factor's error bound is in the rows'
+// sizes (sqrt(c_ii c_jj) for the entry (i, j) of the Schur complement) either
+// way.  Direct solves of one subdomain (3-D log-normal diffusion 14^3 .. 26^3,
+// Poisson 65^2 .. 200^2, elasticity 6^3 .. 11^3, six seeds, four right-hand
+// sides): residuals with this 0.95 to 1.01 times those of the CUDA cores, errors
+// against 64 bits 0.84 to 1.16 times (geometric mean 0.99).  (Ozaki, Ogita, Oishi and Rump, error-free transformation of a matrix
 // product by slices, Numer. Algorithms 59, 2012.)
 //
 // mf_split writes the slices once per super-panel, in the shared-memory

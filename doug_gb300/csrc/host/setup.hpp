@@ -39,7 +39,7 @@ struct Controls {
   int reuse_factors = 0;            // 1: a solve after the first keeps the numeric factors
   int elemental_matvec = 0;         // 1: PCG products with the stored element matrices
   // tuning of the multifrontal batches (dg_autotune chooses them)
-  int panel_rows = 512;             // fronts up to this size (and panel + E <= 96 KB): one CTA each
+  int panel_rows = 512;             // fronts up to this size (and panel + E <= 96 KB) may be factored by one CTA each
   int fwd_task_kb = 96;             // KB of E per forward task of a large front
   int lean_task_kb = 80;            // levels with smaller average tasks use 128-thread CTAs
   int thin_level_fronts = 1500;     // levels with fewer small fronts solve them one CTA per task
@@ -48,7 +48,7 @@ struct Controls {
   int factor_overlap = 1;           // 1: a level's one-CTA fronts factored on a side stream beside its large fronts
   int executable = -1;              // which reference driver: -1/0 doug_aggr, 1 doug_geom
   int device_setup = 1;             // 1: smoothing, re-bucketing and Galerkin products on the GPU when one is visible
-  int tensor_update = 1;            // FP32 super-panel trailing updates: 1 tcgen05 (TMEM accumulator), 0 mma.sync
+  int tensor_update = 1;            // super-panel updates: 1 tcgen05 (TMEM accumulators), 0 FP32 mma.sync, FP64 CUDA cores
   int super_panel = 128;           // columns of L per trailing update of a large front (multiple of 32)
   int split_blocks = 4096;         // FP64 tensor-core updates: 64-row blocks of digit slices (128 KB) held at once, 0 none
   int split_always = 0;            // 1: those updates on the tensor cores whatever they cost (tests)

@@ -301,9 +301,13 @@ mf_update_split(MfView v, const int4 *__restrict__ tasks, int ntasks, int nupd, 
       if (!ok) break;
       tc::mma_commit(tc::smem_u32(&done));
       t += gridDim.x;
-      if (t < ntasks) task = tasks[t];
-      ok = tc::mbar_wait(&done, p0, kTcWaitPolls);  // (of the last tile too: its MMAs use the tensor memory)
-      if (!ok || t >= ntasks) break;
+      if (t >= ntasks) {  // (the last tile's MMAs too use the tensor memory)
+        ok = tc::mbar_wait(&done, p0, kTcWaitPolls);
+        break;
+      }
+      task = tasks[t];
+      ok = tc::mbar_wait(&done, p0, kTcWaitPolls);
+      if (!ok) break;
       p0 ^= 1;
       if (two) p1 ^= 1;
       load_first(task);

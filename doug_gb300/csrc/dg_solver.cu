@@ -2210,7 +2210,7 @@ dg_status do_solve(dg_handle *h, const double *d_b, double *d_x, dg_stats *st, c
   const int n = h->n;
   const int grid = h->vec_grid;
   const SolvePlan pl = plan_of(h, c);
-  const bool fine = pl.fine, sgs = pl.sgs, coarse = pl.coarse, mixed = pl.mixed;
+  const bool coarse = pl.coarse, mixed = pl.mixed;
   int launches = 0;
   dg_stats out{};
   out.n = n;
